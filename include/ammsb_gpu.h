@@ -82,9 +82,9 @@ typedef struct ammsb_options {
   int32_t device;               /* CUDA device ordinal, default 0 */
   int32_t use_graph;            /* capture the iteration in a CUDA graph (1) */
   int32_t verbose;              /* info lines on stderr like learner.cc:105-120 */
-  int32_t pipeline;             /* 1 (default): the draws of the next two
+  int32_t pipeline;             /* 1 (default): the draws of the next eight
                                    iterations run on a second stream during the
-                                   update; 0: run()'s loop order on one stream,
+                                   updates of eight; 0: run()'s loop order on one stream,
                                    draws then update (cc:126-170) */
 } ammsb_options;
 

@@ -7,11 +7,11 @@
 // shape: blockIdx.y selects the chain, whose model, graph and buffer sets
 // come from a device array of ChainArgs.  Chains of different row widths,
 // minibatch sizes and graphs therefore run in a handful of launches per
-// iteration instead of five per chain, and the whole iteration of all
-// chains -- the update of iteration t and, on a second stream, the draws of
-// t + 1 -- is captured as one graph per buffer parity.  Every chain keeps
-// its own step counter and Philox key, so a chain advanced in a batch goes
-// through exactly the states it goes through on its own.
+// iteration instead of five per chain, and a block of iterations of all
+// chains -- their updates and, on a second stream, one launch of all their
+// next block's draws -- is captured as one graph per block of the ring.
+// Every chain keeps its own step counter and Philox key, so a chain advanced
+// in a batch goes through exactly the states it goes through on its own.
 #include <algorithm>
 #include <cstdlib>
 #include <cstdio>
@@ -153,12 +153,15 @@ struct ammsb_batch {
   int theta_gx = 1;
   int nbr_gx = 1;
   size_t mb_smem = 0, nbr_smem = 0;
-  cudaGraphExec_t exec[2] = {nullptr, nullptr};
-  cudaGraphExec_t execL[2] = {nullptr, nullptr};  // graph_iters iterations per launch
-  int graph_iters = 8;
-  int parity = 0;
-  bool prefetched = false;
+  // captured iterations, as for one chain (ammsb_handle): a block with the
+  // other block's draws alongside, both in turn, runs of updates in a block
+  cudaGraphExec_t graphB[2] = {}, graphL[2] = {};
+  cudaGraphExec_t graphU[kMaxRing][4] = {};
+  int block = kMaxBlock;  // iterations per draws launch: the smallest of the chains'
+  int slot = 0;           // ring slot of the next iteration, in every chain's ring
+  int ahead = 0;          // iterations drawn from `slot` on, as ammsb_handle::ahead
   std::vector<uint64_t> expect_step;  // each chain's step_count after the last batch step
+  std::vector<uint64_t> expect_gen;   // and its ring_gen
   std::string err;
 };
 
@@ -201,23 +204,56 @@ cudaError_t launch_update_chains(ammsb_batch* bt, int p) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_sampling_chains(ammsb_batch* bt, int p, cudaStream_t st) {
-  const unsigned n = (unsigned)bt->h.size();
-  k_sample_minibatch_chains<<<dim3(1, n), 1024, bt->mb_smem, st>>>(bt->d_all, p);
+// Draws of one block of every chain, into the buffer sets from s0 on.
+cudaError_t launch_sampling_chains(ammsb_batch* bt, int s0, cudaStream_t st) {
+  const unsigned n = (unsigned)bt->h.size(), D = (unsigned)bt->block;
+  k_sample_minibatch_chains<<<dim3(D, n), 1024, bt->mb_smem, st>>>(bt->d_all, s0);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_sample_neighbors_chains<8><<<dim3(bt->nbr_gx, n), 256, bt->nbr_smem, st>>>(bt->d_all, p);
+  k_sample_neighbors_chains<8><<<dim3(bt->nbr_gx, n, D), 256, bt->nbr_smem, st>>>(bt->d_all, s0);
   return cudaGetLastError();
 }
 
-cudaError_t launch_pipelined_chains(ammsb_batch* bt, int p) {
+cudaError_t launch_updates_chains(ammsb_batch* bt, int s, int count) {
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < count && e == cudaSuccess; ++i) e = launch_update_chains(bt, s + i);
+  return e;
+}
+
+// The draws of block `blk` forked onto the side stream, and their join (as
+// fork_draws / join_draws for one chain).
+cudaError_t fork_draws_chains(ammsb_batch* bt, int blk) {
   cudaError_t e = cudaEventRecord(bt->ev_fork, bt->stream);
   if (e != cudaSuccess) return e;
   if ((e = cudaStreamWaitEvent(bt->side, bt->ev_fork, 0)) != cudaSuccess) return e;
-  if ((e = launch_update_chains(bt, p)) != cudaSuccess) return e;
-  if ((e = launch_sampling_chains(bt, 1 - p, bt->side)) != cudaSuccess) return e;
-  if ((e = cudaEventRecord(bt->ev_join, bt->side)) != cudaSuccess) return e;
+  if ((e = launch_sampling_chains(bt, blk * bt->block, bt->side)) != cudaSuccess) return e;
+  return cudaEventRecord(bt->ev_join, bt->side);
+}
+
+cudaError_t launch_block_chains(ammsb_batch* bt, int blk) {
+  cudaError_t e = fork_draws_chains(bt, 1 - blk);
+  if (e != cudaSuccess) return e;
+  if ((e = launch_updates_chains(bt, blk * bt->block, bt->block)) != cudaSuccess) return e;
   return cudaStreamWaitEvent(bt->stream, bt->ev_join, 0);
+}
+
+// Launches `work` as a captured graph kept in g.
+template <typename F>
+int launch_graph(ammsb_batch* bt, cudaGraphExec_t& g, F&& work) {
+  if (!g) {
+    cudaGraph_t graph;
+    BK(cudaStreamBeginCapture(bt->stream, cudaStreamCaptureModeThreadLocal));
+    cudaError_t e = work();
+    cudaError_t e2 = cudaStreamEndCapture(bt->stream, &graph);
+    if (e != cudaSuccess || e2 != cudaSuccess) {
+      bt->err = std::string("graph capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2);
+      return AMMSB_E_CUDA;
+    }
+    BK(cudaGraphInstantiate(&g, graph, cudaGraphInstantiateFlagUseNodePriority));
+    cudaGraphDestroy(graph);
+  }
+  BK(cudaGraphLaunch(g, bt->stream));
+  return AMMSB_OK;
 }
 
 template <typename T>
@@ -243,9 +279,12 @@ void ammsb_batch_destroy(ammsb_batch* bt) {
   cudaSetDevice(bt->device);
   if (bt->stream) cudaStreamSynchronize(bt->stream);
   if (bt->side) cudaStreamSynchronize(bt->side);
-  for (auto* set : {bt->exec, bt->execL})
-    for (int q = 0; q < 2; ++q)
-      if (set[q]) cudaGraphExecDestroy(set[q]);
+  for (int q = 0; q < 2; ++q)
+    for (cudaGraphExec_t g : {bt->graphB[q], bt->graphL[q]})
+      if (g) cudaGraphExecDestroy(g);
+  for (auto& per_slot : bt->graphU)
+    for (cudaGraphExec_t g : per_slot)
+      if (g) cudaGraphExecDestroy(g);
   for (void* p : bt->allocs) cudaFree(p);
   for (cudaEvent_t ev : {bt->ev_fork, bt->ev_join, bt->ev_done, bt->ev_groups})
     if (ev) cudaEventDestroy(ev);
@@ -287,8 +326,8 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     bt->h.push_back(h);
   }
   bt->device = handles[0]->device;
-  if (const char* env = std::getenv("AMMSB_BATCH_GRAPH_ITERS"))  // even; 1 = one iteration per launch
-    bt->graph_iters = std::max(1, std::min(64, std::atoi(env) & ~1));
+  if (const char* env = std::getenv("AMMSB_BATCH_GRAPH_ITERS"))  // iterations of both blocks
+    bt->block = std::max(1, std::min(kMaxBlock, std::atoi(env) / 2));
   int prio_lo = 0, prio_hi = 0;  // the draws ahead at the higher priority, as for one chain
   if (cudaSetDevice(bt->device) != cudaSuccess ||
       cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) != cudaSuccess ||
@@ -306,8 +345,8 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     ChainArgs& a = args[i];
     a.m = h->m;
     a.g = h->g;
-    a.b[0] = h->bufs[0];
-    a.b[1] = h->bufs[1];
+    a.b = h->b;
+    bt->block = std::min(bt->block, h->block);
     a.ncommit = h->ncommit;
     a.smem_hash = h->mb_smem > 0 ? 1 : 0;
     bt->mb_smem = std::max(bt->mb_smem, h->mb_smem);
@@ -412,6 +451,7 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     return bail(AMMSB_E_CUDA);
   }
   bt->expect_step.assign(n, 0);
+  bt->expect_gen.assign(n, 0);
   *out = bt;
   return AMMSB_OK;
 }
@@ -429,57 +469,72 @@ int ammsb_batch_step(ammsb_batch* bt, int64_t n_iters) {
   if (n_iters == 0) return AMMSB_OK;
   // chains stepped on their own since the last batch step lose the batch's
   // draws made ahead: start from each chain's own step counter again
-  bool in_sync = bt->prefetched;
-  for (size_t i = 0; i < bt->h.size() && in_sync; ++i) {
-    ammsb_handle* h = bt->h[i];
-    in_sync = h->ahead >= 1 && h->slot == bt->parity && h->step_count == bt->expect_step[i];
-  }
+  bool in_sync = bt->ahead > 0;
+  for (size_t i = 0; i < bt->h.size() && in_sync; ++i)
+    in_sync = bt->h[i]->ring_gen == bt->expect_gen[i] && bt->h[i]->step_count == bt->expect_step[i];
   for (ammsb_handle* h : bt->h) BK(cudaStreamSynchronize(h->stream));
+  const int D = bt->block, R = 2 * D;
+  uint32_t drawn = 0;  // iterations drawn by this call
   if (!in_sync) {
-    for (ammsb_handle* h : bt->h) {
-      int rc = ammsb_detail::invalidate_prefetch(h);
+    for (size_t i = 0; i < bt->h.size(); ++i) {
+      ammsb_handle* h = bt->h[i];
+      ammsb_detail::invalidate_prefetch(h);
+      bt->expect_gen[i] = h->ring_gen;
+      int rc = ammsb_detail::point_draws(h, h->step_count, h->stream);
       if (rc) {
         bt->err = h->err;
         return rc;
       }
-      h->slot = 0;
       BK(cudaStreamSynchronize(h->stream));
     }
-    bt->parity = 0;
+    bt->slot = 0;
     BK(launch_sampling_chains(bt, 0, bt->stream));
-    bt->prefetched = true;
+    bt->ahead = D;
+    drawn += (uint32_t)D;
   }
-  // graph_iters iterations per graph launch while that many are left (an
-  // even count: the launch ends on the parity it started from), then one
-  for (int64_t it = 0; it < n_iters;) {
-    const int p = bt->parity;
-    const int L = (bt->graph_iters > 1 && n_iters - it >= bt->graph_iters) ? bt->graph_iters : 1;
-    cudaGraphExec_t& g = (L > 1) ? bt->execL[p] : bt->exec[p];
-    if (!g) {
-      cudaGraph_t graph;
-      BK(cudaStreamBeginCapture(bt->stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t e = cudaSuccess;
-      for (int j = 0; j < L && e == cudaSuccess; ++j) e = launch_pipelined_chains(bt, p ^ (j & 1));
-      cudaError_t e2 = cudaStreamEndCapture(bt->stream, &graph);
-      if (e != cudaSuccess || e2 != cudaSuccess) {
-        bt->err = std::string("graph capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2);
-        return AMMSB_E_CUDA;
+  bool forked = false;
+  int64_t left = n_iters;
+  while (left > 0) {  // as ammsb_step
+    const int s = bt->slot, pos = s % D, blk = s / D;
+    int n, rc;
+    if (pos == 0 && left >= D) {
+      const bool both = left >= 2 * (int64_t)D;
+      n = both ? 2 * D : D;
+      rc = launch_graph(bt, both ? bt->graphL[blk] : bt->graphB[blk], [&] {
+        cudaError_t e = launch_block_chains(bt, blk);
+        return e == cudaSuccess && both ? launch_block_chains(bt, 1 - blk) : e;
+      });
+      drawn += (uint32_t)n;
+    } else {
+      if (pos == 0) {
+        BK(fork_draws_chains(bt, 1 - blk));
+        forked = true;
+        drawn += (uint32_t)D;
+        bt->ahead += D;
       }
-      BK(cudaGraphInstantiate(&g, graph, cudaGraphInstantiateFlagUseNodePriority));
-      cudaGraphDestroy(graph);
+      const int most = (int)std::min<int64_t>(left, D - pos);
+      int lg = 0;
+      while (lg < 3 && (2 << lg) <= most) ++lg;
+      n = 1 << lg;
+      rc = launch_graph(bt, bt->graphU[s][lg], [&] { return launch_updates_chains(bt, s, n); });
+      bt->ahead -= n;
+      if (forked && (s + n) % D == 0) {
+        BK(cudaStreamWaitEvent(bt->stream, bt->ev_join, 0));
+        forked = false;
+      }
     }
-    BK(cudaGraphLaunch(g, bt->stream));
-    bt->parity ^= (L & 1);
-    it += L;
+    if (rc) return rc;
+    bt->slot = (s + n) % R;
+    left -= n;
   }
+  if (forked) BK(cudaStreamWaitEvent(bt->stream, bt->ev_join, 0));
   BK(cudaEventRecord(bt->ev_done, bt->stream));
   for (size_t i = 0; i < bt->h.size(); ++i) {
     ammsb_handle* h = bt->h[i];
     BK(cudaStreamWaitEvent(h->stream, bt->ev_done, 0));  // later work on the chain's own stream
     h->step_count += (uint64_t)n_iters;
-    h->slot = bt->parity;
-    h->ahead = 1;  // the batch draws one iteration ahead, into buffer sets 0 and 1
-    h->last = bt->parity ^ 1;
+    h->dev_next += drawn;
+    h->last = (bt->slot + R - 1) % R;
     bt->expect_step[i] = h->step_count;
   }
   BK(cudaStreamSynchronize(bt->stream));

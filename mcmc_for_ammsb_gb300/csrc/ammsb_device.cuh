@@ -48,9 +48,9 @@ enum : int32_t {
 
 // Per-iteration scalars of one minibatch buffer set, resident in device
 // memory so that a captured CUDA graph can replay the iteration without host
-// involvement.  The sampler keeps a ring of buffer sets: the draws of
-// iterations t+2 and t+3 are made while iterations t and t+1 update the
-// state.
+// involvement.  The sampler keeps a ring of buffer sets in two blocks: the
+// draws of a block's iterations are made by one launch while the iterations
+// of the other block update the state.
 struct DevState {
   uint32_t step;   // step_count of the iteration these draws belong to
   float eps;       // eps_t of that iteration
@@ -59,13 +59,13 @@ struct DevState {
   int32_t n_edges;
   int32_t n_nodes;
   int32_t rounds;
-  int32_t pad;
+  int32_t err;  // error bits of these draws, raised when the iteration is applied
 };
 
 // Sampler-wide counters shared by all buffer sets.
 struct DevCounters {
-  uint32_t next_step;        // step_count the next sampling pass draws for
-  int32_t err;               // error bits
+  uint32_t next_step;        // step_count the next draws launch starts from
+  int32_t err;               // error bits of the iterations applied so far
   unsigned long long evals;  // running sum of n_nodes * n_out (edge evaluations)
   unsigned long long iters;  // running count of updated iterations
 };

@@ -230,9 +230,14 @@ cudaError_t launch_normalize(ammsb_handle* h) {
 // Records `ev` on `s` when timing (ev != nullptr).  Inside a stream
 // capture an external record becomes an event-record node of the graph, so
 // the event is recorded every time the graph runs (a plain record would only
-// mark a dependency of the capture).
+// mark a dependency of the capture; outside a capture the flag is not valid).
 inline cudaError_t mark(cudaEvent_t ev, cudaStream_t s) {
-  return ev ? cudaEventRecordWithFlags(ev, s, cudaEventRecordExternal) : cudaSuccess;
+  if (!ev) return cudaSuccess;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &st);
+  if (e != cudaSuccess) return e;
+  return cudaEventRecordWithFlags(ev, s, st == cudaStreamCaptureStatusActive ? cudaEventRecordExternal
+                                                                             : cudaEventRecordDefault);
 }
 
 // The iteration's kernels in order; `b` carries the fed-noise pointers when
@@ -256,125 +261,134 @@ cudaError_t launch_update_phase(ammsb_handle* h, const Buffers& b, const cudaEve
   return mark(ev ? ev[2] : nullptr, h->stream);
 }
 
-// Draws of one iteration (minibatch + neighbour sets) into buffer set b;
-// with `ev`, events after each of the two kernels.
-cudaError_t launch_sampling_phase(ammsb_handle* h, const Buffers& b, cudaStream_t s,
+// Buffer set `slot` of the handle's ring.
+Buffers ring_set(const ammsb_handle* h, int slot) { return slot_buffers(h->m, h->b, slot); }
+
+// Draws of `count` iterations (minibatches + neighbour sets, from the
+// device's next step on) into the buffer sets from s0 on; with `ev`, events
+// before and after each of the two kernels.
+cudaError_t launch_sampling_phase(ammsb_handle* h, int s0, int count, cudaStream_t s,
                                   const cudaEvent_t* ev = nullptr) {
-  k_sample_minibatch<<<1, 1024, h->mb_smem, s>>>(h->m, h->g, b, h->mb_smem > 0);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess || (e = mark(ev ? ev[0] : nullptr, s)) != cudaSuccess) return e;
-  k_sample_neighbors<8><<<h->nbr_blocks, 256, h->nbr_smem, s>>>(h->m, h->g, b);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  return mark(ev ? ev[1] : nullptr, s);
-}
-
-// `n` (1 or 2) pipelined iterations from ring slot s: the updates of slots
-// s .. s+n-1 on the handle's stream, concurrently with the draws of the
-// iterations two ahead (slots s+2 .. s+n+1) on the side stream (fork/join by
-// events; inside a capture these become graph edges).  Draws depend only on
-// the step index, so they can run ahead; taking two iterations per join
-// lets the short updates of link-stratum iterations and the longer draws of
-// the non-link ones even out.
-// With `ev` (run()'s timers): events ev[0] before the first update and
-// ev[1 + 3i ..] after each phase of update i on the update stream, then
-// ev[1 + 3n] before the first draws and ev[2 + 3n + 2i ..] after each of
-// draws i on the draws' stream.
-// `first_pdl`: the previous pair's theta step is the kernel ahead of the
-// first update (a long graph of several pairs), which may then start early
-// too.
-cudaError_t launch_pipelined(ammsb_handle* h, int s, int n, const cudaEvent_t* ev = nullptr,
-                             bool first_pdl = false) {
-  cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
+  cudaError_t e = mark(ev ? ev[0] : nullptr, s);
   if (e != cudaSuccess) return e;
-  if ((e = cudaStreamWaitEvent(h->side, h->ev_fork, 0)) != cudaSuccess) return e;
-  if ((e = mark(ev ? ev[0] : nullptr, h->stream)) != cudaSuccess) return e;
-  // the second update follows the first one's theta step directly (its
-  // draws were joined before this launch)
-  for (int i = 0; i < n; ++i)
-    if ((e = launch_update_phase(h, h->bufs[(s + i) % kRing], ev ? ev + 1 + 3 * i : nullptr,
-                                 (i > 0 || first_pdl) && !ev)) != cudaSuccess)
-      return e;
-  if ((e = mark(ev ? ev[1 + 3 * n] : nullptr, h->side)) != cudaSuccess) return e;
-  for (int i = 0; i < n; ++i)
-    if ((e = launch_sampling_phase(h, h->bufs[(s + 2 + i) % kRing], h->side,
-                                   ev ? ev + 2 + 3 * n + 2 * i : nullptr)) != cudaSuccess)
-      return e;
-  if ((e = cudaEventRecord(h->ev_join, h->side)) != cudaSuccess) return e;
-  return cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+  k_sample_minibatch<<<count, 1024, h->mb_smem, s>>>(h->m, h->g, h->b, s0, h->mb_smem > 0);
+  if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(ev ? ev[1] : nullptr, s)) != cudaSuccess) return e;
+  k_sample_neighbors<8><<<dim3(h->nbr_blocks, count), 256, h->nbr_smem, s>>>(h->m, h->g, h->b, s0);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return mark(ev ? ev[2] : nullptr, s);
 }
 
-// `n` (1 or 2) iterations from ring slot s in run()'s loop order on the
-// handle's stream, each drawn right before its update (the pipeline
-// option off).  With `ev`: per iteration i, events ev[6i] before the draws,
-// ev[6i + 1], ev[6i + 2] after each draw kernel and ev[6i + 3 ..] after
-// each update phase.
-cudaError_t launch_serial(ammsb_handle* h, int s, int n, const cudaEvent_t* ev = nullptr) {
+// `count` updates from ring slot s on; `first_pdl`: the theta step of the
+// iteration before is the kernel ahead of the first one in the stream.  With
+// `timed`, each records its buffer set's events.
+cudaError_t launch_updates(ammsb_handle* h, int s, int count, bool timed, bool first_pdl = false) {
   cudaError_t e = cudaSuccess;
-  for (int i = 0; i < n; ++i) {
-    const Buffers& b = h->bufs[(s + i) % kRing];
-    if ((e = mark(ev ? ev[6 * i] : nullptr, h->stream)) != cudaSuccess) return e;
-    if ((e = launch_sampling_phase(h, b, h->stream, ev ? ev + 6 * i + 1 : nullptr)) != cudaSuccess) return e;
-    if ((e = launch_update_phase(h, b, ev ? ev + 6 * i + 3 : nullptr)) != cudaSuccess) return e;
+  for (int i = 0; i < count && e == cudaSuccess; ++i) {
+    const cudaEvent_t* ev = timed ? h->ev_upd[(s + i) % h->m.ring] : nullptr;
+    e = mark(ev ? ev[0] : nullptr, h->stream);
+    // an update after another follows its theta step directly (its draws
+    // were joined before this launch)
+    if (e == cudaSuccess)
+      e = launch_update_phase(h, ring_set(h, (s + i) % h->m.ring), ev ? ev + 1 : nullptr,
+                              (i > 0 || first_pdl) && !ev);
   }
   return e;
 }
 
-// Adds the phase durations of a finished timed launch (n iterations from
-// slot s) to run()'s timers; waits for the launch's events.
-int read_phase_events(ammsb_handle* h, int n, int s) {
-  const cudaEvent_t* ev = h->ev_phase[n - 1][s];
-  if (!h->opt.pipeline) {  // launch_serial's layout: 6 events per iteration
-    CK(cudaEventSynchronize(ev[6 * n - 1]));
-    const int order[5] = {ammsb_handle::kTMiniBatch, ammsb_handle::kTNeighbors, ammsb_handle::kTPhi,
-                          ammsb_handle::kTPi, ammsb_handle::kTBeta};
-    for (int i = 0; i < n; ++i)
-      for (int q = 0; q < 5; ++q) {
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, ev[6 * i + q], ev[6 * i + q + 1]));
-        h->timers[order[q]].seconds += ms * 1e-3;
-      }
-    h->timers[ammsb_handle::kTMiniBatch].ticks += (uint64_t)n;
-    h->timers[ammsb_handle::kTPi].ticks += (uint64_t)n;
-    h->timers[ammsb_handle::kTBeta].ticks += (uint64_t)n;
-    return AMMSB_OK;
-  }
-  const cudaEvent_t* sv = ev + 1 + 3 * n;
-  CK(cudaEventSynchronize(ev[3 * n]));
-  CK(cudaEventSynchronize(sv[2 * n]));
+// Forks the draws of block `blk` onto the side stream, behind everything
+// queued on the handle's stream (the updates that read the block's buffer
+// sets last among it); join_draws makes the handle's stream wait for them.
+cudaError_t fork_draws(ammsb_handle* h, int blk, bool timed) {
+  cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
+  if (e != cudaSuccess) return e;
+  if ((e = cudaStreamWaitEvent(h->side, h->ev_fork, 0)) != cudaSuccess) return e;
+  const int s = blk * h->block;
+  if ((e = launch_sampling_phase(h, s, h->block, h->side, timed ? h->ev_drw[s] : nullptr)) != cudaSuccess)
+    return e;
+  return cudaEventRecord(h->ev_join, h->side);
+}
+cudaError_t join_draws(ammsb_handle* h) { return cudaStreamWaitEvent(h->stream, h->ev_join, 0); }
+
+// The iterations of block `blk` on the handle's stream, concurrently with
+// the draws of the other block on the side stream (inside a capture the
+// events become graph edges).  One draws launch per block: the single-CTA
+// minibatch kernel and the neighbour kernel are chains of dependent loads
+// (25 to 80 us an iteration on the 400k-node workload, 14 on a 5k-node one),
+// which eight iterations side by side pay once; with a launch per iteration
+// the draws were the longer branch of every small chain and of every
+// link-stratum iteration.
+cudaError_t launch_block(ammsb_handle* h, int blk, bool timed, bool first_pdl = false) {
+  cudaError_t e = fork_draws(h, 1 - blk, timed);
+  if (e != cudaSuccess) return e;
+  if ((e = launch_updates(h, blk * h->block, h->block, timed, first_pdl)) != cudaSuccess) return e;
+  return join_draws(h);
+}
+
+// One iteration at ring slot s in run()'s loop order on the handle's
+// stream, drawn right before its update (the pipeline option off).
+cudaError_t launch_serial(ammsb_handle* h, int s, bool timed) {
+  cudaError_t e = launch_sampling_phase(h, s, 1, h->stream, timed ? h->ev_drw[s] : nullptr);
+  return e != cudaSuccess ? e : launch_updates(h, s, 1, timed);
+}
+
+// Adds the phase durations of the timed launches whose events are pending
+// to run()'s timers, waiting for them: buffer sets s0 .. s0 + count - 1.
+int read_phase_events(ammsb_handle* h, int s0, int count) {
   auto add = [&](int t, cudaEvent_t a, cudaEvent_t b) -> int {
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, a, b));
     h->timers[t].seconds += ms * 1e-3;
     return AMMSB_OK;
   };
-  for (int i = 0; i < n; ++i) {
-    int rc = add(ammsb_handle::kTPhi, ev[3 * i], ev[3 * i + 1]);
-    if (!rc) rc = add(ammsb_handle::kTPi, ev[3 * i + 1], ev[3 * i + 2]);
-    if (!rc) rc = add(ammsb_handle::kTBeta, ev[3 * i + 2], ev[3 * i + 3]);
-    if (!rc) rc = add(ammsb_handle::kTMiniBatch, sv[2 * i], sv[2 * i + 1]);
-    if (!rc) rc = add(ammsb_handle::kTNeighbors, sv[2 * i + 1], sv[2 * i + 2]);
+  for (int s = s0; s < s0 + count; ++s) {
+    int rc = AMMSB_OK;
+    if (h->drw_pending[s]) {
+      const cudaEvent_t* ev = h->ev_drw[s];
+      CK(cudaEventSynchronize(ev[2]));
+      rc = add(ammsb_handle::kTMiniBatch, ev[0], ev[1]);
+      if (!rc) rc = add(ammsb_handle::kTNeighbors, ev[1], ev[2]);
+      h->drw_pending[s] = false;
+    }
+    if (!rc && h->upd_pending[s]) {
+      const cudaEvent_t* ev = h->ev_upd[s];
+      CK(cudaEventSynchronize(ev[3]));
+      rc = add(ammsb_handle::kTPhi, ev[0], ev[1]);
+      if (!rc) rc = add(ammsb_handle::kTPi, ev[1], ev[2]);
+      if (!rc) rc = add(ammsb_handle::kTBeta, ev[2], ev[3]);
+      h->timers[ammsb_handle::kTMiniBatch].ticks += 1;
+      h->timers[ammsb_handle::kTPi].ticks += 1;
+      h->timers[ammsb_handle::kTBeta].ticks += 1;
+      h->upd_pending[s] = false;
+    }
     if (rc) return rc;
   }
-  h->timers[ammsb_handle::kTMiniBatch].ticks += (uint64_t)n;
-  h->timers[ammsb_handle::kTPi].ticks += (uint64_t)n;
-  h->timers[ammsb_handle::kTBeta].ticks += (uint64_t)n;
   return AMMSB_OK;
 }
 
-// Reads every pending timed launch (all of them, or those up to and
-// including the one that used event set (n, s)).
-int drain_phase_events(ammsb_handle* h, int n = 0, int s = -1) {
-  size_t upto = h->pending.size();
-  if (s >= 0) {
-    upto = 0;
-    for (size_t q = 0; q < h->pending.size(); ++q)
-      if (h->pending[q].n == n && h->pending[q].s == s) upto = q + 1;
-  }
-  for (size_t q = 0; q < upto; ++q) {
-    int rc = read_phase_events(h, h->pending[q].n, h->pending[q].s);
+// Makes the event sets of `count` updates from slot s and of a draws launch
+// into slot d (-1: none) ready for a timed launch, reading what is pending,
+// and marks them.
+int take_phase_events(ammsb_handle* h, int s, int count, int d) {
+  auto take = [&](cudaEvent_t* ev, int n, bool* pending, int slot) -> int {
+    if (!ev[0])
+      for (int q = 0; q < n; ++q) CK(cudaEventCreate(&ev[q]));
+    if (*pending) {
+      int rc = read_phase_events(h, slot, 1);
+      if (rc) return rc;
+    }
+    return AMMSB_OK;
+  };
+  for (int i = 0; i < count; ++i) {
+    const int q = (s + i) % h->m.ring;
+    int rc = take(h->ev_upd[q], 4, &h->upd_pending[q], q);
     if (rc) return rc;
   }
-  h->pending.erase(h->pending.begin(), h->pending.begin() + (long)upto);
+  if (d >= 0) {
+    int rc = take(h->ev_drw[d], 3, &h->drw_pending[d], d);
+    if (rc) return rc;
+    h->drw_pending[d] = true;
+  }
+  for (int i = 0; i < count; ++i) h->upd_pending[(s + i) % h->m.ring] = true;
   return AMMSB_OK;
 }
 
@@ -426,13 +440,29 @@ int check_device_err(ammsb_handle* h) {
   return AMMSB_OK;
 }
 
-// Drops draws made ahead of time (their step no longer follows) and points
-// the device's next draw at the host's step_count.
-int invalidate_prefetch(ammsb_handle* h) {
-  if (h->ahead == 0) return AMMSB_OK;
+// The error bits of a drawn, not yet applied, iteration as a status.
+int check_draw_err(ammsb_handle* h, int slot) {
+  DevState st;
+  CK(cudaMemcpyAsync(&st, ring_set(h, slot).st, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
+  int rc = check_device_err(h);  // synchronises
+  if (rc || !st.err) return rc;
+  h->err = "device error bits " + std::to_string(st.err) +
+           " (1 minibatch cap, 2 neighbour cap, 4 capacity, 8 init cap)";
+  return (st.err & kErrCapacity) ? AMMSB_E_CAPACITY : AMMSB_E_SAMPLING;
+}
+
+// Drops draws made ahead of time (their step no longer follows, or their
+// buffer sets are about to be written).
+void invalidate_prefetch(ammsb_handle* h) {
   h->ahead = 0;
-  uint32_t s = (uint32_t)h->step_count;
-  CK(cudaMemcpyAsync(&h->gc->next_step, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
+  ++h->ring_gen;
+}
+
+int point_draws(ammsb_handle* h, uint64_t step, cudaStream_t s) {
+  const uint32_t next = (uint32_t)step;
+  if (h->dev_next == next) return AMMSB_OK;
+  CK(cudaMemcpyAsync(&h->gc->next_step, &next, sizeof(next), cudaMemcpyHostToDevice, s));
+  h->dev_next = next;
   return AMMSB_OK;
 }
 
@@ -441,12 +471,13 @@ int reset_counters(ammsb_handle* h) {
   h->average_count = 1;
   h->ppx_history.clear();
   h->slot = 0;
-  h->ahead = 0;
   h->last = -1;
+  invalidate_prefetch(h);
   DevCounters gc{};
   gc.next_step = 1;
   CK(cudaMemcpyAsync(h->gc, &gc, sizeof(gc), cudaMemcpyHostToDevice, h->stream));
-  for (int p = 0; p < kRing; ++p) CK(cudaMemsetAsync(h->bufs[p].st, 0, sizeof(DevState), h->stream));
+  h->dev_next = 1;
+  CK(cudaMemsetAsync(h->b.st, 0, sizeof(DevState) * h->m.ring, h->stream));
   CK(cudaMemsetAsync(h->d_ppx, 0, sizeof(float) * std::max<int64_t>(h->H, 1), h->stream));
   return AMMSB_OK;
 }
@@ -486,8 +517,6 @@ void choose_config(ammsb_handle* h) {
   // 100k-node one); the commit's early start measured no gain
   c.pdl = kPdlPhi | kPdlTheta;
   if (const char* env = std::getenv("AMMSB_PDL")) c.pdl = std::atoi(env) & (kPdlPhi | kPdlCommit | kPdlTheta);
-  c.graph_pairs = 8;
-  if (const char* env = std::getenv("AMMSB_GRAPH_PAIRS")) c.graph_pairs = std::max(1, std::min(64, std::atoi(env)));
   if (const char* env = std::getenv("AMMSB_PHI_KERNEL")) {  // "ring" or "regs"
     if (std::strcmp(env, "regs") == 0) c.ring = 0;
   }
@@ -502,11 +531,27 @@ void choose_config(ammsb_handle* h) {
   h->cfg = c;
 }
 
+// Destroys the captured iterations (their kernels or buffers changed, or
+// the handle goes).
+void drop_graphs(ammsb_handle* h) {
+  auto drop = [](cudaGraphExec_t& g) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  };
+  for (int q = 0; q < 2; ++q)
+    for (auto* set : {h->graphB, h->graphL, h->graphBt}) drop(set[q]);
+  for (int s = 0; s < kMaxRing; ++s) {
+    for (auto& g : h->graphU[s]) drop(g);
+    for (auto* set : {h->graphS, h->graphUt, h->graphSt}) drop(set[s]);
+  }
+}
+
 }  // namespace
 
 namespace ammsb_detail {
 int check_device_err(ammsb_handle* h) { return ::check_device_err(h); }
-int invalidate_prefetch(ammsb_handle* h) { return ::invalidate_prefetch(h); }
+void invalidate_prefetch(ammsb_handle* h) { ::invalidate_prefetch(h); }
+int point_draws(ammsb_handle* h, uint64_t step, cudaStream_t s) { return ::point_draws(h, step, s); }
 }  // namespace ammsb_detail
 
 extern "C" {
@@ -547,15 +592,15 @@ const char* ammsb_last_error(const ammsb_handle* h) { return h ? h->err.c_str() 
 void ammsb_destroy(ammsb_handle* h) {
   if (!h) return;
   cudaSetDevice(h->device);
-  for (auto* set : {h->graph1, h->graph2, h->graph1t, h->graph2t, h->graphL})
-    for (int s = 0; s < kRing; ++s)
-      if (set[s]) cudaGraphExecDestroy(set[s]);
+  drop_graphs(h);
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->side) cudaStreamSynchronize(h->side);
-  for (auto& per_n : h->ev_phase)
-    for (auto& set : per_n)
-      for (auto& e : set)
-        if (e) cudaEventDestroy(e);
+  for (int s = 0; s < kMaxRing; ++s) {
+    for (auto& e : h->ev_upd[s])
+      if (e) cudaEventDestroy(e);
+    for (auto& e : h->ev_drw[s])
+      if (e) cudaEventDestroy(e);
+  }
   for (void* p : h->allocs) cudaFree(p);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   if (h->ev_join) cudaEventDestroy(h->ev_join);
@@ -787,30 +832,41 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
   TRY(dev_alloc(h, &b.stage, (size_t)m.max_nodes * Kp));
   TRY(dev_alloc(h, &b.beta, (size_t)Kp));
   TRY(dev_alloc(h, &b.theta, 2 * (size_t)K));
-  for (int p = 0; p < kRing; ++p) {  // the ring of minibatch buffer sets
-    Buffers& bp = h->bufs[p];
-    TRY(dev_alloc(h, &bp.nodes, (size_t)m.max_nodes));
-    TRY(dev_alloc(h, &bp.ea, (size_t)m.max_edges));
-    TRY(dev_alloc(h, &bp.eb, (size_t)m.max_edges));
-    TRY(dev_alloc(h, &bp.ey, (size_t)m.max_edges));
-    TRY(dev_alloc(h, &bp.nbr, (size_t)m.max_nodes * m.n_out));
-    TRY(dev_alloc(h, &bp.st, 1));
-  }
   // a minibatch round examines up to max(remaining, 4096) candidates while
   // the dedup hash stays at most half full
-  TRY(dev_alloc(h, &b.cand, (size_t)std::max<int64_t>(o.mini_batch_size, 4096)));
+  m.slot_cand = std::max<int64_t>(o.mini_batch_size, 4096);
   // ... and numbers the nodes of a general edge list (random-edge, several
   // link sources) in the same table: at most max_nodes distinct vertices
   int64_t hneed = std::max<int64_t>(8192, 2 * o.mini_batch_size);
   if (multi_src || rand_edge) hneed = std::max<int64_t>(hneed, 2 * (int64_t)m.max_nodes);
   const int hcap = next_pow2(hneed);
-  TRY(dev_alloc(h, &b.htab_key, (size_t)hcap));
-  TRY(dev_alloc(h, &b.htab_idx, (size_t)hcap));
   b.hmask = (uint32_t)(hcap - 1);
   // the dedup hash lives in shared memory when it fits (up to 16Ki entries)
   if (hcap <= 16384 &&
       ammsb_detail::raise_smem_limit(k_sample_minibatch, 2 * sizeof(uint32_t) * hcap) == cudaSuccess)
     h->mb_smem = 2 * sizeof(uint32_t) * (size_t)hcap;
+  // the ring of minibatch buffer sets: two blocks of iterations
+  m.slot_nodes = (m.max_nodes + 31ll) / 32 * 32;
+  m.slot_edges = (m.max_edges + 31ll) / 32 * 32;
+  m.slot_nbr = (m.slot_nodes * m.n_out + 31) / 32 * 32;
+  if (const char* env = std::getenv("AMMSB_GRAPH_PAIRS"))
+    h->block = std::max(1, std::min(kMaxBlock, std::atoi(env)));
+  const int64_t set_bytes = 4 * (m.slot_nodes + m.slot_nbr) + 9 * m.slot_edges + 2 * m.slot_cand +
+                            (h->mb_smem ? 0 : 4ll * hcap);
+  if (2 * h->block * set_bytes > kRingBytes) h->block = std::min(h->block, 2);
+  m.ring = 2 * h->block;
+  const size_t nring = (size_t)m.ring;
+  TRY(dev_alloc(h, &b.nodes, nring * m.slot_nodes));
+  TRY(dev_alloc(h, &b.ea, nring * m.slot_edges));
+  TRY(dev_alloc(h, &b.eb, nring * m.slot_edges));
+  TRY(dev_alloc(h, &b.ey, nring * m.slot_edges));
+  TRY(dev_alloc(h, &b.nbr, nring * m.slot_nbr));
+  TRY(dev_alloc(h, &b.st, nring));
+  TRY(dev_alloc(h, &b.cand, (size_t)h->block * m.slot_cand));
+  if (!h->mb_smem) {
+    TRY(dev_alloc(h, &b.htab_key, (size_t)h->block * hcap));
+    TRY(dev_alloc(h, &b.htab_idx, (size_t)h->block * hcap));
+  }
   TRY(dev_alloc(h, &b.beta_part, (size_t)m.nbb * 2 * Kp));
   TRY(dev_alloc(h, &h->gc, 1));
   b.gc = h->gc;
@@ -819,21 +875,6 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
   TRY(dev_alloc(h, &h->d_fed_theta_noise, 2 * (size_t)K));
   b.fed_phi_noise = nullptr;
   b.fed_theta_noise = nullptr;
-  for (int p = 0; p < kRing; ++p) {  // shared state + this set's minibatch arrays
-    Buffers own = h->bufs[p];
-    h->bufs[p] = b;
-    h->bufs[p].nodes = own.nodes;
-    h->bufs[p].ea = own.ea;
-    h->bufs[p].eb = own.eb;
-    h->bufs[p].ey = own.ey;
-    h->bufs[p].nbr = own.nbr;
-    h->bufs[p].st = own.st;
-  }
-  b.nodes = nullptr;
-  b.ea = b.eb = nullptr;
-  b.ey = nullptr;
-  b.nbr = nullptr;
-  b.st = nullptr;
 #undef TRY
   // commit blocks (4 rows each, grid-strided): two per SM, so an iteration
   // of few nodes does not launch a thousand idle blocks
@@ -942,9 +983,9 @@ int ammsb_set_step(ammsb_handle* h, uint64_t step_count) {
   if (!h || step_count < 1 || step_count > 0xffffffffull) return AMMSB_E_ARG;
   CK(cudaSetDevice(h->device));
   h->step_count = step_count;
-  h->ahead = 0;
-  uint32_t s = (uint32_t)step_count;
-  CK(cudaMemcpyAsync(&h->gc->next_step, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
+  invalidate_prefetch(h);
+  int rc = point_draws(h, step_count, h->stream);
+  if (rc) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return AMMSB_OK;
 }
@@ -957,79 +998,104 @@ int ammsb_step(ammsb_handle* h, int64_t n_iters) {
   }
   CK(cudaSetDevice(h->device));
   if (n_iters == 0) return AMMSB_OK;
-  // the draws of the next two iterations, where they are not made yet
-  while (h->opt.pipeline && h->ahead < 2) {
-    CK(launch_sampling_phase(h, h->bufs[(h->slot + h->ahead) % kRing], h->stream));
-    ++h->ahead;
-  }
-  auto launch = [&](int s, int n, const cudaEvent_t* ev) {
-    return h->opt.pipeline ? launch_pipelined(h, s, n, ev) : launch_serial(h, s, n, ev);
+  // launches `work` as a captured graph (kept in g), or directly
+  auto launch = [&](cudaGraphExec_t& g, auto&& work) -> int {
+    if (!h->opt.use_graph) {
+      CK(work());
+      return AMMSB_OK;
+    }
+    if (!g) {
+      cudaGraph_t graph;
+      CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+      cudaError_t e = work();
+      cudaError_t e2 = cudaStreamEndCapture(h->stream, &graph);
+      if (e != cudaSuccess || e2 != cudaSuccess) {
+        h->err = std::string("graph capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2);
+        return AMMSB_E_CUDA;
+      }
+      CK(cudaGraphInstantiate(&g, graph, cudaGraphInstantiateFlagUseNodePriority));
+      cudaGraphDestroy(graph);
+    }
+    CK(cudaGraphLaunch(g, h->stream));
+    return AMMSB_OK;
   };
+  const int D = h->block, R = h->m.ring;
+  const bool timed = h->timing;
+  int rc = AMMSB_OK;
+  if (!h->opt.pipeline) {  // the loop's order, one iteration at a time
+    invalidate_prefetch(h);
+    if ((rc = point_draws(h, h->step_count, h->stream))) return rc;
+    for (int64_t i = 0; i < n_iters; ++i) {
+      const int s = h->slot;
+      if (timed && (rc = take_phase_events(h, s, 1, s))) return rc;
+      if ((rc = launch(timed ? h->graphSt[s] : h->graphS[s], [&] { return launch_serial(h, s, timed); })))
+        return rc;
+      ++h->dev_next;
+      h->last = s;
+      h->slot = (s + 1) % R;
+    }
+    h->step_count += (uint64_t)n_iters;
+    return AMMSB_OK;
+  }
+  if (h->ahead == 0) {  // the first block's draws
+    ++h->ring_gen;
+    h->slot = 0;
+    if ((rc = point_draws(h, h->step_count, h->stream))) return rc;
+    CK(launch_sampling_phase(h, 0, D, h->stream));
+    h->dev_next += (uint32_t)D;
+    h->ahead = D;
+  }
+  bool forked = false;  // draws on the side stream that this stream has not joined
   int64_t left = n_iters;
   while (left > 0) {
-    // long graphs: graph_pairs pipelined pairs per launch, so that every
-    // update but the launch's first follows a theta step inside the graph
-    // (and may start early), with fewer graph launches
-    const int L = h->cfg.graph_pairs;
-    if (L > 1 && h->opt.use_graph && h->opt.pipeline && !h->timing && left >= 2 * (int64_t)L) {
-      const int s = h->slot;
-      cudaGraphExec_t& g = h->graphL[s];
-      if (!g) {
-        cudaGraph_t graph;
-        CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = cudaSuccess;
-        for (int j = 0; j < L && e == cudaSuccess; ++j) e = launch_pipelined(h, (s + 2 * j) % kRing, 2, nullptr, j > 0);
-        cudaError_t e2 = cudaStreamEndCapture(h->stream, &graph);
-        if (e != cudaSuccess || e2 != cudaSuccess) {
-          h->err = std::string("graph capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2);
-          return AMMSB_E_CUDA;
-        }
-        CK(cudaGraphInstantiate(&g, graph, cudaGraphInstantiateFlagUseNodePriority));
-        cudaGraphDestroy(graph);
-      }
-      CK(cudaGraphLaunch(g, h->stream));
-      h->last = (s + 2 * L - 1) % kRing;
-      h->slot = (s + 2 * L) % kRing;
-      left -= 2 * L;
-      continue;
-    }
-    const int n = left >= 2 ? 2 : 1;
-    const int s = h->slot;
-    // run()'s timers: the launch records events between the phases; the
-    // events of an earlier launch with the same event set are read first
-    const cudaEvent_t* ev = nullptr;
-    if (h->timing) {
-      cudaEvent_t* set = h->ev_phase[n - 1][s];
-      if (!set[0])
-        for (int q = 0; q < 12; ++q) CK(cudaEventCreate(&set[q]));
-      int rc = drain_phase_events(h, n, s);
+    const int s = h->slot, pos = s % D, blk = s / D;
+    int n;
+    if (pos == 0 && left >= D) {
+      // whole blocks; both in turn in one launch, so that every update but
+      // the launch's first follows a theta step inside the graph (and may
+      // start early)
+      const bool both = h->opt.use_graph && !timed && left >= 2 * (int64_t)D;
+      n = both ? 2 * D : D;
+      if (timed && (rc = take_phase_events(h, s, D, (1 - blk) * D))) return rc;
+      if (both)
+        rc = launch(h->graphL[blk], [&] {
+          cudaError_t e = launch_block(h, blk, false);
+          return e != cudaSuccess ? e : launch_block(h, 1 - blk, false, true);
+        });
+      else
+        rc = launch(timed ? h->graphBt[blk] : h->graphB[blk], [&] { return launch_block(h, blk, timed); });
       if (rc) return rc;
-      ev = set;
-    }
-    if (h->opt.use_graph) {
-      cudaGraphExec_t& g = h->timing ? ((n == 2) ? h->graph2t[s] : h->graph1t[s])
-                                     : ((n == 2) ? h->graph2[s] : h->graph1[s]);
-      if (!g) {
-        cudaGraph_t graph;
-        CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = launch(s, n, ev);
-        cudaError_t e2 = cudaStreamEndCapture(h->stream, &graph);
-        if (e != cudaSuccess || e2 != cudaSuccess) {
-          h->err = std::string("graph capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2);
-          return AMMSB_E_CUDA;
-        }
-        CK(cudaGraphInstantiate(&g, graph, cudaGraphInstantiateFlagUseNodePriority));
-        cudaGraphDestroy(graph);
-      }
-      CK(cudaGraphLaunch(g, h->stream));
+      h->dev_next += (uint32_t)n;
     } else {
-      CK(launch(s, n, ev));
+      // part of a block: the other block's draws go out with its first
+      // iteration, as they do in a whole one
+      if (pos == 0) {
+        if (timed && (rc = take_phase_events(h, 0, 0, (1 - blk) * D))) return rc;
+        CK(fork_draws(h, 1 - blk, timed));
+        forked = true;
+        h->dev_next += (uint32_t)D;
+        h->ahead += D;
+      }
+      const int most = (int)std::min<int64_t>(left, D - pos);
+      int lg = 0;  // runs of a power of two of them, so that few graphs are kept
+      while (!timed && lg < 3 && (2 << lg) <= most) ++lg;
+      n = 1 << lg;
+      if (timed && (rc = take_phase_events(h, s, 1, -1))) return rc;
+      if ((rc = launch(timed ? h->graphUt[s] : h->graphU[s][lg], [&] { return launch_updates(h, s, n, timed); })))
+        return rc;
+      h->ahead -= n;
+      if (forked && (s + n) % D == 0) {
+        CK(join_draws(h));
+        forked = false;
+      }
     }
-    if (h->timing) h->pending.push_back({n, s});
-    h->last = (s + n - 1) % kRing;
-    h->slot = (s + n) % kRing;
+    h->last = (s + n - 1) % R;
+    h->slot = (s + n) % R;
     left -= n;
   }
+  // whatever follows on the handle's stream (state changes, other draws)
+  // comes after the draws made ahead
+  if (forked) CK(join_draws(h));
   h->step_count += (uint64_t)n_iters;
   return AMMSB_OK;
 }
@@ -1069,9 +1135,8 @@ int ammsb_step_fed(ammsb_handle* h, uint32_t step, int32_t n_edges, const int32_
     packed[q] = (uint32_t)nbrs[q] | ((nbr_y[q] ? 1u : 0u) << 31);
   }
   CK(cudaSetDevice(h->device));
-  int rc0 = invalidate_prefetch(h);
-  if (rc0) return rc0;
-  const Buffers& bp = h->bufs[h->slot];
+  invalidate_prefetch(h);
+  const Buffers bp = ring_set(h, h->slot);
   CK(cudaMemcpyAsync(bp.nodes, nodes, sizeof(int32_t) * n_nodes, cudaMemcpyHostToDevice, h->stream));
   if (n_edges > 0) {
     CK(cudaMemcpyAsync(bp.ea, edge_slot_a, sizeof(int32_t) * n_edges, cudaMemcpyHostToDevice, h->stream));
@@ -1136,7 +1201,7 @@ int ammsb_run(ammsb_handle* h, double* last) {
   };
   // the timers (cc:95-102) start from zero and time this run
   for (auto& t : h->timers) t = ammsb_handle::Timer{};
-  h->pending.clear();
+  for (int s = 0; s < kMaxRing; ++s) h->upd_pending[s] = h->drw_pending[s] = false;
   {
     int rc = count_node_ticks(h);  // node ticks count from here
     if (rc) return rc;
@@ -1153,7 +1218,7 @@ int ammsb_run(ammsb_handle* h, double* last) {
   // the outer timer: wall time of the iterations (perplexity included), one
   // tick per iteration; brought up to date at every stats print
   auto stats = [&]() -> int {
-    int rc = drain_phase_events(h);
+    int rc = read_phase_events(h, 0, h->m.ring);
     if (!rc) rc = count_node_ticks(h);
     if (rc) return rc;
     const auto now = clk::now();
@@ -1267,7 +1332,7 @@ int ammsb_get_last_minibatch(ammsb_handle* h, int32_t* flag, int32_t* n_edges, i
     h->err = "no iteration has run yet";
     return AMMSB_E_STATE;
   }
-  const Buffers& bl = h->bufs[h->last];
+  const Buffers bl = ring_set(h, h->last);
   DevState st;
   DevCounters gc;
   CK(cudaMemcpyAsync(&st, bl.st, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
@@ -1327,16 +1392,14 @@ int ammsb_profile_step(ammsb_handle* h, double* ms5) {
     return AMMSB_E_STATE;
   }
   CK(cudaSetDevice(h->device));
-  int rc0 = invalidate_prefetch(h);
+  invalidate_prefetch(h);
+  int rc0 = point_draws(h, h->step_count, h->stream);
   if (rc0) return rc0;
-  const Buffers& bp = h->bufs[h->slot];
+  const Buffers bp = ring_set(h, h->slot);
   cudaEvent_t ev[6];
   for (auto& e : ev) CK(cudaEventCreate(&e));
-  CK(cudaEventRecord(ev[0], h->stream));
-  k_sample_minibatch<<<1, 1024, h->mb_smem, h->stream>>>(h->m, h->g, bp, h->mb_smem > 0);
-  CK(cudaEventRecord(ev[1], h->stream));
-  k_sample_neighbors<8><<<h->nbr_blocks, 256, h->nbr_smem, h->stream>>>(h->m, h->g, bp);
-  CK(cudaEventRecord(ev[2], h->stream));
+  CK(launch_sampling_phase(h, h->slot, 1, h->stream, ev));
+  ++h->dev_next;
   CK(h->opt.pi_dtype == AMMSB_PI_BF16 ? launch_phi<__nv_bfloat16>(h, bp) : launch_phi<float>(h, bp));
   CK(cudaEventRecord(ev[3], h->stream));
   CK(h->opt.pi_dtype == AMMSB_PI_BF16 ? launch_commit<__nv_bfloat16>(h, bp) : launch_commit<float>(h, bp));
@@ -1419,12 +1482,7 @@ int apply_phi_cfg(ammsb_handle* h, const KernelCfg& c) {
       return AMMSB_E_CUDA;
     }
   }
-  for (auto* gs : {h->graph1, h->graph2, h->graph1t, h->graph2t, h->graphL})  // the captured iterations used the old kernels
-    for (int i = 0; i < kRing; ++i)
-      if (gs[i]) {
-        cudaGraphExecDestroy(gs[i]);
-        gs[i] = nullptr;
-      }
+  drop_graphs(h);  // the captured iterations used the old kernels
   return AMMSB_OK;
 }
 
@@ -1449,11 +1507,13 @@ int ammsb_autotune(ammsb_handle* h, int32_t reps, int32_t flags) {
   // a non-link minibatch and its neighbour sets into buffer set 0
   Model mt = h->m;
   mt.strategy = AMMSB_STRATIFIED_RANDOM_NODE_NONLINKS;
-  const Buffers& b0 = h->bufs[0];
-  k_sample_minibatch<<<1, 1024, h->mb_smem, h->stream>>>(mt, h->g, b0, h->mb_smem > 0);
+  invalidate_prefetch(h);
+  const Buffers b0 = ring_set(h, 0);
+  k_sample_minibatch<<<1, 1024, h->mb_smem, h->stream>>>(mt, h->g, h->b, 0, h->mb_smem > 0);
   CK(cudaGetLastError());
-  k_sample_neighbors<8><<<h->nbr_blocks, 256, h->nbr_smem, h->stream>>>(h->m, h->g, b0);
+  k_sample_neighbors<8><<<dim3(h->nbr_blocks, 1), 256, h->nbr_smem, h->stream>>>(h->m, h->g, h->b, 0);
   CK(cudaGetLastError());
+  ++h->dev_next;
   float* scratch = nullptr;
   const size_t phi_bytes = sizeof(float) * (size_t)h->m.N * h->m.Kp;
   CK(cudaMalloc(&scratch, phi_bytes));
@@ -1500,16 +1560,15 @@ int ammsb_autotune(ammsb_handle* h, int32_t reps, int32_t flags) {
     rc = AMMSB_E_CUDA;
   }
   // the tuning draws are not an iteration: the next draw is step_count's
-  const uint32_t s = (uint32_t)h->step_count;
-  CK(cudaMemcpyAsync(&h->gc->next_step, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
-  h->ahead = 0;
+  const int rc1 = point_draws(h, h->step_count, h->stream);
   h->slot = 0;
   h->last = -1;
   int rc2 = apply_phi_cfg(h, best);
   CK(cudaStreamSynchronize(h->stream));
   if (rc) return rc;
+  if (rc1) return rc1;
   if (rc2) return rc2;
-  rc = ammsb_detail::check_device_err(h);
+  rc = check_draw_err(h, 0);
   if (rc) return rc;
   std::lock_guard<std::mutex> lock(g_tune_mu);
   g_tune_cache[key] = best;
@@ -1596,14 +1655,15 @@ int ammsb_shard_draw(ammsb_handle* h) {
   CK(cudaSetDevice(h->device));
   int rc = shard_buffers(h);
   if (rc) return rc;
-  h->ahead = 0;  // nothing drawn ahead survives: the draw is for step_count
-  const uint32_t s = (uint32_t)h->step_count;
-  CK(cudaMemcpyAsync(&h->gc->next_step, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
-  CK(launch_sampling_phase(h, h->bufs[h->slot], h->stream));
+  invalidate_prefetch(h);  // nothing drawn ahead survives: the draw is for step_count
+  rc = point_draws(h, h->step_count, h->stream);
+  if (rc) return rc;
+  CK(launch_sampling_phase(h, h->slot, 1, h->stream));
+  ++h->dev_next;
   h->shard_drawn = h->slot;
   h->last = h->slot;
   h->shard_phase = 1;
-  return check_device_err(h);
+  return check_draw_err(h, h->slot);
 }
 
 int ammsb_shard_update(ammsb_handle* h, int32_t n_owned, const int32_t* slots, float* rows_out) {
@@ -1613,7 +1673,7 @@ int ammsb_shard_update(ammsb_handle* h, int32_t n_owned, const int32_t* slots, f
     return AMMSB_E_STATE;
   }
   CK(cudaSetDevice(h->device));
-  const Buffers& D = h->bufs[h->shard_drawn];
+  const Buffers D = ring_set(h, h->shard_drawn);
   int rc = AMMSB_OK;
   DevState st = read_state(h, D, &rc);
   if (rc) return rc;
@@ -1627,7 +1687,7 @@ int ammsb_shard_update(ammsb_handle* h, int32_t n_owned, const int32_t* slots, f
   if (n_owned == 0) return AMMSB_OK;
   // the owned nodes and their neighbour sets, compacted into the next
   // buffer set, then update_phi of those alone
-  const Buffers& W = h->bufs[(h->shard_drawn + 1) % kRing];
+  const Buffers W = ring_set(h, (h->shard_drawn + 1) % h->m.ring);
   CK(cudaMemcpyAsync(h->d_shard_idx, slots, sizeof(int32_t) * n_owned, cudaMemcpyHostToDevice, h->stream));
   const int64_t work = (int64_t)n_owned * h->m.n_out;
   k_shard_gather_nodes<<<(int)std::min<int64_t>((work + 255) / 256, 152 * 8), 256, 0, h->stream>>>(
@@ -1653,7 +1713,7 @@ int ammsb_shard_commit(ammsb_handle* h, const float* rows_all, int32_t n_owned_e
     return AMMSB_E_STATE;
   }
   CK(cudaSetDevice(h->device));
-  const Buffers& D = h->bufs[h->shard_drawn];
+  const Buffers D = ring_set(h, h->shard_drawn);
   int rc = AMMSB_OK;
   DevState st = read_state(h, D, &rc);
   if (rc) return rc;
@@ -1667,7 +1727,7 @@ int ammsb_shard_commit(ammsb_handle* h, const float* rows_all, int32_t n_owned_e
   // every row and the beta partials of the owned edges
   CK(cudaMemcpy2DAsync(h->b.stage, sizeof(float) * h->m.Kp, rows_all, sizeof(float) * h->m.K,
                        sizeof(float) * h->m.K, st.n_nodes, cudaMemcpyHostToDevice, h->stream));
-  const Buffers& W = h->bufs[(h->shard_drawn + 1) % kRing];
+  const Buffers W = ring_set(h, (h->shard_drawn + 1) % h->m.ring);
   if (n_owned_edges > 0)
     CK(cudaMemcpyAsync(h->d_shard_idx, edge_idx, sizeof(int32_t) * n_owned_edges, cudaMemcpyHostToDevice,
                        h->stream));
@@ -1694,18 +1754,16 @@ int ammsb_shard_theta(ammsb_handle* h, const double* R_total) {
     return AMMSB_E_STATE;
   }
   CK(cudaSetDevice(h->device));
-  const Buffers& D = h->bufs[h->shard_drawn];
+  const Buffers D = ring_set(h, h->shard_drawn);
   CK(cudaMemcpyAsync(h->d_shard_R, R_total, sizeof(double) * 2 * h->m.K, cudaMemcpyHostToDevice, h->stream));
   k_theta_given<<<(h->m.K + 31) / 32, 1024, 0, h->stream>>>(h->m, D, h->d_shard_R);
   CK(cudaGetLastError());
   h->last = h->shard_drawn;
-  h->slot = (h->shard_drawn + 1) % kRing;
+  h->slot = (h->shard_drawn + 1) % h->m.ring;
   h->step_count += 1;
   h->shard_phase = 0;
   h->shard_drawn = -1;
-  h->ahead = 0;
-  const uint32_t s = (uint32_t)h->step_count;
-  CK(cudaMemcpyAsync(&h->gc->next_step, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
+  invalidate_prefetch(h);
   return check_device_err(h);
 }
 
@@ -1900,8 +1958,7 @@ int ammsb_load_checkpoint(ammsb_handle* h, const char* path) {
   h->step_count = hd.step_count;
   h->average_count = hd.average_count;
   h->ppx_history = hist;
-  const uint32_t s = (uint32_t)hd.step_count;
-  CK(cudaMemcpyAsync(&h->gc->next_step, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
+  if ((rc = point_draws(h, hd.step_count, h->stream))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   h->state_ready = true;
   return AMMSB_OK;

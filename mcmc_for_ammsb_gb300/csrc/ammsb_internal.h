@@ -14,7 +14,15 @@
 
 using namespace ammsb;
 
-constexpr int kRing = 4;  // minibatch buffer sets per handle
+// The draws of an iteration depend on its step alone, so a launch draws a
+// block of iterations at once (ammsb_handle::block of them, a CTA of the minibatch kernel
+// and a slice of the neighbour kernel's grid each) while the other block's
+// iterations update the state; the ring holds both blocks' buffer sets.
+constexpr int kMaxBlock = 16;
+constexpr int kMaxRing = 2 * kMaxBlock;
+// A ring of at most this many bytes takes the full block; larger buffer sets
+// (random-edge over the whole training set) take blocks of two.
+constexpr int64_t kRingBytes = 1ll << 30;
 
 // Launches of the iteration that may start before the kernel ahead of them
 // has finished (programmatic dependent launch): update_phi after the
@@ -29,7 +37,6 @@ struct KernelCfg {
   int ring_few;              // a 16-warp variant takes iterations of few nodes
   int ring_grid;             // CTAs of the many-node ring launch (0: one per node slot)
   int pdl;                   // programmatic dependent launches: kPdl* bits
-  int graph_pairs;           // pairs of iterations per long graph launch (<= 1: none)
   int ppx_lpn, ppx_vpl;      // perplexity
   int kq;                    // commit_beta
 };
@@ -42,11 +49,16 @@ struct ammsb_handle {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   Model m{};
   DevGraph g{};
-  Buffers b{};        // shared state pointers (bufs[s] add the minibatch buffers)
-  Buffers bufs[kRing]{};  // ring of minibatch buffer sets (draws run two iterations ahead)
+  Buffers b{};        // buffer set 0 and the shared state (slot_buffers gives the other sets)
   DevCounters* gc = nullptr;
+  int block = 8;  // iterations per draws launch (half the ring)
   int slot = 0;   // ring slot of the next iteration
-  int ahead = 0;  // iterations from `slot` on whose draws are made or queued (0..2)
+  // iterations from `slot` on whose draws are made or queued: none, or the
+  // rest of slot's block and, past the block's first iteration, the other
+  // block too
+  int ahead = 0;
+  uint32_t dev_next = 1;    // gc->next_step once the queued work is done
+  uint64_t ring_gen = 0;    // raised whenever the ring's draws change hands
   int last = -1;            // buffer set of the last applied iteration
   KernelCfg cfg{};
   int64_t E = 0, H = 0, T = 0;
@@ -71,10 +83,12 @@ struct ammsb_handle {
   uint64_t average_count = 1;  // learner.cc:30
   std::vector<double> ppx_history;
   bool state_ready = false;
-  // captured iterations per ring slot: one iteration, and two iterations
-  // with the draws of the following two made alongside
-  cudaGraphExec_t graph1[kRing] = {}, graph2[kRing] = {};
-  cudaGraphExec_t graphL[kRing] = {};  // cfg.graph_pairs pipelined pairs of iterations in one launch
+  // captured iterations: whole blocks with the other block's draws made
+  // alongside (one block, and both in turn), runs of 1, 2, 4, 8 updates inside
+  // a block, and single iterations in the loop's order (pipeline off)
+  cudaGraphExec_t graphB[2] = {}, graphL[2] = {};
+  cudaGraphExec_t graphU[kMaxRing][4] = {};
+  cudaGraphExec_t graphS[kMaxRing] = {};
   // run()'s per-phase timers (mcmc_sampler_stochastic.cc:93-102), printed
   // as PrintStats does (cc:185-198): wall time and ticks per timer
   struct Timer {
@@ -84,15 +98,13 @@ struct ammsb_handle {
   enum { kTOuter, kTPerplexity, kTMiniBatch, kTNodes, kTNeighbors, kTPhi, kTPi, kTBeta, kTimers };
   Timer timers[kTimers];
   bool timing = false;  // run() launches the timed captures below
-  // the same iterations with CUDA events between the phases: per launch of
-  // n iterations, 1 + 3n events on the update stream, then 1 + 2n on the
-  // draws' stream; one event set per (n, slot)
-  cudaGraphExec_t graph1t[kRing] = {}, graph2t[kRing] = {};
-  cudaEvent_t ev_phase[2][kRing][12] = {};
-  struct Pending {
-    int n, s;
-  };
-  std::vector<Pending> pending;  // timed launches whose events are not read yet
+  // the same with CUDA events between the phases: an event set per buffer
+  // set for its update (before it and after each of its three phases), and
+  // one for the draws launch that starts there (before it and after each of
+  // its two kernels)
+  cudaGraphExec_t graphBt[2] = {}, graphUt[kMaxRing] = {}, graphSt[kMaxRing] = {};
+  cudaEvent_t ev_upd[kMaxRing][4] = {}, ev_drw[kMaxRing][3] = {};
+  bool upd_pending[kMaxRing] = {}, drw_pending[kMaxRing] = {};  // event sets not read yet
   uint64_t evals_read = 0;       // edge evaluations counted into the timers' ticks
   // a sharded iteration in progress (ammsb_shard_*): the drawn buffer set
   // and the device arrays of its phases
@@ -151,6 +163,9 @@ cudaError_t raise_smem_limit(F* kernel, size_t bytes) {
 
 // Reads the device error word of a handle (synchronises its stream).
 int check_device_err(ammsb_handle* h);
-// Drops draws made ahead of time and points the next draw at step_count.
-int invalidate_prefetch(ammsb_handle* h);
+// Drops draws made ahead of time: the next ones start from step_count.
+void invalidate_prefetch(ammsb_handle* h);
+// Points the device's next draws at `step` on stream s, unless queued work
+// leaves it there.
+int point_draws(ammsb_handle* h, uint64_t step, cudaStream_t s);
 }  // namespace ammsb_detail

@@ -47,6 +47,11 @@ struct Model {
   int32_t max_source;   // sampler.max-source (link stratum)
   int32_t full_set;     // random-edge: the minibatch is the whole training set
   int64_t n_entries;    // 2E: entries of the symmetric CSR
+  // the ring of minibatch buffer sets: element strides between consecutive
+  // sets (set s of Buffers::nodes starts at s * slot_nodes, and so on), and
+  // between the scratch areas of a draws launch's iterations
+  int32_t ring;         // buffer sets
+  int64_t slot_nodes, slot_edges, slot_nbr, slot_cand;
 };
 
 struct Buffers {
@@ -71,13 +76,32 @@ struct Buffers {
   DevCounters* gc;     // sampler-wide counters
 };
 
+// Buffer set `slot` of the ring whose set 0 is b0, with scratch area j (a
+// draws launch gives each of its iterations an area of its own).
+__host__ __device__ __forceinline__ Buffers slot_buffers(const Model& m, const Buffers& b0, int slot,
+                                                         int j = 0) {
+  Buffers b = b0;
+  b.nodes += slot * m.slot_nodes;
+  b.ea += slot * m.slot_edges;
+  b.eb += slot * m.slot_edges;
+  b.ey += slot * m.slot_edges;
+  b.nbr += slot * m.slot_nbr;
+  b.st += slot;
+  b.cand += j * m.slot_cand;
+  if (b.htab_key) {
+    b.htab_key += (int64_t)j * ((int64_t)b.hmask + 1);
+    b.htab_idx += (int64_t)j * ((int64_t)b.hmask + 1);
+  }
+  return b;
+}
+
 // One chain of a multi-chain launch (blockIdx.y selects the chain): its
-// model, graph and both buffer sets, plus the per-chain launch parameters
-// of the single-chain kernels.
+// model, graph and buffer set 0 of its ring, plus the per-chain launch
+// parameters of the single-chain kernels.
 struct ChainArgs {
   Model m;
   DevGraph g;
-  Buffers b[2];
+  Buffers b;
   int32_t ncommit;    // k_commit_beta: blocks of the commit part
   int32_t smem_hash;  // k_sample_minibatch: the dedup hash fits shared memory
 };
@@ -251,7 +275,10 @@ static __device__ int assign_node_slots(const Buffers& b, int count, int max_nod
 }
 
 // ---------------------------------------------------------------------------
-// k_sample_minibatch: one 1024-thread CTA.  Stratified random node
+// k_sample_minibatch: one 1024-thread CTA per iteration drawn (CTA j draws
+// iteration next_step + j into buffer set (s0 + j) % ring; the draws depend on
+// the step alone, so a launch takes as many iterations as half the ring
+// holds).  Stratified random node
 // (network.cc:410-421): flag = randint(0,1); non-link stratum
 // (network.cc:274-349): source v and the first m valid new partners u in
 // candidate order (u != v, (v,u) not an edge, not held-out, not test); link
@@ -262,7 +289,7 @@ static __device__ int assign_node_slots(const Buffers& b, int count, int max_nod
 // them -- exactly the sequential scan of the oracle.
 // ---------------------------------------------------------------------------
 static __device__ __forceinline__ void sample_minibatch_body(const Model& m, const DevGraph& g,
-                                                             const Buffers& b, int smem_hash) {
+                                                             const Buffers& b, int j, int smem_hash) {
   extern __shared__ uint32_t s_htab[];  // dedup hash in shared memory when it fits
   constexpr int kRowCap = 2048;         // the source's row, staged when it fits
   __shared__ int32_t s_row[kRowCap];
@@ -274,9 +301,8 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
   const int tid = threadIdx.x;
   const Stream rs{m.seed, m.chain};
   if (tid == 0) {
-    const uint32_t step = b.gc->next_step;
+    const uint32_t step = b.gc->next_step + (uint32_t)j;
     b.st->step = step;
-    b.gc->next_step = step + 1;
     int flag;
     if (m.strategy == 0)
       flag = (int)uniform_below(rs.draw_u64(kTagMbFlag, 0, step, 0), 2ull);
@@ -640,28 +666,32 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
     b.st->n_edges = err ? 0 : s_count;
     b.st->n_nodes = err ? 0 : s_nodes;
     b.st->rounds = rounds;
-    if (err) atomicOr(&b.gc->err, err);
+    b.st->err = err;
   }
 }
-static __global__ void __launch_bounds__(1024) k_sample_minibatch(Model m, DevGraph g, Buffers b,
+static __global__ void __launch_bounds__(1024) k_sample_minibatch(Model m, DevGraph g, Buffers b0, int s0,
                                                                   int smem_hash) {
-  sample_minibatch_body(m, g, b, smem_hash);
+  const int j = blockIdx.x;
+  sample_minibatch_body(m, g, slot_buffers(m, b0, (s0 + j) % m.ring, j), j, smem_hash);
 }
-// one CTA per chain (blockIdx.y), buffer set p
+// a CTA per iteration (blockIdx.x) and chain (blockIdx.y)
 static __global__ void __launch_bounds__(1024) k_sample_minibatch_chains(const ChainArgs* __restrict__ c,
-                                                                         int p) {
+                                                                         int s0) {
   const ChainArgs& a = c[blockIdx.y];
-  sample_minibatch_body(a.m, a.g, a.b[p], a.smem_hash);
+  const int j = blockIdx.x;
+  sample_minibatch_body(a.m, a.g, slot_buffers(a.m, a.b, s0 + j, j), j, a.smem_hash);
 }
 
 // ---------------------------------------------------------------------------
-// k_sample_neighbors: one warp per minibatch node.  n_out distinct ids j,
+// k_sample_neighbors: one warp per minibatch node of iteration j of a draws
+// launch (the grid's last dimension).  n_out distinct ids j,
 // j != i, (i,j) neither held-out nor test (h:87-108); 32 candidates per
 // round, the first valid new ones in candidate order are kept; y_ij is the
 // graph membership the update needs (cc:279-283).
 // ---------------------------------------------------------------------------
 template <int WARPS>
-__device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevGraph& g, const Buffers& b) {
+__device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevGraph& g, const Buffers& b,
+                                                      int j0, int count0) {
   // per warp: a set of the ids accepted so far (open addressing, capacity a
   // power of two >= 2 n_out, -1 empty) in dynamic shared memory
   extern __shared__ int32_t s_sets[];
@@ -680,8 +710,12 @@ __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevG
   // without a node (the grid has a warp more than the nodes) and which no
   // other warp waits for; in the single-CTA minibatch kernel its latency
   // delayed every block barrier (2.8 us of each minibatch)
-  if (blockIdx.x == gridDim.x - 1 && warp == WARPS - 1 && lane == 0)
+  if (blockIdx.x == gridDim.x - 1 && warp == WARPS - 1 && lane == 0) {
     b.st->eps = eps_schedule(m.a, m.b, m.c, step);
+    // iteration 0 of the launch moves the counter past its `count0`
+    // iterations: the minibatch launch ahead has read it, nothing here does
+    if (j0 == 0) b.gc->next_step = step + (uint32_t)count0;
+  }
   for (int slot = blockIdx.x * WARPS + warp; slot < n_nodes; slot += gridDim.x * WARPS) {
     const int32_t i = b.nodes[slot];
     const int64_t ir0 = g.row_ptr[i];
@@ -695,7 +729,7 @@ __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevG
     uint64_t t = 0;
     while (count < m.n_out) {
       if (t >= cap) {
-        if (lane == 0) atomicOr(&b.gc->err, kErrNeighborCap);
+        if (lane == 0) atomicOr(&b.st->err, kErrNeighborCap);
         break;
       }
       const int32_t j = (int32_t)uniform_below(rs.draw_u64(kTagNbr, (uint32_t)i, step, t + lane),
@@ -740,14 +774,16 @@ __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevG
   }
 }
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) k_sample_neighbors(Model m, DevGraph g, Buffers b) {
-  sample_neighbors_body<WARPS>(m, g, b);
+__global__ void __launch_bounds__(WARPS * 32) k_sample_neighbors(Model m, DevGraph g, Buffers b0, int s0) {
+  const int j = blockIdx.y;
+  sample_neighbors_body<WARPS>(m, g, slot_buffers(m, b0, (s0 + j) % m.ring), j, (int)gridDim.y);
 }
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_sample_neighbors_chains(const ChainArgs* __restrict__ c,
-                                                                      int p) {
+                                                                      int s0) {
   const ChainArgs& a = c[blockIdx.y];
-  sample_neighbors_body<WARPS>(a.m, a.g, a.b[p]);
+  const int j = blockIdx.z;
+  sample_neighbors_body<WARPS>(a.m, a.g, slot_buffers(a.m, a.b, s0 + j), j, (int)gridDim.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -962,7 +998,7 @@ template <typename PiT, int LPN, int VPL, int SPLIT, int NPB>
 __global__ void __launch_bounds__(NPB * SPLIT * LPN) k_update_phi_chains(const ChainArgs* __restrict__ c,
                                                                          int p) {
   const ChainArgs& a = c[blockIdx.y];
-  update_phi_body<PiT, LPN, VPL, SPLIT, NPB>(a.m, a.b[p]);
+  update_phi_body<PiT, LPN, VPL, SPLIT, NPB>(a.m, slot_buffers(a.m, a.b, p));
 }
 
 // ---------------------------------------------------------------------------
@@ -1089,7 +1125,7 @@ __global__ void __launch_bounds__(128) k_commit_beta(Model m, Buffers b, int nco
 template <typename PiT, int KQ>
 __global__ void __launch_bounds__(128) k_commit_beta_chains(const ChainArgs* __restrict__ c, int p) {
   const ChainArgs& a = c[blockIdx.y];
-  commit_beta_body<PiT, KQ>(a.m, a.b[p], a.ncommit);
+  commit_beta_body<PiT, KQ>(a.m, slot_buffers(a.m, a.b, p), a.ncommit);
 }
 
 // ---------------------------------------------------------------------------
@@ -1228,7 +1264,8 @@ static __device__ __forceinline__ void theta_body(const Model& m, const Buffers&
     pre.nz0 = s_pre[3][lane];
     pre.nz1 = s_pre[4][lane];
   }
-  if (k == 0) {  // the iteration's edge evaluations, counted once it is applied
+  if (k == 0) {  // the iteration's edge evaluations and errors, counted once it is applied
+    if (b.st->err) atomicOr(&b.gc->err, b.st->err);
     b.gc->evals += (unsigned long long)b.st->n_nodes * (unsigned long long)m.n_out;
     b.gc->iters += 1ull;
   }
@@ -1253,7 +1290,7 @@ static __global__ void __launch_bounds__(1024) k_theta_given(Model m, Buffers b,
 }
 static __global__ void __launch_bounds__(1024) k_theta_chains(const ChainArgs* __restrict__ c, int p) {
   const ChainArgs& a = c[blockIdx.y];
-  theta_body(a.m, a.b[p]);
+  theta_body(a.m, slot_buffers(a.m, a.b, p));
 }
 
 // ---------------------------------------------------------------------------

@@ -550,9 +550,10 @@ template <typename PiT, int VPL, int SPLIT, int STAGES, bool FULL>
 __global__ void __launch_bounds__(SPLIT * 32, ring_min_blocks<SPLIT>())
     k_update_phi_ring_chains(const ChainArgs* __restrict__ c, int p, int n_lo, int n_hi) {
   const ChainArgs& a = c[blockIdx.y];
-  const int n_nodes = a.b[p].st->n_nodes;
+  const Buffers b = slot_buffers(a.m, a.b, p);
+  const int n_nodes = b.st->n_nodes;
   if (n_nodes <= n_lo || n_nodes > n_hi) return;
-  update_phi_ring_body<PiT, VPL, SPLIT, STAGES, FULL>(a.m, a.b[p]);
+  update_phi_ring_body<PiT, VPL, SPLIT, STAGES, FULL>(a.m, b);
 }
 
 }  // namespace ammsb
