@@ -40,9 +40,11 @@ struct PhiGroup {
 
 struct CommitGroup {
   int dtype, kq;
+  int chunk;  // k_commit_star's edges per summing warp at once; 0: k_commit_beta
   std::vector<int> chains;
   ChainArgs* d = nullptr;
   int gx = 1;
+  size_t smem = 0;
 };
 
 constexpr int kRingSplitB = 4;
@@ -122,17 +124,29 @@ cudaError_t phi_chains(const PhiGroup& g, int p, cudaStream_t st, bool configure
   return cudaErrorInvalidConfiguration;
 }
 
-template <typename PiT>
-cudaError_t commit_chains(const CommitGroup& g, int p, cudaStream_t st) {
+template <typename PiT, int KQ>
+cudaError_t commit_chains_k(const CommitGroup& g, int p, cudaStream_t st, bool configure) {
   const dim3 grid(g.gx, (unsigned)g.chains.size());
+  auto go = [&](auto* kern, int threads) -> cudaError_t {
+    if (configure) return ammsb_detail::raise_smem_limit(kern, g.smem);
+    kern<<<grid, threads, g.smem, st>>>(g.d, p);
+    return cudaGetLastError();
+  };
+  switch (g.chunk) {
+    case 0: return go(k_commit_beta_chains<PiT, KQ>, 128);
+    case 1: return go(k_commit_star_chains<PiT, KQ, 1>, 128);
+    default: return go(k_commit_star_chains<PiT, KQ, kStarChunk>, 128 * kStarChunk);
+  }
+}
+template <typename PiT>
+cudaError_t commit_chains(const CommitGroup& g, int p, cudaStream_t st, bool configure) {
   switch (g.kq) {
-    case 1: k_commit_beta_chains<PiT, 1><<<grid, 128, 0, st>>>(g.d, p); break;
-    case 2: k_commit_beta_chains<PiT, 2><<<grid, 128, 0, st>>>(g.d, p); break;
-    case 4: k_commit_beta_chains<PiT, 4><<<grid, 128, 0, st>>>(g.d, p); break;
-    case 8: k_commit_beta_chains<PiT, 8><<<grid, 128, 0, st>>>(g.d, p); break;
+    case 1: return commit_chains_k<PiT, 1>(g, p, st, configure);
+    case 2: return commit_chains_k<PiT, 2>(g, p, st, configure);
+    case 4: return commit_chains_k<PiT, 4>(g, p, st, configure);
+    case 8: return commit_chains_k<PiT, 8>(g, p, st, configure);
     default: return cudaErrorInvalidConfiguration;
   }
-  return cudaGetLastError();
 }
 
 }  // namespace
@@ -196,11 +210,11 @@ cudaError_t launch_update_chains(ammsb_batch* bt, int p) {
   for (size_t gi = 1; gi < ng; ++gi)
     if ((e = cudaStreamWaitEvent(bt->stream, bt->gevent[gi - 1], 0)) != cudaSuccess) return e;
   for (const CommitGroup& g : bt->commit) {
-    cudaError_t e = (g.dtype == AMMSB_PI_BF16) ? commit_chains<__nv_bfloat16>(g, p, bt->stream)
-                                               : commit_chains<float>(g, p, bt->stream);
+    cudaError_t e = (g.dtype == AMMSB_PI_BF16) ? commit_chains<__nv_bfloat16>(g, p, bt->stream, false)
+                                               : commit_chains<float>(g, p, bt->stream, false);
     if (e != cudaSuccess) return e;
   }
-  k_theta_chains<<<dim3(bt->theta_gx, (unsigned)bt->h.size()), 1024, 0, bt->stream>>>(bt->d_all, p);
+  k_theta_chains<<<dim3(bt->theta_gx, (unsigned)bt->h.size()), kThetaThreads, 0, bt->stream>>>(bt->d_all, p);
   return cudaGetLastError();
 }
 
@@ -348,6 +362,7 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     a.b = h->b;
     bt->block = std::min(bt->block, h->block);
     a.ncommit = h->ncommit;
+    a.star = h->star ? 1 : 0;
     a.smem_hash = h->mb_smem > 0 ? 1 : 0;
     bt->mb_smem = std::max(bt->mb_smem, h->mb_smem);
     bt->nbr_smem = std::max(bt->nbr_smem, h->nbr_smem);
@@ -360,7 +375,7 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
   }
   // group the update_phi launches by compiled shape, the commits by K-tile
   std::map<std::tuple<int, int, int, int, int, int, int>, int> pg;
-  std::map<std::pair<int, int>, int> cg;
+  std::map<std::tuple<int, int, int>, int> cg;
   for (int i = 0; i < n; ++i) {
     ammsb_handle* h = bt->h[i];
     const KernelCfg& c = h->cfg;
@@ -390,18 +405,22 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
                            npb * std::max(1, c.split * c.lpn / 32)) * sizeof(float);
       g.smem = std::max(g.smem, smem);
     }
-    auto ck = std::make_pair((int)h->opt.pi_dtype, c.kq);
+    const int chunk = h->star ? star_chunk(h->m) : 0;
+    auto ck = std::make_tuple((int)h->opt.pi_dtype, c.kq, chunk);
     auto jt = cg.find(ck);
     if (jt == cg.end()) {
       CommitGroup g2;
       g2.dtype = h->opt.pi_dtype;
       g2.kq = c.kq;
+      g2.chunk = chunk;
       jt = cg.emplace(ck, (int)bt->commit.size()).first;
       bt->commit.push_back(g2);
     }
     CommitGroup& g2 = bt->commit[jt->second];
     g2.chains.push_back(i);
-    g2.gx = std::max(g2.gx, h->ncommit + h->m.nbb);
+    g2.gx = std::max(g2.gx, (chunk ? 0 : h->ncommit) + h->m.nbb + (h->m.K + 31) / 32);
+    if (chunk)
+      g2.smem = std::max(g2.smem, chunk == 1 ? commit_star_smem<1>(h->m.Kp) : commit_star_smem<kStarChunk>(h->m.Kp));
   }
   for (PhiGroup& g : bt->phi) {
     std::vector<ChainArgs> a;
@@ -440,6 +459,12 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     for (int i : g.chains) a.push_back(args[i]);
     if (dev_upload(bt, &g.d, a) != cudaSuccess) {
       bt->err = "upload of a group table failed";
+      return bail(AMMSB_E_CUDA);
+    }
+    cudaError_t e = (g.dtype == AMMSB_PI_BF16) ? commit_chains<__nv_bfloat16>(g, 0, bt->stream, true)
+                                               : commit_chains<float>(g, 0, bt->stream, true);
+    if (e != cudaSuccess) {
+      bt->err = std::string("commit group configuration: ") + cudaGetErrorString(e);
       return bail(AMMSB_E_CUDA);
     }
   }

@@ -189,7 +189,7 @@ cudaError_t launch_phi(ammsb_handle* h, const Buffers& b, bool pdl = false) {
 // `pdl`: as a programmatic dependent launch after update_phi
 template <typename PiT>
 cudaError_t launch_commit(ammsb_handle* h, const Buffers& b, bool pdl = false) {
-  const int grid = h->ncommit + h->m.nbb;
+  const int grid = h->ncommit + h->m.nbb + (h->m.K + 31) / 32;  // ... and theta_pre_block's
   switch (h->cfg.kq) {
     case 1: return launch_k(k_commit_beta<PiT, 1>, grid, 128, 0, h->stream, pdl, h->m, b, h->ncommit);
     case 2: return launch_k(k_commit_beta<PiT, 2>, grid, 128, 0, h->stream, pdl, h->m, b, h->ncommit);
@@ -227,6 +227,34 @@ cudaError_t launch_normalize(ammsb_handle* h) {
   return cudaGetLastError();
 }
 
+template <typename PiT, int KQ>
+cudaError_t launch_star_k(ammsb_handle* h, const Buffers& b, bool configure, bool pdl) {
+  auto go = [&](auto* kern, int threads, size_t smem) {
+    if (configure) return ammsb_detail::raise_smem_limit(kern, smem);
+    return launch_k(kern, h->m.nbb + (h->m.K + 31) / 32, threads, smem, h->stream, pdl, h->m, b);
+  };
+  return star_chunk(h->m) == 1
+             ? go(k_commit_star<PiT, KQ, 1>, 128, commit_star_smem<1>(h->m.Kp))
+             : go(k_commit_star<PiT, KQ, kStarChunk>, 128 * kStarChunk, commit_star_smem<kStarChunk>(h->m.Kp));
+}
+template <typename PiT>
+cudaError_t launch_star(ammsb_handle* h, const Buffers& b, bool configure, bool pdl = false) {
+  switch (h->cfg.kq) {
+    case 1: return launch_star_k<PiT, 1>(h, b, configure, pdl);
+    case 2: return launch_star_k<PiT, 2>(h, b, configure, pdl);
+    case 4: return launch_star_k<PiT, 4>(h, b, configure, pdl);
+    case 8: return launch_star_k<PiT, 8>(h, b, configure, pdl);
+    default: return cudaErrorInvalidConfiguration;
+  }
+}
+
+// The commit of a minibatch, `star` if it is one.
+cudaError_t launch_commits(ammsb_handle* h, const Buffers& b, bool star, bool pdl = false) {
+  if (h->opt.pi_dtype == AMMSB_PI_BF16)
+    return star ? launch_star<__nv_bfloat16>(h, b, false, pdl) : launch_commit<__nv_bfloat16>(h, b, pdl);
+  return star ? launch_star<float>(h, b, false, pdl) : launch_commit<float>(h, b, pdl);
+}
+
 // Records `ev` on `s` when timing (ev != nullptr).  Inside a stream
 // capture an external record becomes an event-record node of the graph, so
 // the event is recorded every time the graph runs (a plain record would only
@@ -247,16 +275,16 @@ inline cudaError_t mark(cudaEvent_t ev, cudaStream_t s) {
 // theta step start as programmatic dependent launches (cfg.pdl).  `pdl`:
 // the previous iteration's theta step is the kernel ahead in the stream and
 // this iteration's draws are complete (update_phi may then start early).
-cudaError_t launch_update_phase(ammsb_handle* h, const Buffers& b, const cudaEvent_t* ev = nullptr,
+// `star`: the minibatch is one.
+cudaError_t launch_update_phase(ammsb_handle* h, const Buffers& b, bool star, const cudaEvent_t* ev = nullptr,
                                 bool pdl = false) {
   const int early = ev ? 0 : h->cfg.pdl;
   cudaError_t e = (h->opt.pi_dtype == AMMSB_PI_BF16) ? launch_phi<__nv_bfloat16>(h, b, pdl)
                                                       : launch_phi<float>(h, b, pdl);
   if (e != cudaSuccess || (e = mark(ev ? ev[0] : nullptr, h->stream)) != cudaSuccess) return e;
-  e = (h->opt.pi_dtype == AMMSB_PI_BF16) ? launch_commit<__nv_bfloat16>(h, b, early & kPdlCommit)
-                                          : launch_commit<float>(h, b, early & kPdlCommit);
+  e = launch_commits(h, b, star, early & kPdlCommit);
   if (e != cudaSuccess || (e = mark(ev ? ev[1] : nullptr, h->stream)) != cudaSuccess) return e;
-  e = launch_k(k_theta, (h->m.K + 31) / 32, 1024, 0, h->stream, early & kPdlTheta, h->m, b);
+  e = launch_k(k_theta, (h->m.K + 31) / 32, kThetaThreads, 0, h->stream, early & kPdlTheta, h->m, b, (int)star);
   if (e != cudaSuccess) return e;
   return mark(ev ? ev[2] : nullptr, h->stream);
 }
@@ -289,7 +317,7 @@ cudaError_t launch_updates(ammsb_handle* h, int s, int count, bool timed, bool f
     // an update after another follows its theta step directly (its draws
     // were joined before this launch)
     if (e == cudaSuccess)
-      e = launch_update_phase(h, ring_set(h, (s + i) % h->m.ring), ev ? ev + 1 : nullptr,
+      e = launch_update_phase(h, ring_set(h, (s + i) % h->m.ring), h->star, ev ? ev + 1 : nullptr,
                               (i > 0 || first_pdl) && !ev);
   }
   return e;
@@ -512,10 +540,11 @@ void choose_config(ammsb_handle* h) {
     sms = 152;
   c.ring_grid = 16 * sms;
   if (const char* env = std::getenv("AMMSB_PHI_GRID")) c.ring_grid = std::max(0, std::atoi(env));
-  // early starts of update_phi after theta and of theta after the commit:
-  // 1.7% less time per BF16 iteration on the 4M-node workload (1.6% on the
-  // 100k-node one); the commit's early start measured no gain
-  c.pdl = kPdlPhi | kPdlTheta;
+  // early starts of all three: of update_phi and theta 1.7% less time per
+  // BF16 iteration on the 4M-node workload; of the commit, whose
+  // theta_pre_block then runs under update_phi, a 100k-node interval of 500
+  // iterations 7.51 to 6.84 ms, a 5k-node one of 100 1.54 to 1.51
+  c.pdl = kPdlPhi | kPdlCommit | kPdlTheta;
   if (const char* env = std::getenv("AMMSB_PDL")) c.pdl = std::atoi(env) & (kPdlPhi | kPdlCommit | kPdlTheta);
   if (const char* env = std::getenv("AMMSB_PHI_KERNEL")) {  // "ring" or "regs"
     if (std::strcmp(env, "regs") == 0) c.ring = 0;
@@ -868,6 +897,7 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
     TRY(dev_alloc(h, &b.htab_idx, (size_t)h->block * hcap));
   }
   TRY(dev_alloc(h, &b.beta_part, (size_t)m.nbb * 2 * Kp));
+  TRY(dev_alloc(h, &b.theta_pre, 5 * (size_t)K));
   TRY(dev_alloc(h, &h->gc, 1));
   b.gc = h->gc;
   TRY(dev_alloc(h, &h->d_err_init, 1));
@@ -888,6 +918,15 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
     if (ammsb_detail::raise_smem_limit(k_sample_neighbors<8>, h->nbr_smem) != cudaSuccess) {
       h->err = "num_node_sample too large for the neighbour kernel";
       return bail(AMMSB_E_ARG);
+    }
+  }
+  h->star = !multi_src && !rand_edge;
+  {
+    cudaError_t e = (o.pi_dtype == AMMSB_PI_BF16) ? launch_star<__nv_bfloat16>(h, h->b, true)
+                                                  : launch_star<float>(h, h->b, true);
+    if (e != cudaSuccess) {
+      h->err = std::string("commit shared memory configuration: ") + cudaGetErrorString(e);
+      return bail(AMMSB_E_CUDA);
     }
   }
   if (h->cfg.ring) {
@@ -1157,7 +1196,10 @@ int ammsb_step_fed(ammsb_handle* h, uint32_t step, int32_t n_edges, const int32_
   Buffers fb = bp;
   fb.fed_phi_noise = h->d_fed_phi_noise;
   fb.fed_theta_noise = h->d_fed_theta_noise;
-  CK(launch_update_phase(h, fb));
+  bool star = n_edges > 0 && n_nodes == n_edges + 1;
+  for (int32_t e = 0; e < n_edges && star; ++e)
+    star = edge_slot_a[e] == 0 && edge_slot_b[e] == e + 1 && !edge_y[e] == !edge_y[0];
+  CK(launch_update_phase(h, fb, star));
   h->last = h->slot;
   return check_device_err(h);
 }
@@ -1402,9 +1444,9 @@ int ammsb_profile_step(ammsb_handle* h, double* ms5) {
   ++h->dev_next;
   CK(h->opt.pi_dtype == AMMSB_PI_BF16 ? launch_phi<__nv_bfloat16>(h, bp) : launch_phi<float>(h, bp));
   CK(cudaEventRecord(ev[3], h->stream));
-  CK(h->opt.pi_dtype == AMMSB_PI_BF16 ? launch_commit<__nv_bfloat16>(h, bp) : launch_commit<float>(h, bp));
+  CK(launch_commits(h, bp, h->star));
   CK(cudaEventRecord(ev[4], h->stream));
-  k_theta<<<(h->m.K + 31) / 32, 1024, 0, h->stream>>>(h->m, bp);
+  k_theta<<<(h->m.K + 31) / 32, kThetaThreads, 0, h->stream>>>(h->m, bp, (int)h->star);
   CK(cudaGetLastError());
   CK(cudaEventRecord(ev[5], h->stream));
   CK(cudaEventSynchronize(ev[5]));
@@ -1738,8 +1780,8 @@ int ammsb_shard_commit(ammsb_handle* h, const float* rows_all, int32_t n_owned_e
   DevState ws = st;
   ws.n_edges = n_owned_edges;
   CK(cudaMemcpyAsync(W.st, &ws, sizeof(ws), cudaMemcpyHostToDevice, h->stream));
-  CK(h->opt.pi_dtype == AMMSB_PI_BF16 ? launch_commit<__nv_bfloat16>(h, W) : launch_commit<float>(h, W));
-  k_beta_sums<<<(h->m.K + 31) / 32, 1024, 0, h->stream>>>(h->m, W, h->d_shard_R);
+  CK(launch_commits(h, W, false));  // any subset of the edges
+  k_beta_sums<<<(h->m.K + 31) / 32, kThetaThreads, 0, h->stream>>>(h->m, W, h->d_shard_R);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(R_out, h->d_shard_R, sizeof(double) * 2 * h->m.K, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -1756,7 +1798,7 @@ int ammsb_shard_theta(ammsb_handle* h, const double* R_total) {
   CK(cudaSetDevice(h->device));
   const Buffers D = ring_set(h, h->shard_drawn);
   CK(cudaMemcpyAsync(h->d_shard_R, R_total, sizeof(double) * 2 * h->m.K, cudaMemcpyHostToDevice, h->stream));
-  k_theta_given<<<(h->m.K + 31) / 32, 1024, 0, h->stream>>>(h->m, D, h->d_shard_R);
+  k_theta_given<<<(h->m.K + 31) / 32, kThetaThreads, 0, h->stream>>>(h->m, D, h->d_shard_R);
   CK(cudaGetLastError());
   h->last = h->shard_drawn;
   h->slot = (h->shard_drawn + 1) % h->m.ring;

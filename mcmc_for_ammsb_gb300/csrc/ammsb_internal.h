@@ -38,8 +38,15 @@ struct KernelCfg {
   int ring_grid;             // CTAs of the many-node ring launch (0: one per node slot)
   int pdl;                   // programmatic dependent launches: kPdl* bits
   int ppx_lpn, ppx_vpl;      // perplexity
-  int kq;                    // commit_beta
+  int kq;                    // commit: 128-element pieces of a row per lane
 };
+
+// The minibatch's shape decides the commit kernel: a star (one source, as the
+// default strategies draw) takes k_commit_star, with kStarChunk edges per
+// summing warp at once where the minibatch gives a warp more than one (4,096
+// edges over 1,024 summing warps) and one where it does not.
+constexpr int kStarChunk = 4;
+inline int star_chunk(const Model& m) { return m.max_edges > 4 * m.nbb ? kStarChunk : 1; }
 
 struct ammsb_handle {
   ammsb_options opt{};
@@ -76,6 +83,7 @@ struct ammsb_handle {
   float* d_fed_theta_noise = nullptr;
   int32_t* d_err_init = nullptr;
   int ncommit = 1;
+  bool star = false;  // drawn minibatches are stars
   int nbr_blocks = 1, phi_blocks = 1;
   size_t phi_smem = 0, phi_smem_wide = 0, nbr_smem = 0, mb_smem = 0;
   // host mirrors

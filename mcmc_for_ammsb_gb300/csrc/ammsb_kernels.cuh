@@ -24,9 +24,10 @@ namespace ammsb {
 #define AMMSB_MAX_BETA_BLOCKS 256
 #endif
 constexpr int kMaxBetaBlocks = AMMSB_MAX_BETA_BLOCKS;
-// k_theta's 31 summing warps read up to 9 partials each in one pass
-constexpr int kThetaSumWarps = 31, kThetaPerPass = 9;
-static_assert(kMaxBetaBlocks <= kThetaSumWarps * kThetaPerPass, "k_theta reads the partials in one pass");
+// k_theta adds the partials in 31 chains of up to 9
+constexpr int kThetaChains = 31, kThetaPerChain = 9;
+static_assert(kMaxBetaBlocks <= kThetaChains * kThetaPerChain, "k_theta reads the partials in one pass");
+constexpr int kThetaThreads = 256;
 
 struct Model {
   int32_t K;      // communities
@@ -70,6 +71,7 @@ struct Buffers {
   uint32_t* htab_idx;
   uint32_t hmask;
   float* beta_part;    // nbb x 2 x Kp
+  double* theta_pre;   // 5 x K: the theta step's parts that do not need the sums
   const float* fed_phi_noise;    // max_nodes x K or null
   const float* fed_theta_noise;  // K x 2 or null
   DevState* st;        // this buffer set's per-iteration scalars
@@ -103,6 +105,7 @@ struct ChainArgs {
   DevGraph g;
   Buffers b;
   int32_t ncommit;    // k_commit_beta: blocks of the commit part
+  int32_t star;       // the commit is k_commit_star (one class of partials)
   int32_t smem_hash;  // k_sample_minibatch: the dedup hash fits shared memory
 };
 
@@ -1010,11 +1013,69 @@ __global__ void __launch_bounds__(NPB * SPLIT * LPN) k_update_phi_chains(const C
 // gradient only needs R_yk = sum_{e: y_e = y} f_ek / P_e (k_theta applies the
 // theta factors), accumulated per warp in registers, then per block.
 // ---------------------------------------------------------------------------
+// ---------------------------------------------------------------------------
+// The parts of k's theta step that do not depend on the sums:
+// 1/(theta0+theta1), the two gradient factors 1/theta_kc - 1/ts, and the two
+// noise terms sqrt(eps theta_kc) n_kc -- three FP64 divisions and two square
+// roots, about 2.5 us at GB300's FP64 rate.  They are formed by blocks of one
+// working warp (32 values of k) beside the commit's own, because nothing of
+// them waits for update_phi: in the theta kernel they were the longest part
+// between the commit's end and the step.
+// ---------------------------------------------------------------------------
+static __device__ __forceinline__ void theta_pre_block(const Model& m, const Buffers& b, int block) {
+  const int k = block * 32 + (int)threadIdx.x;
+  if (threadIdx.x < 32 && k < m.K) {
+    const double eps_t = (double)b.st->eps;
+    const double th0 = b.theta[2 * k], th1 = b.theta[2 * k + 1];
+    const double ts_inv = 1.0 / (th0 + th1);
+    double n0, n1;
+    if (b.fed_theta_noise) {
+      n0 = b.fed_theta_noise[2 * k];
+      n1 = b.fed_theta_noise[2 * k + 1];
+    } else {
+      const Stream rs{m.seed, m.chain};
+      n0 = normal_draw(rs, kTagThetaNoise, 0, b.st->step, 2ull * k);
+      n1 = normal_draw(rs, kTagThetaNoise, 0, b.st->step, 2ull * k + 1);
+    }
+    b.theta_pre[k] = ts_inv;
+    b.theta_pre[m.K + k] = 1.0 / th0 - ts_inv;
+    b.theta_pre[2 * m.K + k] = 1.0 / th1 - ts_inv;
+    b.theta_pre[3 * m.K + k] = sqrt(eps_t * th0) * n0;
+    b.theta_pre[4 * m.K + k] = sqrt(eps_t * th1) * n1;
+  }
+  grid_dependency_wait();
+}
+
+// f_k = pi_ak pi_bk of one lane's 4 elements, added to the lane's sums of f
+// and of w f (w = beta for a link, 1 - beta otherwise); and 1 / P_e from
+// their warp sums.  The roundings are spelled out because k_commit_beta and
+// k_commit_star have to give the same bits.
+__device__ __forceinline__ float4 edge_terms(const float4& xa, const float4& xb, const float4& w, float& fsum,
+                                             float& psum) {
+  const float4 f = make_float4(__fmul_rn(xa.x, xb.x), __fmul_rn(xa.y, xb.y), __fmul_rn(xa.z, xb.z),
+                               __fmul_rn(xa.w, xb.w));
+  fsum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(fsum, f.x), f.y), f.z), f.w);
+  psum = __fmaf_rn(w.w, f.w, __fmaf_rn(w.z, f.z, __fmaf_rn(w.y, f.y, __fmaf_rn(w.x, f.x, psum))));
+  return f;
+}
+__device__ __forceinline__ float edge_inv_prob(float fsum, float psum, bool y, float epsilon) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
+    psum += __shfl_xor_sync(0xffffffffu, psum, o);
+  }
+  return 1.0f / __fmaf_rn(y ? epsilon : 1.0f - epsilon, 1.0f - fsum, psum);
+}
+
 template <typename PiT, int KQ>
 __device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& b, int ncommit) {
   using TR = PiTraits<PiT>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int Kp = m.Kp, K = m.K;
+  if ((int)blockIdx.x >= ncommit + m.nbb) {
+    theta_pre_block(m, b, (int)blockIdx.x - ncommit - m.nbb);
+    return;
+  }
   if ((int)blockIdx.x < ncommit) {
     const int n_nodes = b.st->n_nodes;
     constexpr int EV = TR::kPerVec;
@@ -1048,7 +1109,7 @@ __device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& 
   __shared__ float s_part[4][2][KQ * 128];
   const int bb = blockIdx.x - ncommit;
   const int n_edges = b.st->n_edges;
-  if (bb >= m.nbb || bb * 4 >= n_edges) {  // no edges for this block: k_theta skips its partial
+  if (bb * 4 >= n_edges) {  // no edges for this block: k_theta skips its partial
     grid_dependency_wait();
     return;
   }
@@ -1078,24 +1139,17 @@ __device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& 
         xa = *reinterpret_cast<const float4*>(pa + k0);
         xb = *reinterpret_cast<const float4*>(pb + k0);
       }
-      f[q * 4 + 0] = xa.x * xb.x;
-      f[q * 4 + 1] = xa.y * xb.y;
-      f[q * 4 + 2] = xa.z * xb.z;
-      f[q * 4 + 3] = xa.w * xb.w;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float fk = f[q * 4 + e];
-        fsum += fk;
-        psum += (y ? bt[q * 4 + e] : (k0 + e < K ? 1.0f - bt[q * 4 + e] : 0.f)) * fk;
-      }
+      const bool in = k0 < K;  // past K the rows hold zeros
+      const float4 w = y ? make_float4(bt[q * 4], bt[q * 4 + 1], bt[q * 4 + 2], bt[q * 4 + 3])
+                         : make_float4(in ? 1.0f - bt[q * 4] : 0.f, in ? 1.0f - bt[q * 4 + 1] : 0.f,
+                                       in ? 1.0f - bt[q * 4 + 2] : 0.f, in ? 1.0f - bt[q * 4 + 3] : 0.f);
+      const float4 t = edge_terms(xa, xb, w, fsum, psum);
+      f[q * 4 + 0] = t.x;
+      f[q * 4 + 1] = t.y;
+      f[q * 4 + 2] = t.z;
+      f[q * 4 + 3] = t.w;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
-      psum += __shfl_xor_sync(0xffffffffu, psum, o);
-    }
-    const float prob0 = (y ? m.epsilon : 1.0f - m.epsilon) * (1.0f - fsum);
-    const float invP = 1.0f / (psum + prob0);
+    const float invP = edge_inv_prob(fsum, psum, y, m.epsilon);
     if (y) {
 #pragma unroll
       for (int e = 0; e < KQ * 4; ++e) R1[e] = fmaf(f[e], invP, R1[e]);
@@ -1129,33 +1183,140 @@ __global__ void __launch_bounds__(128) k_commit_beta_chains(const ChainArgs* __r
 }
 
 // ---------------------------------------------------------------------------
-// The parts of k's step that do not depend on the sums: 1/(theta0+theta1),
-// the two gradient factors 1/theta_kc - 1/ts, and the two noise terms
-// sqrt(eps theta_kc) n_kc -- three FP64 divisions and two square roots.
-struct ThetaPre {
-  double ts_inv, f0, f1, nz0, nz1;
-};
-static __device__ __forceinline__ ThetaPre theta_pre(const Model& m, const Buffers& b, int k,
-                                                     uint32_t step, double eps_t, double th0,
-                                                     double th1) {
-  ThetaPre p;
-  p.ts_inv = 1.0 / (th0 + th1);
-  p.f0 = 1.0 / th0 - p.ts_inv;
-  p.f1 = 1.0 / th1 - p.ts_inv;
-  const Stream rs{m.seed, m.chain};
-  double n0, n1;
-  if (b.fed_theta_noise) {
-    n0 = b.fed_theta_noise[2 * k];
-    n1 = b.fed_theta_noise[2 * k + 1];
-  } else {
-    n0 = normal_draw(rs, kTagThetaNoise, 0, step, 2ull * k);
-    n1 = normal_draw(rs, kTagThetaNoise, 0, step, 2ull * k + 1);
-  }
-  p.nz0 = sqrt(eps_t * th0) * n0;
-  p.nz1 = sqrt(eps_t * th1) * n1;
-  return p;
+// k_commit_star: k_commit_beta for a star minibatch (one source: edge e joins
+// slot 0 to slot e + 1, one y for all edges), the minibatch of the default
+// strategies.  Every staged row is read once, by the warp of its edge, which
+// also commits it to pi; the source's row is shared in shared memory; and
+// only the R of the minibatch's y is kept and written (the other is zero).
+//
+// The sums are k_commit_beta's bit for bit: CTA bb stands for its block bb,
+// whose warp w adds f_k / P_e of the edges bb*4 + w + j*nbb*4 in the order of
+// j.  Here 4*JC warps take JC of those j at once: each forms its edge's f_k
+// (kept in shared memory) and 1 / P_e, then the CTA's threads, one float pair
+// of k each, add the JC terms of the four w in that order.
+// Bound by latency, not bytes: one round of row loads and one warp sum per
+// JC*4 edges where k_commit_beta made a round per edge and warp.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void store_pi4(float* dst, const float4& x) {
+  *reinterpret_cast<float4*>(dst) = x;
+}
+__device__ __forceinline__ void store_pi4(__nv_bfloat16* dst, const float4& x) {
+  using TR = PiTraits<__nv_bfloat16>;
+  *reinterpret_cast<uint2*>(dst) = make_uint2(TR::pack2(x.x, x.y), TR::pack2(x.z, x.w));
 }
 
+template <int JC>
+constexpr size_t commit_star_smem(int Kp) {  // f, the source's row, w, 1 / P
+  return ((size_t)(4 * JC + 2) * Kp + 4 * JC) * sizeof(float);
+}
+
+template <typename PiT, int KQ, int JC>
+__device__ __forceinline__ void commit_star_body(const Model& m, const Buffers& b) {
+  constexpr int NT = 128 * JC;
+  constexpr int NIT = (KQ * 64 + NT - 1) / NT;  // float pairs of k per thread
+  extern __shared__ __align__(16) float s_star[];
+  const int Kp = m.Kp, K = m.K;
+  float* s_f = s_star;               // 4*JC rows
+  float* s_xa = s_f + 4 * JC * Kp;   // the source's new row
+  float* s_w = s_xa + Kp;            // beta or 1 - beta
+  float* s_inv = s_w + Kp;           // 4*JC
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int bb = blockIdx.x, n_edges = b.st->n_edges, per = m.nbb * 4;
+  if (bb >= m.nbb) {
+    theta_pre_block(m, b, bb - m.nbb);
+    return;
+  }
+  if (bb * 4 >= n_edges) {
+    grid_dependency_wait();
+    return;
+  }
+  const bool y = b.ey[0] != 0;
+  PiT* pi = reinterpret_cast<PiT*>(b.pi);
+  for (int k = tid; k < Kp; k += NT) s_w[k] = k < K ? (y ? b.beta[k] : 1.0f - b.beta[k]) : 0.f;
+  int ed = bb * 4 + (warp & 3) + per * (warp >> 2);
+  int32_t node = ed < n_edges ? b.nodes[ed + 1] : 0;
+  const int32_t source = b.nodes[0];
+  float2 R[NIT][4];
+#pragma unroll
+  for (int i = 0; i < NIT; ++i)
+#pragma unroll
+    for (int w = 0; w < 4; ++w) R[i][w] = make_float2(0.f, 0.f);
+  // the staged rows come from update_phi, the launch ahead of this one,
+  // which also still reads the pi rows written here
+  grid_dependency_wait();
+  grid_launch_dependents();
+  for (int k = 4 * tid; k < Kp; k += 4 * NT) {
+    const float4 x = *reinterpret_cast<const float4*>(b.stage + k);
+    *reinterpret_cast<float4*>(s_xa + k) = x;
+    if (bb == 0) store_pi4(pi + (int64_t)source * Kp + k, x);
+  }
+  for (int e0 = bb * 4; e0 < n_edges; e0 += per * JC) {
+    const bool on = ed < n_edges;
+    float4 x[KQ];
+    if (on) {
+      const float* row = b.stage + (int64_t)(ed + 1) * Kp;
+#pragma unroll
+      for (int q = 0; q < KQ; ++q) {
+        const int k0 = q * 128 + lane * 4;
+        x[q] = k0 < Kp ? *reinterpret_cast<const float4*>(row + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+    __syncthreads();  // s_xa, s_w; the terms of the last round have been added
+    if (on) {
+      float fsum = 0.f, psum = 0.f;
+#pragma unroll
+      for (int q = 0; q < KQ; ++q) {
+        const int k0 = q * 128 + lane * 4;
+        if (k0 < Kp) {
+          store_pi4(pi + (int64_t)node * Kp + k0, x[q]);
+          const float4 f = edge_terms(*reinterpret_cast<const float4*>(s_xa + k0), x[q],
+                                      *reinterpret_cast<const float4*>(s_w + k0), fsum, psum);
+          *reinterpret_cast<float4*>(s_f + warp * Kp + k0) = f;
+        }
+      }
+      const float invP = edge_inv_prob(fsum, psum, y, m.epsilon);
+      if (lane == 0) s_inv[warp] = invP;
+    }
+    __syncthreads();
+    ed += per * JC;
+    if (ed < n_edges) node = b.nodes[ed + 1];
+#pragma unroll
+    for (int i = 0; i < NIT; ++i) {
+      const int k = 2 * (tid + i * NT);
+      if (k < Kp) {
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+#pragma unroll
+          for (int j = 0; j < JC; ++j)
+            if (e0 + w + j * per < n_edges) {
+              const float2 f = *reinterpret_cast<const float2*>(s_f + (w + 4 * j) * Kp + k);
+              const float inv = s_inv[w + 4 * j];
+              R[i][w].x = fmaf(f.x, inv, R[i][w].x);
+              R[i][w].y = fmaf(f.y, inv, R[i][w].y);
+            }
+      }
+    }
+  }
+  float* out = b.beta_part + ((int64_t)bb * 2 + (y ? 1 : 0)) * Kp;
+#pragma unroll
+  for (int i = 0; i < NIT; ++i) {
+    const int k = 2 * (tid + i * NT);
+    if (k < Kp)
+      *reinterpret_cast<float2*>(out + k) = make_float2(R[i][0].x + R[i][1].x + R[i][2].x + R[i][3].x,
+                                                        R[i][0].y + R[i][1].y + R[i][2].y + R[i][3].y);
+  }
+}
+template <typename PiT, int KQ, int JC>
+__global__ void __launch_bounds__(128 * JC, JC == 1 ? 4 : 2) k_commit_star(Model m, Buffers b) {
+  commit_star_body<PiT, KQ, JC>(m, b);
+}
+template <typename PiT, int KQ, int JC>
+__global__ void __launch_bounds__(128 * JC, JC == 1 ? 4 : 2) k_commit_star_chains(const ChainArgs* __restrict__ c, int p) {
+  const ChainArgs& a = c[blockIdx.y];
+  commit_star_body<PiT, KQ, JC>(a.m, slot_buffers(a.m, a.b, p));
+}
+
+// ---------------------------------------------------------------------------
 // k_theta: theta step of update_beta (cc:241-266) in FP64.  With the block
 // sums R0_k, R1_k and beta_k the gradients of cc:236-239 are
 //   G_k0 = beta R1 (0 - 1/ts) + (1-beta) R0 (1/theta_k0 - 1/ts)
@@ -1163,134 +1324,130 @@ static __device__ __forceinline__ ThetaPre theta_pre(const Model& m, const Buffe
 // ---------------------------------------------------------------------------
 // With R_given the sums are read from it (R0_k, R1_k at 2k, 2k + 1) instead
 // of being formed from the partials; with R_out the sums are written there
-// and no step is taken (the phases of a sharded iteration).
-static __device__ __forceinline__ void theta_body(const Model& m, const Buffers& b,
+// and no step is taken (the phases of a sharded iteration).  `star`: the
+// partials are k_commit_star's, of the minibatch's y alone.
+//
+// A latency chain (partial loads, compensated sums, FP64 at 1/64 of the FP32
+// rate), so what does not need the partials is done elsewhere: the divisions,
+// square roots and normals beside the commit (theta_pre_block), the scalars,
+// theta, beta and the counters before the wait.  256 threads rather than
+// 1,024, so that the CTA fits an SM that still holds commit CTAs.
+static __device__ __forceinline__ void theta_body(const Model& m, const Buffers& b, int star,
                                                   const double* R_given = nullptr,
                                                   double* R_out = nullptr) {
-  // 32 consecutive k per CTA (lane = k); warps 0-30 sum the partials of the
-  // active beta blocks w, w+31, ... in FP32 with Kahan compensation while
-  // warp 31 forms the FP64 parts of the step that do not need the sums;
-  // then warp 0 adds the 31 warp sums in fixed order (deterministic) and
-  // finishes the step: two FMA chains and one division after the barrier.
-  constexpr int kSumWarps = kThetaSumWarps;
-  __shared__ float s_r0[kSumWarps][33], s_c0[kSumWarps][33], s_r1[kSumWarps][33], s_c1[kSumWarps][33];
-  __shared__ double s_pre[5][32];
+  // 32 consecutive k per CTA (lane = k).  31 chains add the partials of the
+  // active beta blocks c, c+31, ... in FP32 with Kahan compensation, up to 4
+  // chains per warp side by side; then warp 0 adds the 31 sums in fixed order
+  // (deterministic) and finishes the step: two FMA chains and one division.
+  constexpr int C = kThetaChains, P = kThetaPerChain, W = kThetaThreads / 32, CW = (C + W - 1) / W;
+  __shared__ float s_r[2][C][33], s_c[2][C][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
   const int Kp = m.Kp;
   const int active = min(m.nbb, (b.st->n_edges + 3) / 4);  // blocks that saw edges
-  // the step's scalars and this k's theta and beta, fetched now so that their
-  // latency overlaps the partial sums
-  const uint32_t step = b.st->step;
   const double eps_t = (double)b.st->eps;
   const double scale = (double)b.st->scale;
   const bool kin = k < m.K;
-  const double th0 = kin ? b.theta[2 * k] : 1.0, th1 = kin ? b.theta[2 * k + 1] : 1.0;
-  const double bt = kin ? (double)b.beta[k] : 0.0;
-  grid_dependency_wait();  // the beta partials: k_commit_beta, the launch ahead
-  grid_launch_dependents();
-  double R0, R1;
-  ThetaPre pre;
-  if (R_given) {
-    if (warp != 0 || !kin) return;
-    R0 = R_given[2 * k];
-    R1 = R_given[2 * k + 1];
-    pre = theta_pre(m, b, k, step, eps_t, th0, th1);
-  } else {
-    if (warp == kSumWarps) {
-      if (kin && !R_out) {
-        const ThetaPre q = theta_pre(m, b, k, step, eps_t, th0, th1);
-        s_pre[0][lane] = q.ts_inv;
-        s_pre[1][lane] = q.f0;
-        s_pre[2][lane] = q.f1;
-        s_pre[3][lane] = q.nz0;
-        s_pre[4][lane] = q.nz1;
-      }
-    } else {
-      // the warp's partials (blocks warp, warp + 31, ...) loaded together,
-      // then added in block order
-      float r0 = 0.f, c0 = 0.f, r1 = 0.f, c1 = 0.f;
-      constexpr int P = kThetaPerPass;
-      for (int base = warp; base < active; base += kSumWarps * P) {
-        float p0v[P], p1v[P];
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-          const int bb = base + kSumWarps * q;
-          const bool on = kin && bb < active;
-          const float* p0 = b.beta_part + (int64_t)bb * 2 * Kp + k;
-          p0v[q] = on ? p0[0] : 0.f;
-          p1v[q] = on ? p0[Kp] : 0.f;
-        }
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-          if (base + kSumWarps * q < active) {
-            const float y0 = p0v[q] - c0, y1 = p1v[q] - c1;
-            const float t0 = r0 + y0, t1 = r1 + y1;
-            c0 = (t0 - r0) - y0;
-            c1 = (t1 - r1) - y1;
-            r0 = t0;
-            r1 = t1;
-          }
-        }
-      }
-      s_r0[warp][lane] = r0;
-      s_c0[warp][lane] = c0;
-      s_r1[warp][lane] = r1;
-      s_c1[warp][lane] = c1;
-    }
-    __syncthreads();
-    if (warp != 0 || k >= m.K) return;
-    float a0 = 0.f, e0 = 0.f, a1 = 0.f, e1 = 0.f;  // Kahan over the warp sums
-#pragma unroll
-    for (int w = 0; w < kSumWarps; ++w) {
-      const float y0 = (s_r0[w][lane] - s_c0[w][lane]) - e0;
-      const float y1 = (s_r1[w][lane] - s_c1[w][lane]) - e1;
-      const float t0 = a0 + y0, t1 = a1 + y1;
-      e0 = (t0 - a0) - y0;
-      e1 = (t1 - a1) - y1;
-      a0 = t0;
-      a1 = t1;
-    }
-    R0 = (double)a0 - (double)e0;
-    R1 = (double)a1 - (double)e1;
-    if (R_out) {
-      R_out[2 * k] = R0;
-      R_out[2 * k + 1] = R1;
-      return;
-    }
-    pre.ts_inv = s_pre[0][lane];
-    pre.f0 = s_pre[1][lane];
-    pre.f1 = s_pre[2][lane];
-    pre.nz0 = s_pre[3][lane];
-    pre.nz1 = s_pre[4][lane];
+  const int only = star && active > 0 ? (b.ey[0] ? 1 : 0) : -1;  // the class with partials
+  double th0 = 1.0, th1 = 1.0, bt = 0.0;
+  if (warp == 0 && kin && !R_out) {
+    th0 = b.theta[2 * k];
+    th1 = b.theta[2 * k + 1];
+    bt = (double)b.beta[k];
   }
-  if (k == 0) {  // the iteration's edge evaluations and errors, counted once it is applied
+  if (blockIdx.x == 0 && threadIdx.x == 32 && !R_out) {
+    // the iteration's edge evaluations and errors, counted as it is applied
     if (b.st->err) atomicOr(&b.gc->err, b.st->err);
     b.gc->evals += (unsigned long long)b.st->n_nodes * (unsigned long long)m.n_out;
     b.gc->iters += 1ull;
   }
-  const double G0 = bt * R1 * (-pre.ts_inv) + (1.0 - bt) * R0 * pre.f0;
-  const double G1 = bt * R1 * pre.f1 + (1.0 - bt) * R0 * (-pre.ts_inv);
-  double t0 = fabs(th0 + eps_t / 2.0 * ((double)m.eta0 - th0 + scale * G0) + pre.nz0);
-  double t1 = fabs(th1 + eps_t / 2.0 * ((double)m.eta1 - th1 + scale * G1) + pre.nz1);
+  grid_dependency_wait();  // the beta partials and theta_pre: the commit, the launch ahead
+  grid_launch_dependents();
+  double pre[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) pre[i] = (warp == 0 && kin && !R_out) ? b.theta_pre[i * m.K + k] : 0.0;
+  double R[2] = {0.0, 0.0};
+  if (R_given) {
+    if (warp != 0 || !kin) return;
+    R[0] = R_given[2 * k];
+    R[1] = R_given[2 * k + 1];
+  } else {
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      if (only == 1 - y) continue;
+      // the warp's partials loaded together, then added in block order
+      float v[CW][P];
+#pragma unroll
+      for (int j = 0; j < CW; ++j)
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+          const int c = warp + W * j, bb = c + C * q;
+          v[j][q] = (kin && c < C && bb < active) ? b.beta_part[((int64_t)bb * 2 + y) * Kp + k] : 0.f;
+        }
+#pragma unroll
+      for (int j = 0; j < CW; ++j) {
+        float r = 0.f, e = 0.f;
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+          if (warp + W * j + C * q < active) {
+            const float x = v[j][q] - e, t = r + x;
+            e = (t - r) - x;
+            r = t;
+          }
+        }
+        if (warp + W * j < C) {
+          s_r[y][warp + W * j][lane] = r;
+          s_c[y][warp + W * j][lane] = e;
+        }
+      }
+    }
+    __syncthreads();
+    if (warp != 0 || k >= m.K) return;
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      if (only == 1 - y) continue;
+      float r = 0.f, e = 0.f;  // Kahan over the chains' sums
+#pragma unroll
+      for (int w = 0; w < C; ++w) {
+        const float x = (s_r[y][w][lane] - s_c[y][w][lane]) - e;
+        const float t = r + x;
+        e = (t - r) - x;
+        r = t;
+      }
+      R[y] = (double)r - (double)e;
+    }
+    if (R_out) {
+      R_out[2 * k] = R[0];
+      R_out[2 * k + 1] = R[1];
+      return;
+    }
+  }
+  const double R0 = R[0], R1 = R[1];
+  const double ts_inv = pre[0], f0 = pre[1], f1 = pre[2], nz0 = pre[3], nz1 = pre[4];
+  const double G0 = bt * R1 * (-ts_inv) + (1.0 - bt) * R0 * f0;
+  const double G1 = bt * R1 * f1 + (1.0 - bt) * R0 * (-ts_inv);
+  double t0 = fabs(th0 + eps_t / 2.0 * ((double)m.eta0 - th0 + scale * G0) + nz0);
+  double t1 = fabs(th1 + eps_t / 2.0 * ((double)m.eta1 - th1 + scale * G1) + nz1);
   if (t0 < 1.0e-24) t0 = 1.0e-24;
   if (t1 < 1.0e-24) t1 = 1.0e-24;
   b.theta[2 * k] = t0;
   b.theta[2 * k + 1] = t1;
   b.beta[k] = (float)(t1 / (t0 + t1));
 }
-static __global__ void __launch_bounds__(1024) k_theta(Model m, Buffers b) { theta_body(m, b); }
+static __global__ void __launch_bounds__(kThetaThreads) k_theta(Model m, Buffers b, int star) {
+  theta_body(m, b, star);
+}
 // the per-k sums R0, R1 of the beta partials, without the step
-static __global__ void __launch_bounds__(1024) k_beta_sums(Model m, Buffers b, double* R_out) {
-  theta_body(m, b, nullptr, R_out);
+static __global__ void __launch_bounds__(kThetaThreads) k_beta_sums(Model m, Buffers b, double* R_out) {
+  theta_body(m, b, 0, nullptr, R_out);
 }
 // the theta step from given sums
-static __global__ void __launch_bounds__(1024) k_theta_given(Model m, Buffers b, const double* R) {
-  theta_body(m, b, R, nullptr);
+static __global__ void __launch_bounds__(kThetaThreads) k_theta_given(Model m, Buffers b, const double* R) {
+  theta_body(m, b, 0, R, nullptr);
 }
-static __global__ void __launch_bounds__(1024) k_theta_chains(const ChainArgs* __restrict__ c, int p) {
+static __global__ void __launch_bounds__(kThetaThreads) k_theta_chains(const ChainArgs* __restrict__ c, int p) {
   const ChainArgs& a = c[blockIdx.y];
-  theta_body(a.m, slot_buffers(a.m, a.b, p));
+  theta_body(a.m, slot_buffers(a.m, a.b, p), a.star);
 }
 
 // ---------------------------------------------------------------------------
