@@ -70,15 +70,17 @@ struct DevCounters {
   unsigned long long iters;  // running count of updated iterations
 };
 
-// Graph in device memory: symmetric CSR with sorted rows, plus an
-// open-addressing hash (linear probing, power-of-two capacity, load <= 1/2)
-// of the held-out and test pairs.
+// Graph in device memory: symmetric CSR with sorted rows, and the held-out
+// and test pairs as a second one.  A sampler that draws many partners of one
+// node stages both of the node's rows once; a hash of the held-out pairs, one
+// probe per candidate, made every candidate a dependent read of global memory
+// (under an update that keeps HBM busy, some 2 us each).
 struct DevGraph {
   int64_t n;
   const int64_t* row_ptr;
   const int32_t* col;
-  const unsigned long long* excl;  // keys min<<32|max, empty = ~0ull
-  uint32_t excl_mask;
+  const int64_t* xrow;  // held-out and test pairs: row pointers, partners
+  const int32_t* xcol;
 };
 
 // Membership of b in a sorted row held in shared memory.
@@ -94,31 +96,6 @@ __device__ __forceinline__ bool row_contains(const int32_t* row, int32_t deg, in
   return lo < deg && row[lo] == b;
 }
 
-constexpr unsigned long long kEmptyKey = ~0ull;
-
-__host__ __device__ __forceinline__ unsigned long long pair_key(int32_t a, int32_t b) {
-  uint32_t lo = (uint32_t)(a < b ? a : b), hi = (uint32_t)(a < b ? b : a);
-  return ((unsigned long long)lo << 32) | hi;
-}
-
-__host__ __device__ __forceinline__ uint64_t hash64_full(unsigned long long k) {
-  k ^= k >> 33;
-  k *= 0xff51afd7ed558ccdull;
-  k ^= k >> 33;
-  k *= 0xc4ceb9fe1a85ec53ull;
-  k ^= k >> 33;
-  return k;
-}
-
-__host__ __device__ __forceinline__ uint32_t hash64(unsigned long long k) {
-  k ^= k >> 33;
-  k *= 0xff51afd7ed558ccdull;
-  k ^= k >> 33;
-  k *= 0xc4ceb9fe1a85ec53ull;
-  k ^= k >> 33;
-  return (uint32_t)k;
-}
-
 __host__ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   x ^= x >> 16;
   x *= 0x7feb352du;
@@ -128,49 +105,41 @@ __host__ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   return x;
 }
 
-// Edge::in(held_out_map) || Edge::in(test_map)
-__device__ __forceinline__ bool is_excluded(const DevGraph& g, int32_t a, int32_t b) {
-  const unsigned long long key = pair_key(a, b);
-  uint32_t slot = hash64(key) & g.excl_mask;
-  for (uint32_t probe = 0; probe <= g.excl_mask; ++probe) {
-    unsigned long long k = __ldg(g.excl + slot);
-    if (k == key) return true;
-    if (k == kEmptyKey) return false;
-    slot = (slot + 1) & g.excl_mask;
-  }
-  return false;
-}
-
-// Finishes a linear-probing lookup whose first slot `slot` was already
-// loaded as `first` (so callers can issue several first loads at once).
-__device__ __forceinline__ bool probe_resolve(const unsigned long long* tab,
-                                              unsigned long long mask,
-                                              unsigned long long key,
-                                              unsigned long long slot,
-                                              unsigned long long first) {
-  if (first == key) return true;
-  if (first == kEmptyKey) return false;
-  for (unsigned long long probe = 1; probe <= mask; ++probe) {
-    slot = (slot + 1) & mask;
-    const unsigned long long k = __ldg(tab + slot);
-    if (k == key) return true;
-    if (k == kEmptyKey) return false;
-  }
-  return false;
-}
-
-// Edge::in(NetworkGraph) by binary search in the sorted row of a.
-__device__ __forceinline__ bool has_edge(const DevGraph& g, int32_t a, int32_t b) {
-  int64_t lo = __ldg(g.row_ptr + a), hi = __ldg(g.row_ptr + a + 1);
+// Membership of b in entries [lo, hi) of a sorted row in global memory.
+__device__ __forceinline__ bool span_contains(const int32_t* col, int64_t lo, int64_t hi, int32_t b) {
   const int64_t end = hi;
   while (lo < hi) {
-    int64_t mid = lo + ((hi - lo) >> 1);
-    if (__ldg(g.col + mid) < b)
+    const int64_t mid = lo + ((hi - lo) >> 1);
+    if (__ldg(col + mid) < b)
       lo = mid + 1;
     else
       hi = mid;
   }
-  return lo < end && __ldg(g.col + lo) == b;
+  return lo < end && __ldg(col + lo) == b;
+}
+
+// Edge::in(held_out_map) || Edge::in(test_map)
+__device__ __forceinline__ bool is_excluded(const DevGraph& g, int32_t a, int32_t b) {
+  return span_contains(g.xcol, __ldg(g.xrow + a), __ldg(g.xrow + a + 1), b);
+}
+
+// A node's sorted row of a CSR, staged into `cap` words of shared memory by
+// the calling threads (tid of nt) when it fits; the caller synchronises.
+struct StagedRow {
+  const int32_t* smem;  // null: too long
+  const int32_t* col;
+  int64_t r0;
+  int32_t deg;
+  __device__ __forceinline__ bool contains(int32_t b) const {
+    return smem ? row_contains(smem, deg, b) : span_contains(col, r0, r0 + deg, b);
+  }
+};
+__device__ __forceinline__ StagedRow stage_row(const int32_t* col, int64_t r0, int64_t r1, int32_t* smem, int cap,
+                                               int tid, int nt) {
+  const int32_t deg = (int32_t)(r1 - r0);
+  if (deg <= cap)
+    for (int q = tid; q < deg; q += nt) smem[q] = __ldg(col + r0 + q);
+  return StagedRow{deg <= cap ? smem : nullptr, col, r0, deg};
 }
 
 // ---- pi storage types -------------------------------------------------------

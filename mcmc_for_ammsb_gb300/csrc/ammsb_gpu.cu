@@ -800,29 +800,33 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
   g.n = N;
   g.row_ptr = d_row;
   g.col = d_col;
-  {  // held-out + test exclusion hash
-    const int64_t nex = h->H + h->T;
-    const int cap = next_pow2(std::max<int64_t>(16, 2 * nex));
-    std::vector<unsigned long long> keys(cap, kEmptyKey);
-    auto insert = [&](const ammsb_edge_set* s) {
-      if (!s) return;
-      for (int64_t i = 0; i < s->count; ++i) {
-        unsigned long long k = pair_key(s->a[i], s->b[i]);
-        uint32_t slot = hash64(k) & (uint32_t)(cap - 1);
-        while (keys[slot] != kEmptyKey && keys[slot] != k) slot = (slot + 1) & (uint32_t)(cap - 1);
-        keys[slot] = k;
-      }
+  {  // held-out and test pairs as a symmetric CSR with sorted rows
+    std::vector<int64_t> xrow((size_t)N + 1, 0);
+    auto each = [&](auto&& f) {
+      for (const ammsb_edge_set* s : {held_out, test})
+        for (int64_t i = 0; s && i < s->count; ++i) {
+          f(s->a[i], s->b[i]);
+          f(s->b[i], s->a[i]);
+        }
     };
-    insert(held_out);
-    insert(test);
-    unsigned long long* d_ex = nullptr;
-    TRY(dev_alloc(h, &d_ex, cap));
-    if (cudaMemcpyAsync(d_ex, keys.data(), sizeof(unsigned long long) * cap, cudaMemcpyHostToDevice, h->stream) != cudaSuccess) {
+    each([&](int32_t a, int32_t) { ++xrow[(size_t)a + 1]; });
+    for (int64_t v = 0; v < N; ++v) xrow[v + 1] += xrow[v];
+    std::vector<int32_t> xcol((size_t)std::max<int64_t>(xrow[N], 1));
+    std::vector<int64_t> at(xrow.begin(), xrow.end() - 1);
+    each([&](int32_t a, int32_t b) { xcol[at[a]++] = b; });
+    for (int64_t v = 0; v < N; ++v)
+      if (xrow[v + 1] - xrow[v] > 1) std::sort(xcol.begin() + xrow[v], xcol.begin() + xrow[v + 1]);
+    int64_t* d_xrow = nullptr;
+    int32_t* d_xcol = nullptr;
+    TRY(dev_alloc(h, &d_xrow, N + 1));
+    TRY(dev_alloc(h, &d_xcol, xcol.size()));
+    if (cudaMemcpyAsync(d_xrow, xrow.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+        cudaMemcpyAsync(d_xcol, xcol.data(), sizeof(int32_t) * xcol.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess) {
       h->err = "exclusion upload failed";
       return bail(AMMSB_E_CUDA);
     }
-    g.excl = d_ex;
-    g.excl_mask = (uint32_t)(cap - 1);
+    g.xrow = d_xrow;
+    g.xcol = d_xcol;
   }
   // held-out set for perplexity
   TRY(dev_alloc(h, &h->d_ha, std::max<int64_t>(h->H, 1)));

@@ -295,7 +295,8 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
                                                              const Buffers& b, int j, int smem_hash) {
   extern __shared__ uint32_t s_htab[];  // dedup hash in shared memory when it fits
   constexpr int kRowCap = 2048;         // the source's row, staged when it fits
-  __shared__ int32_t s_row[kRowCap];
+  constexpr int kExclCap = 512;         // and its held-out and test partners
+  __shared__ int32_t s_row[kRowCap], s_xrow[kExclCap];
   __shared__ int s_warp[33];
   __shared__ int s_flag, s_count, s_nodes;
   __shared__ uint32_t s_step;
@@ -334,11 +335,8 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
     }
     if (mb > m.max_edges || mb + 1 > m.max_nodes) err |= kErrCapacity;
     if (tid == 0) b.nodes[0] = v;
-    const int64_t vr0 = g.row_ptr[v];
-    const int32_t vdeg = (int32_t)(g.row_ptr[v + 1] - vr0);
-    const bool row_in_smem = vdeg <= kRowCap;
-    if (row_in_smem)
-      for (int q = tid; q < vdeg; q += blockDim.x) s_row[q] = g.col[vr0 + q];
+    const StagedRow links = stage_row(g.col, g.row_ptr[v], g.row_ptr[v + 1], s_row, kRowCap, tid, blockDim.x);
+    const StagedRow excl = stage_row(g.xcol, g.xrow[v], g.xrow[v + 1], s_xrow, kExclCap, tid, blockDim.x);
     __syncthreads();
     int count = 0;
     uint64_t t = 0;
@@ -363,57 +361,22 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
       const int want = (int)min(est + est / 8 + 64, (int64_t)half);
       const int R = (int)min((uint64_t)max(need, min(half - count, want)), cap - t);
       const int count0 = count;
-      // pass A: validity and first-occurrence index per value, over chunks
-      // of up to G * 1,024 candidates.  Thread tid examines candidates
-      // c0 + tid + 1024 j of its chunk (one each while the chunk has at most
-      // 1,024); the first exclusion probes of its candidates are issued
-      // together.
-      constexpr int G = 4;
-      const int chunk = G * (int)blockDim.x;
-      for (int c0 = 0; c0 < R; c0 += chunk) {
-        int32_t u[G];
-        bool live[G];
-        unsigned long long key[G], xs[G], xk[G];
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-          const int c = c0 + tid + (int)blockDim.x * j;
-          live[j] = c < R;
-          u[j] = live[j] ? (int32_t)uniform_below(rs.draw_u64(kTagMbCand, 0, step, t + (uint64_t)c),
-                                                  (uint64_t)g.n)
-                         : -1;
-          live[j] = live[j] && (u[j] != v);
-          key[j] = pair_key(v, u[j] < 0 ? 0 : u[j]);
-          xs[j] = hash64(key[j]) & g.excl_mask;
-        }
-#pragma unroll
-        for (int j = 0; j < G; ++j) xk[j] = live[j] ? __ldg(g.excl + xs[j]) : kEmptyKey;
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-          const int c = c0 + tid + (int)blockDim.x * j;
-          if (c >= R) continue;
-          const bool linked = live[j] && (row_in_smem ? row_contains(s_row, vdeg, u[j])
-                                                      : has_edge(g, v, u[j]));
-          const bool ok = live[j] && !linked &&
-                          !probe_resolve(g.excl, g.excl_mask, key[j], xs[j], xk[j]);
-          b.cand[c] = ok ? u[j] : -1;
-          if (ok) {
-            uint32_t slot = hash32((uint32_t)u[j]) & b.hmask;
-            for (uint32_t probe = 0; probe <= b.hmask; ++probe) {
-              const uint32_t prev = atomicCAS(hkey + slot, 0xffffffffu, (uint32_t)u[j]);
-              if (prev == 0xffffffffu || prev == (uint32_t)u[j]) {
-                atomicMin(hidx + slot, (uint32_t)(t + (uint64_t)c));
-                break;
-              }
-              slot = (slot + 1) & b.hmask;
-            }
-          }
-        }
+      // pass A: validity and first-occurrence index per value; both of the
+      // source's rows are in shared memory
+      for (int c = tid; c < R; c += blockDim.x) {
+        const int32_t u = (int32_t)uniform_below(rs.draw_u64(kTagMbCand, 0, step, t + (uint64_t)c),
+                                                 (uint64_t)g.n);
+        const bool ok = u != v && !links.contains(u) && !excl.contains(u);
+        b.cand[c] = ok ? u : -1;
+        if (ok) hash_insert_min(hkey, hidx, b.hmask, (uint32_t)u, (uint32_t)(t + (uint64_t)c));
       }
       __syncthreads();
       // pass B: ordered compaction of first occurrences, one block scan per
-      // chunk (thread-local counts of its g consecutive candidates, g the
-      // fewest per thread that cover the chunk); count is block-uniform, so
-      // every thread leaves the loop together at mb
+      // chunk of up to G * 1,024 (thread-local counts of its g consecutive
+      // candidates, g the fewest per thread that cover the chunk); count is
+      // block-uniform, so every thread leaves the loop together at mb
+      constexpr int G = 4;
+      const int chunk = G * (int)blockDim.x;
       for (int c0 = 0; c0 < R && count < mb; c0 += chunk) {
         const int n = min(R - c0, chunk);
         const int gper = (n + (int)blockDim.x - 1) / (int)blockDim.x;
@@ -427,18 +390,8 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
           acc[j] = false;
           if (j < gper && c < c0 + n) {
             u[j] = b.cand[c];
-            if (u[j] >= 0) {
-              uint32_t slot = hash32((uint32_t)u[j]) & b.hmask;
-              for (uint32_t probe = 0; probe <= b.hmask; ++probe) {
-                const uint32_t kk = hkey[slot];
-                if (kk == (uint32_t)u[j]) {
-                  acc[j] = (hidx[slot] == (uint32_t)(t + (uint64_t)c));
-                  break;
-                }
-                if (kk == 0xffffffffu) break;
-                slot = (slot + 1) & b.hmask;
-              }
-            }
+            if (u[j] >= 0)
+              acc[j] = hash_find(hkey, hidx, b.hmask, (uint32_t)u[j]) == (uint32_t)(t + (uint64_t)c);
           }
           mine += acc[j] ? 1 : 0;
         }
@@ -634,13 +587,14 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
         err |= kErrCapacity;
         break;
       }
+      const int64_t x0 = g.xrow[v], x1 = g.xrow[v + 1];
       for (int64_t base = 0; base < deg; base += blockDim.x) {
         const int64_t q = base + tid;
         int32_t u = -1;
         bool acc = false;
         if (q < deg) {
           u = g.col[r0 + q];
-          acc = !is_excluded(g, v, u);
+          acc = !span_contains(g.xcol, x0, x1, u);
         }
         int total;
         const int pos = block_scan_1024(acc, s_warp, &total);
@@ -699,11 +653,11 @@ __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevG
   // power of two >= 2 n_out, -1 empty) in dynamic shared memory
   extern __shared__ int32_t s_sets[];
   constexpr int kRowCap = 256;  // the node's own row, staged when it fits
-  __shared__ int32_t s_rows[WARPS][kRowCap];
+  constexpr int kExclCap = 32;  // and its held-out and test partners
+  __shared__ int32_t s_rows[WARPS][kRowCap], s_xrows[WARPS][kExclCap];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t smask = (uint32_t)m.nbr_set_cap - 1u;
   int32_t* set = s_sets + (size_t)warp * m.nbr_set_cap;
-  int32_t* srow = s_rows[warp];
   const int n_nodes = b.st->n_nodes;
   const uint32_t step = b.st->step;
   const Stream rs{m.seed, m.chain};
@@ -721,26 +675,31 @@ __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevG
   }
   for (int slot = blockIdx.x * WARPS + warp; slot < n_nodes; slot += gridDim.x * WARPS) {
     const int32_t i = b.nodes[slot];
-    const int64_t ir0 = g.row_ptr[i];
-    const int32_t ideg = (int32_t)(g.row_ptr[i + 1] - ir0);
-    const bool row_in_smem = ideg <= kRowCap;
-    if (row_in_smem)
-      for (int q = lane; q < ideg; q += 32) srow[q] = g.col[ir0 + q];
+    const int64_t r0 = g.row_ptr[i], r1 = g.row_ptr[i + 1], x0 = g.xrow[i], x1 = g.xrow[i + 1];
+    const StagedRow links = stage_row(g.col, r0, r1, s_rows[warp], kRowCap, lane, 32);
+    const StagedRow excl = stage_row(g.xcol, x0, x1, s_xrows[warp], kExclCap, lane, 32);
     for (uint32_t q = lane; q <= smask; q += 32) set[q] = -1;
     __syncwarp();
     int count = 0;
     uint64_t t = 0;
+    int32_t j0 = 0, j1 = 0;  // candidates 2 lane and 2 lane + 1 of a pair of rounds
     while (count < m.n_out) {
       if (t >= cap) {
         if (lane == 0) atomicOr(&b.st->err, kErrNeighborCap);
         break;
       }
-      const int32_t j = (int32_t)uniform_below(rs.draw_u64(kTagNbr, (uint32_t)i, step, t + lane),
-                                               (uint64_t)g.n);
-      const unsigned long long key = pair_key(i, j);
-      const unsigned long long xs = hash64(key) & g.excl_mask;
-      const unsigned long long xk = __ldg(g.excl + xs);
-      bool ok = (j != i) && !probe_resolve(g.excl, g.excl_mask, key, xs, xk);
+      // a Philox block holds two draws: the lanes form 64 candidates with a
+      // block each, and every second round takes the upper half
+      const int half = (int)(t >> 5) & 1;
+      if (half == 0) {
+        const U32x4 o = rs.block(kTagNbr, (uint32_t)i, step, (t >> 1) + lane);
+        j0 = (int32_t)uniform_below((uint64_t)o.x | ((uint64_t)o.y << 32), (uint64_t)g.n);
+        j1 = (int32_t)uniform_below((uint64_t)o.z | ((uint64_t)o.w << 32), (uint64_t)g.n);
+      }
+      const int from = half * 16 + (lane >> 1);
+      const int32_t ja = __shfl_sync(0xffffffffu, j0, from), jb = __shfl_sync(0xffffffffu, j1, from);
+      const int32_t j = (lane & 1) ? jb : ja;
+      bool ok = (j != i) && !(excl.deg > 0 && excl.contains(j));
       if (ok) {  // already accepted in an earlier round?
         uint32_t h = hash32((uint32_t)j) & smask;
         for (uint32_t probe = 0; probe <= smask; ++probe) {
@@ -766,14 +725,14 @@ __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevG
           if (atomicCAS(set + h, -1, j) == -1) break;
           h = (h + 1) & smask;
         }
-        const uint32_t y = (row_in_smem ? row_contains(srow, ideg, j) : has_edge(g, i, j)) ? 1u : 0u;
+        const uint32_t y = links.contains(j) ? 1u : 0u;
         b.nbr[(int64_t)slot * m.n_out + idx] = (uint32_t)j | (y << 31);
       }
       count += min(__popc(bal), need);
       t += 32;
       __syncwarp();
     }
-    __syncwarp();  // srow and set are reused by the warp's next node
+    __syncwarp();  // the rows and the set are reused by the warp's next node
   }
 }
 template <int WARPS>
