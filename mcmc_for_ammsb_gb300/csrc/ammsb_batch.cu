@@ -34,8 +34,8 @@ struct PhiGroup {
   std::vector<int> chains;
   ChainArgs* d = nullptr;  // the group's chains, in order
   int gx = 1;
-  size_t smem = 0;
-  size_t smem_wide = 0;  // ring kernel: its 16-warp variant
+  size_t smem = 0;      // ring kernel: per four-warp group
+  size_t smem_few = 0;  // ring kernel: a 16-warp node
 };
 
 struct CommitGroup {
@@ -47,8 +47,6 @@ struct CommitGroup {
   size_t smem = 0;
 };
 
-constexpr int kRingSplitB = 4;
-
 template <typename PiT, int L, int V, int S>
 cudaError_t phi_reg_chains(const PhiGroup& g, int p, cudaStream_t st) {
   constexpr int NPB = 128 / (L * S) > 0 ? 128 / (L * S) : 1;
@@ -59,28 +57,22 @@ cudaError_t phi_reg_chains(const PhiGroup& g, int p, cudaStream_t st) {
 
 template <typename PiT, int V, int STAGES, bool FULL>
 cudaError_t phi_ring_chains(const PhiGroup& g, int p, cudaStream_t st, bool configure) {
-  // the same pair of launches as one chain: a 16-warp variant for the
-  // iterations of few nodes, the 4-warp kernel for the others
-  constexpr int WS = sizeof(PiT) == 2 ? 4 : 2;
-  auto kern = k_update_phi_ring_chains<PiT, V, kRingSplitB, STAGES, FULL>;
-  auto wide = k_update_phi_ring_chains<PiT, V, kRingSplitWide, WS, FULL>;
-  // every chain of the group configured the variant (its shared memory is
-  // then the largest of theirs), or none did
-  const bool use_wide = g.cfg.ring_few && g.smem_wide > 0 && g.smem_wide <= 200 * 1024;
-  if (configure) {
-    cudaError_t e = ammsb_detail::raise_smem_limit(kern, g.smem);
-    if (e == cudaSuccess && use_wide) e = ammsb_detail::raise_smem_limit(wide, g.smem_wide);
-    return e;
-  }
+  // launched as for one chain; a CTA's groups for every node slot
+  auto kern = k_update_phi_ring_chains<PiT, V, STAGES, FULL>;
+  const RingPlan r = ring_plan(g.cfg, g.smem, g.smem_few);
+  if (configure) return ammsb_detail::raise_smem_limit(kern, r.smem());
   const unsigned n = (unsigned)g.chains.size();
-  if (use_wide) {
-    wide<<<dim3(kRingFewNodes, n), kRingSplitWide * 32, g.smem_wide, st>>>(g.d, p, 0, kRingFewNodes);
+  const dim3 grid(std::max((g.gx + r.groups - 1) / r.groups, r.few), n);
+  if (r.single) {
+    kern<<<grid, 512, r.smem(), st>>>(g.d, p, r.few, kPhiFew | kPhiMany);
+    return cudaGetLastError();
+  }
+  if (r.few > 0) {
+    kern<<<dim3(r.few, n), 512, r.few_bytes, st>>>(g.d, p, r.few, kPhiFew);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    kern<<<dim3(g.gx, n), kRingSplitB * 32, g.smem, st>>>(g.d, p, kRingFewNodes, INT32_MAX);
-  } else {
-    kern<<<dim3(g.gx, n), kRingSplitB * 32, g.smem, st>>>(g.d, p, 0, INT32_MAX);
   }
+  kern<<<grid, r.groups * kPhiGroup, r.groups * r.group_bytes, st>>>(g.d, p, r.few, kPhiMany);
   return cudaGetLastError();
 }
 
@@ -103,9 +95,11 @@ cudaError_t phi_chains(const PhiGroup& g, int p, cudaStream_t st, bool configure
       case 1: return phi_ring_chains_v<PiT, 1>(g, p, st, configure);
       case 2: return phi_ring_chains_v<PiT, 2>(g, p, st, configure);
       case 4: return phi_ring_chains_v<PiT, 4>(g, p, st, configure);
-      case 8: return phi_ring_chains_v<PiT, 8>(g, p, st, configure);
-      default: return cudaErrorInvalidConfiguration;
+      default: break;
     }
+    if constexpr (sizeof(PiT) == 4)
+      if (c.vpl == 8) return phi_ring_chains_v<PiT, 8>(g, p, st, configure);
+    return cudaErrorInvalidConfiguration;
   }
   if (configure) {
     if (g.smem <= 48 * 1024) return cudaSuccess;
@@ -382,7 +376,7 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     const int ev = (h->opt.pi_dtype == AMMSB_PI_BF16) ? 8 : 4;
     const bool full = (h->m.Kp / ev == 32 * c.vpl);
     auto key = std::make_tuple((int)h->opt.pi_dtype, c.ring, c.lpn, c.vpl, c.split,
-                               c.ring ? c.ring_stages : 0, c.ring ? (int)full : 0);
+                               c.ring ? c.ring_stages : 0, c.ring ? (int)full + 2 * (h->phi_smem_few > 0) : 0);
     auto it = pg.find(key);
     if (it == pg.end()) {
       PhiGroup g;
@@ -397,7 +391,7 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     if (c.ring) {
       g.gx = std::max(g.gx, h->m.max_nodes);
       g.smem = std::max(g.smem, h->phi_smem);
-      g.smem_wide = std::max(g.smem_wide, h->phi_smem_wide);
+      g.smem_few = std::max(g.smem_few, h->phi_smem_few);
     } else {
       const int npb = std::max(1, 128 / (c.lpn * c.split));
       g.gx = std::max(g.gx, std::max(1, std::min((h->m.max_nodes + npb - 1) / npb, 152 * 32)));

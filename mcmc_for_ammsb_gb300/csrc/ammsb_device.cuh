@@ -60,6 +60,7 @@ struct DevState {
   int32_t n_nodes;
   int32_t rounds;
   int32_t err;  // error bits of these draws, raised when the iteration is applied
+  uint32_t next_node;  // update_phi's node queue, zero between launches
 };
 
 // Sampler-wide counters shared by all buffer sets.

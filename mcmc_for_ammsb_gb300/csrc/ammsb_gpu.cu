@@ -83,11 +83,6 @@ cudaError_t launch_phi_t(ammsb_handle* h, const Buffers& b) {
   return cudaGetLastError();
 }
 
-#ifndef AMMSB_RING_SPLIT
-#define AMMSB_RING_SPLIT 4
-#endif
-constexpr int kRingSplit = AMMSB_RING_SPLIT;  // warps per node of the many-node ring kernel
-
 // Launches `k` on stream `s`; with `pdl` as a programmatic dependent launch
 // (it may start once every CTA of the kernel ahead of it in the stream has
 // triggered, and waits on the device before reading that kernel's results).
@@ -108,45 +103,31 @@ cudaError_t launch_k(void (*k)(P...), int grid, int block, size_t smem, cudaStre
 }
 
 // `pdl`: the launch directly follows k_theta in the stream and its draws
-// were complete before that kernel started; the update kernels then start
-// as programmatic dependent launches, the many-node kernel first, which
-// overlaps its first row copies and node prologue with the theta step.
+// were complete before that kernel started; it then starts as a programmatic
+// dependent launch, which overlaps its first row copies and node prologues
+// with the theta step.
 template <typename PiT, int VPL, int STAGES, bool FULL>
 cudaError_t launch_phi_ring_t(ammsb_handle* h, const Buffers& b, bool configure, bool pdl = false) {
-  auto kern = k_update_phi_ring<PiT, VPL, kRingSplit, STAGES, FULL>;
-  constexpr int WS = sizeof(PiT) == 2 ? 4 : 2;  // ring depth of the 16-warp variant
-  auto wide = k_update_phi_ring<PiT, VPL, kRingSplitWide, WS, FULL>;
-  const size_t smem = PhiRingSmem<PiT, VPL, kRingSplit, STAGES>::bytes(h->m.Kp, h->m.n_out);
-  const size_t smem_w = PhiRingSmem<PiT, VPL, kRingSplitWide, WS>::bytes(h->m.Kp, h->m.n_out);
-  const bool use_wide = h->cfg.ring_few && smem_w <= 200 * 1024;
+  auto kern = k_update_phi_ring<PiT, VPL, STAGES, FULL>;
+  const RingPlan r = ring_plan(h->cfg, PhiRingSmem<PiT, VPL, 4, STAGES>::bytes(h->m.Kp, h->m.n_out),
+                               PhiRingSmem<PiT, VPL, 16, ring_few_stages<PiT>()>::bytes(h->m.Kp, h->m.n_out));
   if (configure) {
-    cudaError_t e = ammsb_detail::raise_smem_limit(kern, smem);
-    if (e != cudaSuccess) return e;
-    if (use_wide && (e = ammsb_detail::raise_smem_limit(wide, smem_w)) != cudaSuccess) return e;
-    h->phi_smem = smem;
-    h->phi_smem_wide = use_wide ? smem_w : 0;
-    return cudaSuccess;
+    h->phi_smem = r.group_bytes;
+    h->phi_smem_few = r.few_bytes;
+    return ammsb_detail::raise_smem_limit(kern, r.smem());
   }
-  // the many-node kernel walks the node slots grid-stride: one CTA per slot
-  // unless a smaller grid is asked for
-  const int grid = h->cfg.ring_grid > 0 ? std::min(h->cfg.ring_grid, h->m.max_nodes) : h->m.max_nodes;
-  const int grid_w = std::min(kRingFewNodes, h->m.max_nodes);
+  // a CTA per SM, which share the nodes through the buffer set's counter, or
+  // fewer where a minibatch gives each of its groups at most one
   const Model& m = h->m;
-  if (pdl) {
-    cudaError_t e = launch_k(kern, grid, kRingSplit * 32, smem, h->stream, true, m, b,
-                             use_wide ? kRingFewNodes : 0, INT32_MAX);
-    if (e != cudaSuccess || !use_wide) return e;
-    return launch_k(wide, grid_w, kRingSplitWide * 32, smem_w, h->stream, true, m, b, 0, kRingFewNodes);
-  }
-  if (use_wide) {
-    wide<<<grid_w, kRingSplitWide * 32, smem_w, h->stream>>>(m, b, 0, kRingFewNodes);
-    cudaError_t e = cudaGetLastError();
+  const int most = std::max((m.max_nodes + r.groups - 1) / r.groups, std::min(r.few, m.max_nodes));
+  const int grid = h->cfg.ring_grid > 0 ? std::min(h->cfg.ring_grid, most) : most;
+  if (r.single) return launch_k(kern, grid, 512, r.smem(), h->stream, pdl, m, b, r.few, kPhiFew | kPhiMany);
+  if (r.few > 0) {
+    cudaError_t e = launch_k(kern, std::min(r.few, m.max_nodes), 512, r.few_bytes, h->stream, pdl, m, b, r.few,
+                             kPhiFew);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kRingSplit * 32, smem, h->stream>>>(m, b, kRingFewNodes, INT32_MAX);
-  } else {
-    kern<<<grid, kRingSplit * 32, smem, h->stream>>>(m, b, 0, INT32_MAX);
   }
-  return cudaGetLastError();
+  return launch_k(kern, grid, r.groups * kPhiGroup, r.groups * r.group_bytes, h->stream, pdl, m, b, r.few, kPhiMany);
 }
 
 // ring depths the ring kernel is built for; FULL when every lane's
@@ -170,9 +151,12 @@ cudaError_t launch_phi_ring(ammsb_handle* h, const Buffers& b, bool configure, b
     case 1: return launch_phi_ring_v<PiT, 1>(h, b, configure, pdl);
     case 2: return launch_phi_ring_v<PiT, 2>(h, b, configure, pdl);
     case 4: return launch_phi_ring_v<PiT, 4>(h, b, configure, pdl);
-    case 8: return launch_phi_ring_v<PiT, 8>(h, b, configure, pdl);
-    default: return cudaErrorInvalidConfiguration;
+    default: break;
   }
+  // K <= 1024: only FP32 rows reach eight vectors a lane
+  if constexpr (sizeof(PiT) == 4)
+    if (h->cfg.vpl == 8) return launch_phi_ring_v<PiT, 8>(h, b, configure, pdl);
+  return cudaErrorInvalidConfiguration;
 }
 
 template <typename PiT>
@@ -529,16 +513,12 @@ void choose_config(ammsb_handle* h) {
   c.ring_stages = (h->opt.pi_dtype == AMMSB_PI_BF16) ? 4 : 3;  // fastest ring depths on GB300
   c.ring_few = 1;
   if (const char* env = std::getenv("AMMSB_PHI_FEW")) c.ring_few = std::atoi(env) != 0;
-  // the many-node ring launch: 16 CTAs per SM (four waves of the four that
-  // fit an SM), each walking its node slots; a link-stratum iteration, which
-  // leaves this launch idle, then starts 2,432 empty CTAs on a GB300 instead
-  // of one per node slot (4,097 at m = 4,096): 0.6% less time per BF16
-  // iteration on the 4M-node workload; fewer CTAs (12 or 14 per SM) were
-  // slower (uneven node counts per CTA)
+  // the ring launch: one CTA per SM (16 warps at up to 128 registers fill
+  // it); its groups of four warps take the nodes from a counter
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess || sms < 1)
     sms = 152;
-  c.ring_grid = 16 * sms;
+  c.ring_grid = sms;
   if (const char* env = std::getenv("AMMSB_PHI_GRID")) c.ring_grid = std::max(0, std::atoi(env));
   // early starts of all three: of update_phi and theta 1.7% less time per
   // BF16 iteration on the 4M-node workload; of the commit, whose

@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <string>
@@ -34,8 +35,8 @@ struct KernelCfg {
   int lpn, vpl, split, npb;  // update_phi
   int ring;                  // wide rows: the shared-memory ring kernel
   int ring_stages;           // its ring depth
-  int ring_few;              // a 16-warp variant takes iterations of few nodes
-  int ring_grid;             // CTAs of the many-node ring launch (0: one per node slot)
+  int ring_few;              // iterations of few nodes take 16 warps per node
+  int ring_grid;             // CTAs of the ring launch at most (0: one per node of its groups)
   int pdl;                   // programmatic dependent launches: kPdl* bits
   int ppx_lpn, ppx_vpl;      // perplexity
   int kq;                    // commit: 128-element pieces of a row per lane
@@ -85,7 +86,7 @@ struct ammsb_handle {
   int ncommit = 1;
   bool star = false;  // drawn minibatches are stars
   int nbr_blocks = 1, phi_blocks = 1;
-  size_t phi_smem = 0, phi_smem_wide = 0, nbr_smem = 0, mb_smem = 0;
+  size_t phi_smem = 0, phi_smem_few = 0, nbr_smem = 0, mb_smem = 0;
   // host mirrors
   uint64_t step_count = 1;     // learner.cc:37
   uint64_t average_count = 1;  // learner.cc:30
@@ -142,10 +143,29 @@ struct ammsb_handle {
   X(32, 8, 1) X(32, 8, 2) X(32, 8, 4) X(16, 1, 2) X(8, 1, 2) X(8, 1, 4) X(16, 2, 1)     \
   X(8, 2, 1) X(8, 4, 1) X(4, 2, 1) X(4, 4, 1) X(4, 1, 8) X(2, 1, 8) X(1, 1, 8)
 
-// Iterations with at most kRingFewNodes nodes (the link stratum) take a
-// kRingSplitWide-warp variant of the ring update_phi kernel.
+// Iterations with at most kRingFewNodes nodes (the link stratum) take the
+// ring update_phi kernel's 16 warps per node.
 constexpr int kRingFewNodes = 64;
-constexpr int kRingSplitWide = 16;
+
+// How the ring update_phi kernel is launched for rows whose four-warp group
+// takes group_bytes of shared memory and whose 16-warp node few_bytes: four
+// groups to the CTA and both kinds of iteration in one launch where that fits
+// an SM's 227 KB, else a launch per kind.
+struct RingPlan {
+  size_t group_bytes, few_bytes;
+  int groups;   // four-warp groups per CTA
+  int few;      // most nodes that take 16 warps each (0: none do)
+  bool single;  // one launch for both kinds
+  size_t smem() const { return few ? std::max((size_t)groups * group_bytes, few_bytes) : groups * group_bytes; }
+};
+inline RingPlan ring_plan(const KernelCfg& c, size_t group_bytes, size_t few_bytes) {
+  constexpr size_t kSmem = 227 * 1024;
+  RingPlan r{group_bytes, 0, 1, 0, false};
+  r.groups = (int)std::max<size_t>(1, std::min<size_t>(4, kSmem / group_bytes));
+  if (c.ring_few && few_bytes <= 200 * 1024) r.few = kRingFewNodes, r.few_bytes = few_bytes;
+  r.single = r.groups == 4;
+  return r;
+}
 
 // Ring depths the ring update_phi kernel is built for.
 #define AMMSB_PHI_RING_STAGES(X) X(3) X(4) X(6)

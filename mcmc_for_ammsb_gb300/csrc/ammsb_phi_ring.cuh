@@ -1,23 +1,19 @@
 // ammsb_phi_ring.cuh -- update_phi for wide pi rows (>= 512 bytes), with the
 // neighbour rows staged in shared memory through a per-warp ring.
 //
-// One CTA per minibatch node, SPLIT warps.  Warp g handles neighbours
-// g, g+SPLIT, ...: each of its lanes keeps its own 16-byte pieces of the
-// next STAGES rows in flight (cp.async global -> shared, one commit group
-// per row), waits for the row's group, reads back exactly the pieces it
-// copied and does the two FMA passes of the factored gradient (see
-// k_update_phi in ammsb_kernels.cuh for the algebra).  A lane never reads
-// another lane's pieces of a row, so the ring needs no barrier; the waits are
-// on the lane's own copies, which always complete.  (A variant with one
-// cp.async.bulk copy per row and an mbarrier per slot measured 5% slower:
-// its per-row barrier wait, warp vote, __syncwarp and single-lane issue cost
-// more than four 16-byte copies per lane.)
+// SPLIT warps per minibatch node.  Warp g handles neighbours g, g+SPLIT, ...:
+// each of its lanes keeps its own 16-byte pieces of the next rows in flight
+// (cp.async global -> shared, one commit group per chunk of U rows), waits
+// for the chunk's group, reads back exactly the pieces it copied and does the
+// two FMA passes of the factored gradient (see k_update_phi in
+// ammsb_kernels.cuh for the algebra).  A lane never reads another lane's
+// pieces of a row, so the ring needs no barrier; the waits are on the lane's
+// own copies, which always complete.  (A variant with one cp.async.bulk copy
+// per row and an mbarrier per slot measured 5% slower: its per-row barrier
+// wait, warp vote, __syncwarp and single-lane issue cost more than four
+// 16-byte copies per lane.)
 #pragma once
 #include "ammsb_kernels.cuh"
-
-#ifndef AMMSB_RING_WARP_PROLOGUE
-#define AMMSB_RING_WARP_PROLOGUE 0
-#endif
 
 namespace ammsb {
 
@@ -76,18 +72,29 @@ struct PairLoad<__nv_bfloat16> {
   }
 };
 
+// Rows taken together by a warp: their dot products' warp sums (five dependent
+// shuffles each, some 150 cycles) then overlap.  As many as keep a lane at 32
+// floats of rows or fewer beside its w and A; rows of 32 floats a lane (K =
+// 1024 BF16) are bound by HBM with 16 warps per SM and take one at a time.
+template <typename PiT, int VPL>
+__host__ __device__ constexpr int ring_rows() {
+  constexpr int EPL = VPL * PiTraits<PiT>::kPerVec;
+  return EPL <= 8 ? 4 : EPL <= 16 ? 2 : 1;
+}
+
 template <typename PiT, int VPL, int SPLIT, int STAGES>
 struct PhiRingSmem {
+  static constexpr int kRows = STAGES * ring_rows<PiT, VPL>();  // ring slots per warp
   // BF16 rows keep the node's phi row and normals in shared memory across
   // the rows (two more rows of floats)
   static constexpr bool kStash = sizeof(PiT) == 2;
   // the per-warp A vectors of the epilogue reuse the warp's own ring slice
-  static_assert(STAGES * sizeof(PiT) >= sizeof(float), "ring slice must hold a row of floats");
-  static size_t bytes(int Kp, int n_out) {
-    size_t ring = (size_t)SPLIT * STAGES * Kp * sizeof(PiT);
+  static_assert(kRows * sizeof(PiT) >= sizeof(float), "ring slice must hold a row of floats");
+  __host__ __device__ static size_t bytes(int Kp, int n_out) {
+    size_t ring = (size_t)SPLIT * kRows * Kp * sizeof(PiT);
     size_t w = (size_t)(kStash ? 3 : 1) * Kp * sizeof(float);
     size_t misc = (size_t)(4 * SPLIT + 8) * sizeof(float) + (size_t)n_out * sizeof(uint32_t);
-    return ring + w + misc + 128;
+    return (ring + w + misc + 127) / 128 * 128;
   }
 };
 
@@ -151,21 +158,35 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Each warp walks its rows in chunks of STAGES with the ring slot of every
-// row a compile-time constant, refilling each slot with the row STAGES ahead
-// as soon as the row's dot product has taken it into registers; every row
-// commits one group (empty past the node's last row), so
-// cp.async.wait_group STAGES-1 always means "this row is in".  The neighbour
-// word of the row in each slot rides in a register beside the slot.  When
-// FULL the row length is the compile-time 32 * VPL * EV, so row offsets and
-// sizes are constants.  A node's first STAGES rows are sent before its
-// prologue, which they overlap.  With BF16 rows (STASH) the node's phi row
-// and its normals are read and drawn in the prologue and kept in shared
-// memory for the epilogue.
-template <typename PiT, int VPL, int SPLIT, int STAGES, bool FULL>
-__device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffers& b) {
+// The threads of one node: a whole CTA of 16 warps, or one of its groups of
+// four warps (named barrier 1 + group).
+template <int SPLIT>
+__device__ __forceinline__ void node_sync(int group) {
+  if constexpr (SPLIT * 32 == 512)
+    __syncthreads();
+  else
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(SPLIT * 32) : "memory");
+}
+
+// Each warp walks its rows in chunks of U with the ring slots of every chunk
+// compile-time constants, refilling a chunk's slots with the rows STAGES
+// chunks ahead as soon as its dot products have taken it into registers; every
+// chunk commits one group (empty past the node's last row), so
+// cp.async.wait_group STAGES-1 always means "this chunk is in".  When FULL the
+// row length is the compile-time 32 * VPL * EV, so row offsets and sizes are
+// constants.  A node's first STAGES chunks are sent before its prologue, which
+// they overlap.  With BF16 rows (STASH) the node's phi row and its normals are
+// read and drawn in the prologue and kept in shared memory for the epilogue.
+// The first node of the `group` (of `groups` in the grid) is its own number;
+// with DYNAMIC it takes the next ones from the buffer set's counter, one fetch
+// per node, the last of which brings the counter back to zero: the SMs then
+// share the nodes as they finish, without a wave of short CTAs.
+template <typename PiT, int VPL, int SPLIT, int STAGES, bool FULL, bool DYNAMIC>
+__device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffers& b, unsigned char* s_raw,
+                                                     int group, int first, int groups) {
   using TR = PiTraits<PiT>;
   using Smem = PhiRingSmem<PiT, VPL, SPLIT, STAGES>;
+  constexpr int U = ring_rows<PiT, VPL>(), ROWS = Smem::kRows;
   constexpr int EV = TR::kPerVec;
   constexpr int EPL = VPL * EV;
   constexpr int NT = SPLIT * 32;
@@ -173,39 +194,41 @@ __device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffe
   constexpr bool STASH = Smem::kStash;
   // thread's elements of a row: k0 = 4 * (tid + NT * g) .. k0 + 3, g < NG
   constexpr int NG = (EPL * 32 + 4 * NT - 1) / (4 * NT);
-  extern __shared__ __align__(128) unsigned char s_raw[];
   const int Kp = FULL ? 32 * EPL : m.Kp;
   const int K = m.K, n_out = m.n_out;
   PiT* ring = reinterpret_cast<PiT*>(s_raw);
-  float* s_w = reinterpret_cast<float*>(ring + (size_t)SPLIT * STAGES * Kp);
+  float* s_w = reinterpret_cast<float*>(ring + (size_t)SPLIT * ROWS * Kp);
   float* s_phi = s_w + Kp;                    // STASH: the node's phi row
   float* s_nz = s_phi + Kp;                   // STASH: its normals
   float* s_red = s_w + (STASH ? 3 : 1) * Kp;  // 4*SPLIT + 8 floats
   uint32_t* s_nb = reinterpret_cast<uint32_t*>(s_red + 4 * SPLIT + 8);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x & (NT - 1), lane = tid & 31, warp = tid >> 5;
   const int n_nodes = b.st->n_nodes;
   const uint32_t step = b.st->step;
   const float eps_t = b.st->eps;
   const PiT* __restrict__ pi = reinterpret_cast<const PiT*>(b.pi);
   const int nvec = Kp / EV;
+  int* s_next = reinterpret_cast<int*>(s_red + 4 * SPLIT);
   const Stream rs{m.seed, m.chain};
 
-  PiT* my_ring = ring + (size_t)warp * STAGES * Kp;
+  PiT* my_ring = ring + (size_t)warp * ROWS * Kp;
   float* my_A = reinterpret_cast<float*>(my_ring);  // epilogue: this warp's A (Kp floats)
 
-  for (int slot = blockIdx.x; slot < n_nodes; slot += gridDim.x) {
+  int next = 0;
+  for (int slot = first; slot < n_nodes; slot = DYNAMIC ? next : slot + groups) {
+    if (DYNAMIC && tid == 0) next = groups + (int)atomicInc(&b.st->next_node, (unsigned)n_nodes - 1u);
     const int32_t i = b.nodes[slot];
     const float* phi_i = b.phi + (int64_t)i * Kp;
     const uint32_t* nbr_g = b.nbr + (int64_t)slot * n_out;
     // rows of this warp: q = warp + SPLIT * t, t < T
     const int T = (n_out > warp) ? (n_out - warp + SPLIT - 1) / SPLIT : 0;
-    // the first STAGES rows: ids read first, then every lane sends its
-    // pieces, one commit group per row (empty past T), before the node
-    // prologue, which they overlap
-    uint32_t j0[STAGES];
+    // the first chunks: ids read first, then every lane sends its pieces,
+    // one commit group per chunk (empty past T), before the node prologue,
+    // which they overlap
+    uint32_t j0[ROWS];
 #pragma unroll
-    for (int t = 0; t < STAGES; ++t) j0[t] = (t < T) ? (nbr_g[warp + SPLIT * t] & 0x7fffffffu) : 0u;
+    for (int t = 0; t < ROWS; ++t) j0[t] = (t < T) ? (nbr_g[warp + SPLIT * t] & 0x7fffffffu) : 0u;
     // (BF16) the thread's phi elements, loaded before the copies are sent
     float4 ph[STASH ? NG : 1];
     if constexpr (STASH) {
@@ -216,206 +239,156 @@ __device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffe
       }
     }
 #pragma unroll
-    for (int t = 0; t < STAGES; ++t) {
+    for (int t = 0; t < ROWS; ++t) {
       if (t < T) copy_row_lane<PiT, VPL, FULL>(my_ring + (size_t)t * Kp, pi + (int64_t)j0[t] * Kp, lane, nvec);
-      cp_async_commit();
+      if (t % U == U - 1) cp_async_commit();
     }
     float S, si;
     f32x2 w2[NP], A2[NP];
-    if constexpr (STASH && AMMSB_RING_WARP_PROLOGUE) {
-      // ---- node prologue, per warp (BF16 rows): every warp reads the whole
-      // phi row in its lanes' vector layout and forms S = sum phi,
-      // s_i = sum pi and w = pi * (beta - eps) with shuffles alone -- the same
-      // operations on the same values in every warp, so the warps agree bit
-      // for bit without a CTA barrier; the thread's own epilogue elements
-      // (phi and the normals) go to its private stash places
-      // the neighbour words of this warp's rows (q = warp + SPLIT t), which
-      // only this warp reads
-      for (int t = lane; t < T; t += 32) s_nb[warp + SPLIT * t] = nbr_g[warp + SPLIT * t];
+    // ---- node prologue: S = sum phi, s_i = sum pi, w = pi * (beta - eps)
+    S = 0.f;
+    if constexpr (STASH) {
+      for (int q = tid; q < n_out; q += NT) s_nb[q] = nbr_g[q];
 #pragma unroll
       for (int g = 0; g < NG; ++g) {
         const int k0 = 4 * (tid + NT * g);
         if (k0 < K) *reinterpret_cast<float4*>(s_nz + k0) = phi_normals(b, rs, slot, i, step, k0, K);
-        if (k0 < Kp) *reinterpret_cast<float4*>(s_phi + k0) = ph[g];
-      }
-      float phv[EPL];
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int vi = lane + 32 * v;
-#pragma unroll
-        for (int e = 0; e < EV; e += 4) {
-          const float4 q = (FULL || vi < nvec) ? *reinterpret_cast<const float4*>(phi_i + vi * EV + e)
-                                               : make_float4(0.f, 0.f, 0.f, 0.f);
-          phv[v * EV + e] = q.x;
-          phv[v * EV + e + 1] = q.y;
-          phv[v * EV + e + 2] = q.z;
-          phv[v * EV + e + 3] = q.w;
-        }
-      }
-      S = 0.f;
-#pragma unroll
-      for (int e = 0; e < EPL; e += 4) S += (phv[e] + phv[e + 1]) + (phv[e + 2] + phv[e + 3]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
-      const float rS = 1.0f / S;  // pi = phi / S as phi * (1/S): within 1 ulp
-      grid_dependency_wait();  // beta: written by the theta step ahead of this launch
-      grid_launch_dependents();
-      si = 0.f;
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int vi = lane + 32 * v;
-#pragma unroll
-        for (int e = 0; e < EV; e += 4) {
-          float4 bt = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (FULL || vi < nvec) bt = *reinterpret_cast<const float4*>(b.beta + vi * EV + e);
-          const int kb = vi * EV + e;
-          float pv[4], wv[4];
-          const float btv[4] = {bt.x, bt.y, bt.z, bt.w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            pv[u] = phv[v * EV + e + u] * rS;
-            si += pv[u];
-            wv[u] = (kb + u < K) ? pv[u] * (btv[u] - m.epsilon) : 0.f;
-          }
-          w2[(v * EV + e) / 2] = pack_f32x2(wv[0], wv[1]);
-          w2[(v * EV + e) / 2 + 1] = pack_f32x2(wv[2], wv[3]);
-          A2[(v * EV + e) / 2] = 0ull;
-          A2[(v * EV + e) / 2 + 1] = 0ull;
-        }
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) si += __shfl_xor_sync(0xffffffffu, si, o);
-      __syncwarp();  // the warp's neighbour words are in
+      for (int g = 0; g < NG; ++g) S += (ph[g].x + ph[g].y) + (ph[g].z + ph[g].w);
     } else {
-      // ---- node prologue: S = sum phi, s_i = sum pi, w = pi * (beta - eps)
-      S = 0.f;
-      if constexpr (STASH) {
-        for (int q = tid; q < n_out; q += NT) s_nb[q] = nbr_g[q];
+      for (int k = tid; k < Kp; k += NT) S += phi_i[k];
+      for (int q = tid; q < n_out; q += NT) s_nb[q] = nbr_g[q];
+    }
 #pragma unroll
-        for (int g = 0; g < NG; ++g) {
-          const int k0 = 4 * (tid + NT * g);
-          if (k0 < K) *reinterpret_cast<float4*>(s_nz + k0) = phi_normals(b, rs, slot, i, step, k0, K);
-        }
+    for (int o = 16; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
+    if (lane == 0) s_red[warp] = S;
+    node_sync<SPLIT>(group);
+    // beta, read from here on, is written by the theta step ahead of this
+    // launch; everything read before (node ids, neighbour words and rows,
+    // phi) was complete before that step started
+    grid_dependency_wait();
+    grid_launch_dependents();
+    S = 0.f;
 #pragma unroll
-        for (int g = 0; g < NG; ++g) S += (ph[g].x + ph[g].y) + (ph[g].z + ph[g].w);
-      } else {
-        for (int k = tid; k < Kp; k += NT) S += phi_i[k];
-        for (int q = tid; q < n_out; q += NT) s_nb[q] = nbr_g[q];
-      }
+    for (int w = 0; w < SPLIT; ++w) S += s_red[w];
+    si = 0.f;
+    if constexpr (STASH) {
+      const float rS = 1.0f / S;  // pi = phi / S as phi * (1/S): within 1 ulp
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
-      if (lane == 0) s_red[warp] = S;
-      __syncthreads();
-      // beta, read from here on, is written by the theta step ahead of this
-      // launch; everything read before (node ids, neighbour words and rows,
-      // phi) was complete before that step started
-      grid_dependency_wait();
-      grid_launch_dependents();
-      S = 0.f;
-#pragma unroll
-      for (int w = 0; w < SPLIT; ++w) S += s_red[w];
-      si = 0.f;
-      if constexpr (STASH) {
-        const float rS = 1.0f / S;  // pi = phi / S as phi * (1/S): within 1 ulp
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-          const int k0 = 4 * (tid + NT * g);
-          if (k0 < Kp) {
-            const float4 bt = *reinterpret_cast<const float4*>(b.beta + k0);
-            float4 p, wv;
-            p.x = ph[g].x * rS;
-            p.y = ph[g].y * rS;
-            p.z = ph[g].z * rS;
-            p.w = ph[g].w * rS;
-            si += p.x;
-            si += p.y;
-            si += p.z;
-            si += p.w;
-            wv.x = (k0 + 0 < K) ? p.x * (bt.x - m.epsilon) : 0.f;
-            wv.y = (k0 + 1 < K) ? p.y * (bt.y - m.epsilon) : 0.f;
-            wv.z = (k0 + 2 < K) ? p.z * (bt.z - m.epsilon) : 0.f;
-            wv.w = (k0 + 3 < K) ? p.w * (bt.w - m.epsilon) : 0.f;
-            *reinterpret_cast<float4*>(s_w + k0) = wv;
-            *reinterpret_cast<float4*>(s_phi + k0) = ph[g];
-          }
-        }
-      } else {
-        for (int k = tid; k < Kp; k += NT) {
-          const float p = __fdiv_rn(phi_i[k], S);
-          si += p;
-          s_w[k] = (k < K) ? p * (b.beta[k] - m.epsilon) : 0.f;
+      for (int g = 0; g < NG; ++g) {
+        const int k0 = 4 * (tid + NT * g);
+        if (k0 < Kp) {
+          const float4 bt = *reinterpret_cast<const float4*>(b.beta + k0);
+          float4 p, wv;
+          p.x = ph[g].x * rS;
+          p.y = ph[g].y * rS;
+          p.z = ph[g].z * rS;
+          p.w = ph[g].w * rS;
+          si += p.x;
+          si += p.y;
+          si += p.z;
+          si += p.w;
+          wv.x = (k0 + 0 < K) ? p.x * (bt.x - m.epsilon) : 0.f;
+          wv.y = (k0 + 1 < K) ? p.y * (bt.y - m.epsilon) : 0.f;
+          wv.z = (k0 + 2 < K) ? p.z * (bt.z - m.epsilon) : 0.f;
+          wv.w = (k0 + 3 < K) ? p.w * (bt.w - m.epsilon) : 0.f;
+          *reinterpret_cast<float4*>(s_w + k0) = wv;
+          *reinterpret_cast<float4*>(s_phi + k0) = ph[g];
         }
       }
+    } else {
+      for (int k = tid; k < Kp; k += NT) {
+        const float p = __fdiv_rn(phi_i[k], S);
+        si += p;
+        s_w[k] = (k < K) ? p * (b.beta[k] - m.epsilon) : 0.f;
+      }
+    }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) si += __shfl_xor_sync(0xffffffffu, si, o);
-      if (lane == 0) s_red[SPLIT + warp] = si;
-      __syncthreads();
-      si = 0.f;
+    for (int o = 16; o > 0; o >>= 1) si += __shfl_xor_sync(0xffffffffu, si, o);
+    if (lane == 0) s_red[SPLIT + warp] = si;
+    node_sync<SPLIT>(group);
+    si = 0.f;
 #pragma unroll
-      for (int w = 0; w < SPLIT; ++w) si += s_red[SPLIT + w];
+    for (int w = 0; w < SPLIT; ++w) si += s_red[SPLIT + w];
 #pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int vi = lane + 32 * v;
+    for (int v = 0; v < VPL; ++v) {
+      const int vi = lane + 32 * v;
 #pragma unroll
-        for (int e = 0; e < EV; e += 4) {
-          float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (FULL || vi < nvec) q = *reinterpret_cast<const float4*>(s_w + vi * EV + e);
-          w2[(v * EV + e) / 2] = pack_f32x2(q.x, q.y);
-          w2[(v * EV + e) / 2 + 1] = pack_f32x2(q.z, q.w);
-          A2[(v * EV + e) / 2] = 0ull;
-          A2[(v * EV + e) / 2 + 1] = 0ull;
-        }
+      for (int e = 0; e < EV; e += 4) {
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (FULL || vi < nvec) q = *reinterpret_cast<const float4*>(s_w + vi * EV + e);
+        w2[(v * EV + e) / 2] = pack_f32x2(q.x, q.y);
+        w2[(v * EV + e) / 2 + 1] = pack_f32x2(q.z, q.w);
+        A2[(v * EV + e) / 2] = 0ull;
+        A2[(v * EV + e) / 2 + 1] = 0ull;
       }
     }
     // the per-row constants of y = 1 and y = 0
     const float one_m_si = 1.0f - si;
     const float e1si = m.epsilon * si, e0si = (1.0f - m.epsilon) * si;
     const float e1o = m.epsilon * one_m_si, e0o = (1.0f - m.epsilon) * one_m_si;
-    // neighbour word of the row in each ring slot
-    uint32_t nbw[STAGES];
-#pragma unroll
-    for (int u = 0; u < STAGES; ++u) nbw[u] = (u < T) ? s_nb[warp + SPLIT * u] : 0u;
     float Bsum = 0.f;
-    for (int t0 = 0; t0 < T; t0 += STAGES) {
+    for (int t0 = 0; t0 < T; t0 += ROWS) {
 #pragma unroll
       for (int u = 0; u < STAGES; ++u) {
-        const int t = t0 + u;
+        const int t = t0 + u * U;  // rows t .. t + U - 1, in slots u * U ..
         if (t >= T) break;
-        // one group per row, so the lane's pieces of row t are in once no
+        // one group per chunk, so the lane's pieces of it are in once no
         // more than the STAGES - 1 later groups are pending
         cp_async_wait<STAGES - 1>();
-        // neighbour word of the row that refills this slot, read early
-        const int tn = t + STAGES;
-        const uint32_t nxt = (tn < T) ? s_nb[warp + SPLIT * tn] : nbw[u];
-        const bool y = (nbw[u] >> 31) != 0;
-        const PiT* row = my_ring + (size_t)u * Kp;
-        f32x2 x2[NP];
-        load_row_pairs<PiT, VPL, FULL>(row, lane, nvec, x2);
-        // four independent pair accumulators break the FMA dependency chain
-        f32x2 d2[4] = {0ull, 0ull, 0ull, 0ull};
+        // neighbour words of the rows, and of those that refill their slots
+        uint32_t nbw[U], nxt[U];
+        f32x2 x2[U][NP], d2[U][4];
 #pragma unroll
-        for (int e = 0; e < NP; ++e) d2[e & 3] = fma_f32x2(w2[e], x2[e], d2[e & 3]);
-        // refill the lane's pieces of slot u (read above, now in registers)
-        // with row t + STAGES
-        if (tn < T) copy_row_lane<PiT, VPL, FULL>(my_ring + (size_t)u * Kp, pi + (int64_t)(nxt & 0x7fffffffu) * Kp, lane, nvec);
-        cp_async_commit();
-        nbw[u] = nxt;
-        float D;
-        {
-          float lo, hi;
-          unpack_f32x2(add_f32x2(add_f32x2(d2[0], d2[1]), add_f32x2(d2[2], d2[3])), lo, hi);
-          D = lo + hi;
+        for (int r = 0; r < U; ++r) {
+          const int tn = t + r + ROWS;
+          nbw[r] = (r == 0 || t + r < T) ? s_nb[warp + SPLIT * (t + r)] : 0u;
+          nxt[r] = (tn < T) ? s_nb[warp + SPLIT * tn] : 0u;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) D += __shfl_xor_sync(0xffffffffu, D, o);
-        const float Ds = y ? D : -D;
-        const float P = Ds + (y ? e1si : e0si);
-        const float invP = rcp_approx(P);
-        const float cj = y ? invP : -invP;
-        Bsum += ((y ? e1o : e0o) - Ds) * invP;
-        const f32x2 c2 = pack_f32x2(cj, cj);
+        for (int r = 0; r < U; ++r) {
+          if (r > 0 && t + r >= T) break;
+          load_row_pairs<PiT, VPL, FULL>(my_ring + (size_t)(u * U + r) * Kp, lane, nvec, x2[r]);
+          // four independent pair accumulators break the FMA dependency chain
 #pragma unroll
-        for (int e = 0; e < NP; ++e) A2[e] = fma_f32x2(c2, x2[e], A2[e]);
+          for (int e = 0; e < 4; ++e) d2[r][e] = 0ull;
+#pragma unroll
+          for (int e = 0; e < NP; ++e) d2[r][e & 3] = fma_f32x2(w2[e], x2[r][e], d2[r][e & 3]);
+        }
+        // refill the lane's pieces of the chunk's slots (read above, now in
+        // registers)
+#pragma unroll
+        for (int r = 0; r < U; ++r)
+          if (t + r + ROWS < T)
+            copy_row_lane<PiT, VPL, FULL>(my_ring + (size_t)(u * U + r) * Kp,
+                                          pi + (int64_t)(nxt[r] & 0x7fffffffu) * Kp, lane, nvec);
+        cp_async_commit();
+        float D[U];
+#pragma unroll
+        for (int r = 0; r < U; ++r) {
+          float lo = 0.f, hi = 0.f;
+          if (r == 0 || t + r < T)
+            unpack_f32x2(add_f32x2(add_f32x2(d2[r][0], d2[r][1]), add_f32x2(d2[r][2], d2[r][3])), lo, hi);
+          D[r] = lo + hi;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int r = 0; r < U; ++r) D[r] += __shfl_xor_sync(0xffffffffu, D[r], o);
+#pragma unroll
+        for (int r = 0; r < U; ++r) {
+          if (r > 0 && t + r >= T) break;
+          const bool y = (nbw[r] >> 31) != 0;
+          const float Ds = y ? D[r] : -D[r];
+          const float P = Ds + (y ? e1si : e0si);
+          const float invP = rcp_approx(P);
+          const float cj = y ? invP : -invP;
+          Bsum += ((y ? e1o : e0o) - Ds) * invP;
+          const f32x2 c2 = pack_f32x2(cj, cj);
+#pragma unroll
+          for (int e = 0; e < NP; ++e) A2[e] = fma_f32x2(c2, x2[r][e], A2[e]);
+        }
       }
     }
     // every copy of the node is in (the groups after the last row are
@@ -436,7 +409,9 @@ __device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffe
       }
     }
     if (lane == 0) s_red[2 * SPLIT + warp] = Bsum;
-    __syncthreads();
+    if (DYNAMIC && tid == 0) *s_next = next;
+    node_sync<SPLIT>(group);
+    if (DYNAMIC) next = *s_next;
     float Bt = 0.f;
 #pragma unroll
     for (int w2i = 0; w2i < SPLIT; ++w2i) Bt += s_red[2 * SPLIT + w2i];
@@ -471,7 +446,7 @@ __device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffe
 #pragma unroll
         for (int s = 0; s < SPLIT; ++s) {
           const float4 a = *reinterpret_cast<const float4*>(
-              reinterpret_cast<const float*>(ring + (size_t)s * STAGES * Kp) + k0);
+              reinterpret_cast<const float*>(ring + (size_t)s * ROWS * Kp) + k0);
           Ak[0] += a.x;
           Ak[1] += a.y;
           Ak[2] += a.z;
@@ -505,7 +480,7 @@ __device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffe
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) Snew += __shfl_xor_sync(0xffffffffu, Snew, o);
     if (lane == 0) s_red[3 * SPLIT + warp] = Snew;
-    __syncthreads();
+    node_sync<SPLIT>(group);
     Snew = 0.f;
 #pragma unroll
     for (int w2i = 0; w2i < SPLIT; ++w2i) Snew += s_red[3 * SPLIT + w2i];
@@ -523,37 +498,51 @@ __device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffe
         *reinterpret_cast<float4*>(st + k0) = o;
       }
     }
-    __syncthreads();  // smem reuse by the next node
+    node_sync<SPLIT>(group);  // smem reuse by the next node
   }
 }
-// The iteration's node count picks the launch that does the work: the
-// kernel runs when n_lo < n_nodes <= n_hi and returns at once otherwise.
-// Iterations with few nodes (the link stratum: one vertex and its edges)
-// take a 16-warp variant, whose warps each hold a quarter of the rows the
-// 4-warp one gives them, so a node's rows are in flight together.
-// Blocks per SM the register budget is sized for: 16 warps per SM.
-template <int SPLIT>
-constexpr int ring_min_blocks() { return SPLIT >= 16 ? 1 : 16 / SPLIT; }
-template <typename PiT, int VPL, int SPLIT, int STAGES, bool FULL>
-__global__ void __launch_bounds__(SPLIT * 32, ring_min_blocks<SPLIT>())
-    k_update_phi_ring(Model m, Buffers b, int n_lo, int n_hi) {
+// One launch for both kinds of iteration, which the node count picks: up to
+// `few` nodes (the link stratum: one vertex and its edges) take 16 warps each,
+// a node per CTA, so that a node's rows are in flight together; more take
+// four warps each, four nodes to the CTA.  (With a launch per kind, the one
+// without work stood between the theta step and the update: 5 us of a
+// link-stratum iteration.)  A CTA of 16 warps at up to 128 registers fills an
+// SM.  `parts`: the kinds this launch may do (kPhiFew, kPhiMany); ring depths
+// of which four groups do not fit shared memory take a launch per kind, the
+// second with as many groups per CTA as fit.
+constexpr int kPhiFew = 1, kPhiMany = 2;
+constexpr int kPhiGroup = 4 * 32;  // threads of a four-warp node
+template <typename PiT>
+__host__ __device__ constexpr int ring_few_stages() { return sizeof(PiT) == 2 ? 4 : 2; }
+
+template <typename PiT, int VPL, int STAGES, bool FULL>
+__device__ __forceinline__ void update_phi_ring_any(const Model& m, const Buffers& b, int few, int parts) {
+  extern __shared__ __align__(128) unsigned char s_ring[];
+  const int n_nodes = b.st->n_nodes;
+  if (n_nodes <= few) {
+    if (parts & kPhiFew)
+      update_phi_ring_body<PiT, VPL, 16, ring_few_stages<PiT>(), FULL, false>(m, b, s_ring, 0, blockIdx.x,
+                                                                              gridDim.x);
+  } else if (parts & kPhiMany) {
+    const int per = blockDim.x / kPhiGroup, group = threadIdx.x / kPhiGroup;
+    const int Kp = FULL ? 32 * VPL * PiTraits<PiT>::kPerVec : m.Kp;
+    update_phi_ring_body<PiT, VPL, 4, STAGES, FULL, true>(
+        m, b, s_ring + group * PhiRingSmem<PiT, VPL, 4, STAGES>::bytes(Kp, m.n_out), group,
+        blockIdx.x * per + group, gridDim.x * per);
+  }
   // CTAs with no work wait for the kernel ahead before they exit, so that
   // this launch completes after it
-  const int n_nodes = b.st->n_nodes;
-  if (n_nodes <= n_lo || n_nodes > n_hi) {
-    grid_dependency_wait();
-    return;
-  }
-  update_phi_ring_body<PiT, VPL, SPLIT, STAGES, FULL>(m, b);
+  grid_dependency_wait();
 }
-template <typename PiT, int VPL, int SPLIT, int STAGES, bool FULL>
-__global__ void __launch_bounds__(SPLIT * 32, ring_min_blocks<SPLIT>())
-    k_update_phi_ring_chains(const ChainArgs* __restrict__ c, int p, int n_lo, int n_hi) {
+template <typename PiT, int VPL, int STAGES, bool FULL>
+__global__ void __launch_bounds__(512, 1) k_update_phi_ring(Model m, Buffers b, int few, int parts) {
+  update_phi_ring_any<PiT, VPL, STAGES, FULL>(m, b, few, parts);
+}
+template <typename PiT, int VPL, int STAGES, bool FULL>
+__global__ void __launch_bounds__(512, 1) k_update_phi_ring_chains(const ChainArgs* __restrict__ c, int p, int few,
+                                                                   int parts) {
   const ChainArgs& a = c[blockIdx.y];
-  const Buffers b = slot_buffers(a.m, a.b, p);
-  const int n_nodes = b.st->n_nodes;
-  if (n_nodes <= n_lo || n_nodes > n_hi) return;
-  update_phi_ring_body<PiT, VPL, SPLIT, STAGES, FULL>(a.m, b);
+  update_phi_ring_any<PiT, VPL, STAGES, FULL>(a.m, slot_buffers(a.m, a.b, p), few, parts);
 }
 
 }  // namespace ammsb
