@@ -331,7 +331,8 @@ int ammsb_perplexity_noalloc(const void *pi, int32_t pi_dtype, int64_t K,
  * (stride ld_pi), theta K x 2.  Pairs are grouped by source: the pairs of
  * source a are q in [src_ptr[a], src_ptr[a+1]), with neighbour row
  * pair_nbr[q] and label pair_y[q].  The forward writes *loss (device) and
- * keeps p_q and the row sums in `workspace` (caller-owned device memory of
+ * keeps p_q, the row sums and each source's summed gradient terms in
+ * `workspace` (caller-owned device memory of
  * ammsb_edge_loglik_workspace_size bytes); the backward reads them back, so
  * the two calls share one workspace and the same inputs.  Index errors in
  * the pair arrays skip the pair and set bit 1 of the workspace's status
@@ -367,6 +368,28 @@ int ammsb_edge_loglik_backward(int32_t dtype, int64_t K, const void *phi_src,
 /* Status word of a workspace (bits above); synchronises `stream`. */
 int ammsb_edge_loglik_status(const void *workspace, void *stream,
                              int32_t *flags);
+
+/* Groups a pair list (src[q], nbr[q], y[q]), q < n_pairs, by source and by
+ * neighbour into the arrays above: pair_src, pair_nbr and pair_y are the pairs
+ * in a stable order by source and src_ptr its row pointers (n_src + 1);
+ * nbr_pairs are the positions of that order in a stable order by neighbour,
+ * nbr_ptr its row pointers (n_nbr + 1).  Device arrays.  src_keys >= n_src and
+ * nbr_keys >= n_nbr bound the indices (ammsb_check_pairs gives the largest);
+ * pairs at or above n_src or n_nbr come last and under no row.  A pair with an
+ * index below zero or past its bound is put under some row with pair_nbr = -1,
+ * which the forward skips and flags.  Kernels are queued on `stream`; workspace
+ * is caller-owned device memory of ammsb_group_pairs_workspace_size bytes. */
+size_t ammsb_group_pairs_workspace_size(int64_t n_pairs);
+int ammsb_group_pairs(const int64_t *src, const int64_t *nbr,
+                      const uint8_t *y, int64_t n_pairs, int64_t n_src,
+                      int64_t n_nbr, int64_t src_keys, int64_t nbr_keys,
+                      int64_t *src_ptr, int32_t *pair_nbr, uint8_t *pair_y,
+                      int32_t *pair_src, int64_t *nbr_ptr, int32_t *nbr_pairs,
+                      void *workspace, void *stream);
+/* bounds[0..3] (host) = smallest and largest source, smallest and largest
+ * neighbour; n_pairs >= 1.  Same workspace; synchronises `stream`. */
+int ammsb_check_pairs(const int64_t *src, const int64_t *nbr, int64_t n_pairs,
+                      void *workspace, void *stream, int64_t *bounds);
 
 /* ------------------------------------------------------------------------ */
 /* Host-side data preparation (no GPU use).                                 */

@@ -158,6 +158,11 @@ SIGNATURES = [
       ctypes.c_double, _P, ctypes.c_int64, _P, _P, ctypes.c_int64, _P, _P, _P, _P, _P, _P, _P, _P,
       _P]),
     ("ammsb_edge_loglik_status", ctypes.c_int, [_P, _P, _I32P]),
+    ("ammsb_group_pairs_workspace_size", ctypes.c_size_t, [ctypes.c_int64]),
+    ("ammsb_group_pairs", ctypes.c_int,
+     [_P, _P, _P, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64,
+      _P, _P, _P, _P, _P, _P, _P, _P]),
+    ("ammsb_check_pairs", ctypes.c_int, [_P, _P, ctypes.c_int64, _P, _P, _I64P]),
     ("ammsb_generate_graph", ctypes.c_int, [ctypes.POINTER(AmmsbGenParams), ctypes.POINTER(_P)]),
     ("ammsb_graph_from_edges", ctypes.c_int, [ctypes.c_int64, ctypes.c_int64, _I32P, _I32P,
                                               ctypes.POINTER(_P)]),

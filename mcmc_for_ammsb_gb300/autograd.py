@@ -13,8 +13,8 @@ update_beta gradient (cc:212-240): the SGRLD drift.  The gradient in pi_nbr
 is the same expression's derivative in the neighbour row.
 
 Tensors must be CUDA tensors of one dtype (float32 or float64); there is no
-CPU path.  The backward recomputes every per-pair K-vector from the rows and
-keeps only p_q and the row sums from the forward.
+CPU path.  The forward keeps p_q, the row sums and each source's summed
+gradient terms, so that the backward gathers no neighbour row again.
 """
 import ctypes
 
@@ -117,10 +117,57 @@ class EdgeLogLikelihood(torch.autograd.Function):
                 None, None, None, None, None, None, None)
 
 
+def _pair_workspace(src):
+    size = _native.lib().ammsb_group_pairs_workspace_size(src.shape[0])
+    return torch.empty(size, dtype=torch.uint8, device=src.device)
+
+
+def _group_cuda(src, nbr, y, n_src, n_nbr, src_keys, nbr_keys, ws):
+    """The groupings of int64 / uint8 pair lists (ammsb_group_pairs)."""
+    dev = src.device
+    n = src.shape[0]
+    ptr = torch.empty(n_src + 1 + n_nbr + 1, dtype=torch.int64, device=dev)
+    src_ptr, nbr_ptr = ptr[:n_src + 1], ptr[n_src + 1:]
+    words = torch.empty(3, n, dtype=torch.int32, device=dev)
+    pair_nbr, pair_src, nbr_pairs = words[0], words[1], words[2]
+    pair_y = torch.empty(n, dtype=torch.uint8, device=dev)
+    _native.check(_native.lib().ammsb_group_pairs(
+        _ptr(src), _ptr(nbr), _ptr(y), n, n_src, n_nbr, src_keys, nbr_keys, _ptr(src_ptr),
+        _ptr(pair_nbr), _ptr(pair_y), _ptr(pair_src), _ptr(nbr_ptr), _ptr(nbr_pairs), _ptr(ws),
+        _stream(dev)))
+    return src_ptr, pair_nbr, pair_y, pair_src, nbr_ptr, nbr_pairs
+
+
+def _as_lists(src, nbr, y):
+    return (src.to(torch.int64).contiguous(), nbr.to(torch.int64).contiguous(),
+            y.to(torch.uint8).contiguous())
+
+
 def group_pairs(src, nbr, y, n_src, n_nbr):
     """Groups a pair list (src, nbr, y: 1-D CUDA tensors) by source and by
     neighbour: returns (src_ptr, pair_nbr, pair_y, pair_src, nbr_ptr,
     nbr_pairs) in the layout EdgeLogLikelihood takes."""
+    if not src.is_cuda:
+        return _group_torch(src, nbr, y, n_src, n_nbr)
+    src, nbr, y = _as_lists(src, nbr, y)
+    if nbr.shape[0] < src.shape[0] or y.shape[0] < src.shape[0]:
+        raise IndexError("pair lists of different lengths")
+    ws = _pair_workspace(src)
+    src_keys, nbr_keys = n_src, n_nbr
+    if src.shape[0]:
+        bounds = (ctypes.c_int64 * 4)()
+        _native.check(_native.lib().ammsb_check_pairs(_ptr(src), _ptr(nbr), src.shape[0], _ptr(ws),
+                                                      _stream(src.device), bounds))
+        if bounds[0] < 0 or bounds[2] < 0:
+            raise RuntimeError("pair indices must not be negative")
+        if max(bounds[1], bounds[3]) >= 1 << 31:
+            raise IndexError("pair indices out of range")
+        src_keys, nbr_keys = max(n_src, bounds[1] + 1), max(n_nbr, bounds[3] + 1)
+    return _group_cuda(src, nbr, y, n_src, n_nbr, src_keys, nbr_keys, ws)
+
+
+def _group_torch(src, nbr, y, n_src, n_nbr):
+    """group_pairs of CPU tensors, in plain torch."""
     dev = src.device
     src = src.to(torch.int64)
     nbr = nbr.to(torch.int64)
@@ -145,10 +192,12 @@ def edge_log_likelihood(phi_src, pi_nbr, theta, src, nbr, y, epsilon):
         raise RuntimeError("pair arrays must be CUDA tensors: the edge log-likelihood runs on "
                            "the GPU only")
     n_src, n_nbr = phi_src.shape[0], pi_nbr.shape[0]
-    if src.numel():
-        lo = torch.stack([src.min(), nbr.min()]).cpu()
-        hi = torch.stack([src.max(), nbr.max()]).cpu()
-        if int(lo.min()) < 0 or int(hi[0]) >= n_src or int(hi[1]) >= n_nbr:
-            raise IndexError("pair indices out of range")
-    groups = group_pairs(src, nbr, y, n_src, n_nbr)
+    src, nbr, y = _as_lists(src, nbr, y)
+    if nbr.shape[0] < src.shape[0] or y.shape[0] < src.shape[0]:
+        raise IndexError("pair lists of different lengths")
+    if src.shape[0] and (n_src == 0 or n_nbr == 0):
+        raise IndexError("pair indices out of range")
+    # an index out of range marks its pair, which the forward flags: the
+    # status it reads anyway raises the IndexError
+    groups = _group_cuda(src, nbr, y, n_src, n_nbr, n_src, n_nbr, _pair_workspace(src))
     return EdgeLogLikelihood.apply(phi_src, pi_nbr, theta, *groups, epsilon)

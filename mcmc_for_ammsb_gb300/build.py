@@ -18,7 +18,8 @@ LIB = os.path.join(HERE, "libammsb_gpu.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
                      "-Xcompiler", "-Wall", "-diag-suppress", "177"]
-SOURCES = ["ammsb_gpu.cu", "ammsb_batch.cu", "ammsb_host.cpp", "ammsb_noalloc.cu", "ammsb_adjoint.cu"]
+SOURCES = ["ammsb_gpu.cu", "ammsb_batch.cu", "ammsb_host.cpp", "ammsb_noalloc.cu", "ammsb_adjoint.cu",
+           "ammsb_group.cu"]
 # a standalone measurement executable, not part of the library: the
 # random-row gather rate (bench.py --gather-roofline), built on demand
 PROBE_SRC = "gather_roofline.cu"
