@@ -296,7 +296,7 @@ int ammsb_load_checkpoint(ammsb_handle *h, const char *path);
  * row padding holds does not matter.  A pair naming a row outside
  * [0, n_rows) is skipped on the device, before any row is read, and the
  * call returns AMMSB_E_ARG (the other pairs' running averages are
- * updated).  Its scratch is a fixed 256 KB __device__ array, so held_count
+ * updated).  Its scratch is a fixed 128 KB __device__ array, so held_count
  * is limited to 4,194,304 (AMMSB_E_CAPACITY beyond).  The array is shared
  * by every call on a device and keeps the last call's contents: calls whose
  * kernels overlap on the GPU race.  The first call on a device looks up the

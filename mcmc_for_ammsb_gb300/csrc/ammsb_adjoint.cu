@@ -63,8 +63,10 @@ __device__ __forceinline__ T group_sum(T v, uint32_t mask) {
 }
 template <int G>
 __device__ __forceinline__ uint32_t lane_group_mask() {
-  if constexpr (G >= 32) return 0xffffffffu;
-  return ((1u << G) - 1u) << ((threadIdx.x & 31) / G * G);
+  if constexpr (G >= 32)
+    return 0xffffffffu;
+  else
+    return ((1u << G) - 1u) << ((threadIdx.x & 31) / G * G);
 }
 
 // workspace: [err word | beta - eps (K) | S, B, ll (n_src) | p (n_pairs) |

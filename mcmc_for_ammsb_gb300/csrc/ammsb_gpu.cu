@@ -186,13 +186,13 @@ cudaError_t launch_commit(ammsb_handle* h, const Buffers& b, bool pdl = false) {
 template <typename PiT>
 cudaError_t launch_ppx(ammsb_handle* h, float count) {
   const PiT* pi = reinterpret_cast<const PiT*>(h->b.pi);
-  const int nb = h->ppx_blocks;
-#define PPX_CASE(L, V)                                                                         \
-  if (h->cfg.ppx_lpn == L && h->cfg.ppx_vpl == V) {                                            \
-    k_perplexity<PiT, L, V><<<nb, 256, 0, h->stream>>>(h->m, pi, h->b.beta, h->d_ha, h->d_hb, \
-                                                       h->d_hy, h->H, h->d_ppx, count,        \
-                                                       h->d_ppx_part, h->m.N, nullptr);       \
-    return cudaGetLastError();                                                                 \
+  const PpxPlan plan = ppx_plan(h->cfg.ppx_lpn, h->H);
+#define PPX_CASE(L, V)                                                                             \
+  if (h->cfg.ppx_lpn == L && h->cfg.ppx_vpl == V) {                                                \
+    k_perplexity<PiT, L, V><<<plan.blocks, 256, 0, h->stream>>>(                                   \
+        h->m, pi, h->b.beta, h->d_ha, h->d_hb, h->d_hy, h->H, plan.per_block, h->d_ppx, count,     \
+        h->d_ppx_part, h->m.N, h->gc, h->d_ppx_res);                                               \
+    return cudaGetLastError();                                                                     \
   }
   PPX_CASE(1, 1) PPX_CASE(2, 1) PPX_CASE(4, 1) PPX_CASE(8, 1) PPX_CASE(16, 1) PPX_CASE(32, 1)
   PPX_CASE(32, 2) PPX_CASE(32, 4) PPX_CASE(32, 8)
@@ -439,17 +439,19 @@ void print_stats(const ammsb_handle* h) {
   std::fflush(stdout);
 }
 
+// Device error bits as a status and message.
+int device_err_status(ammsb_handle* h, int32_t bits) {
+  if (!bits) return AMMSB_OK;
+  h->err = "device error bits " + std::to_string(bits) +
+           " (1 minibatch cap, 2 neighbour cap, 4 capacity, 8 init cap)";
+  return (bits & kErrCapacity) ? AMMSB_E_CAPACITY : AMMSB_E_SAMPLING;
+}
+
 int check_device_err(ammsb_handle* h) {
   DevCounters gc;
   CK(cudaMemcpyAsync(&gc, h->gc, sizeof(gc), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (gc.err) {
-    h->err = "device error bits " + std::to_string(gc.err) +
-             " (1 minibatch cap, 2 neighbour cap, 4 capacity, 8 init cap)";
-    if (gc.err & kErrCapacity) return AMMSB_E_CAPACITY;
-    return AMMSB_E_SAMPLING;
-  }
-  return AMMSB_OK;
+  return device_err_status(h, gc.err);
 }
 
 // The error bits of a drawn, not yet applied, iteration as a status.
@@ -457,10 +459,7 @@ int check_draw_err(ammsb_handle* h, int slot) {
   DevState st;
   CK(cudaMemcpyAsync(&st, ring_set(h, slot).st, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
   int rc = check_device_err(h);  // synchronises
-  if (rc || !st.err) return rc;
-  h->err = "device error bits " + std::to_string(st.err) +
-           " (1 minibatch cap, 2 neighbour cap, 4 capacity, 8 init cap)";
-  return (st.err & kErrCapacity) ? AMMSB_E_CAPACITY : AMMSB_E_SAMPLING;
+  return rc ? rc : device_err_status(h, st.err);
 }
 
 // Drops draws made ahead of time (their step no longer follows, or their
@@ -821,12 +820,8 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
       return bail(AMMSB_E_CUDA);
     }
   }
-  {
-    const int gpb = 256 / h->cfg.ppx_lpn;
-    h->ppx_blocks = (int)std::max<int64_t>(1, std::min<int64_t>((h->H + gpb - 1) / gpb, 152 * 8));
-  }
-  TRY(dev_alloc(h, &h->d_ppx_part, 2 * (size_t)h->ppx_blocks));
-  TRY(dev_alloc(h, &h->d_ppx_out, 1));
+  TRY(dev_alloc(h, &h->d_ppx_part, (size_t)std::max(1, ppx_plan(h->cfg.ppx_lpn, h->H).blocks)));
+  TRY(dev_alloc(h, &h->d_ppx_res, 1));
   // model state
   void* d_pi = nullptr;
   {
@@ -1196,14 +1191,19 @@ int ammsb_perplexity(ammsb_handle* h, double* out) {
   }
   CK(cudaSetDevice(h->device));
   const float count = (float)h->average_count;
+  double v = 0.0;
+  int rc = AMMSB_OK;
   if (h->H > 0) {
     CK(h->opt.pi_dtype == AMMSB_PI_BF16 ? launch_ppx<__nv_bfloat16>(h, count) : launch_ppx<float>(h, count));
+    // the value and the error bits of the iterations before it in one copy
+    PpxResult res;
+    CK(cudaMemcpyAsync(&res, h->d_ppx_res, sizeof(res), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    v = res.value;
+    rc = device_err_status(h, res.err);
+  } else {
+    rc = check_device_err(h);
   }
-  k_ppx_final<<<1, kPpxFinalThreads, 0, h->stream>>>(h->d_ppx_part, h->H > 0 ? h->ppx_blocks : 0, h->H, h->d_ppx_out);
-  CK(cudaGetLastError());
-  double v = 0.0;
-  CK(cudaMemcpyAsync(&v, h->d_ppx_out, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  int rc = check_device_err(h);  // synchronises
   if (rc) return rc;
   h->average_count++;
   *out = v;

@@ -78,8 +78,7 @@ struct ammsb_handle {
   uint8_t* d_hy = nullptr;
   float* d_ppx = nullptr;
   double* d_ppx_part = nullptr;
-  double* d_ppx_out = nullptr;
-  int ppx_blocks = 1;
+  PpxResult* d_ppx_res = nullptr;
   float* d_fed_phi_noise = nullptr;
   float* d_fed_theta_noise = nullptr;
   int32_t* d_err_init = nullptr;

@@ -1412,21 +1412,70 @@ static __global__ void __launch_bounds__(kThetaThreads) k_theta_chains(const Cha
 // ---------------------------------------------------------------------------
 // Held-out perplexity (learner.cc:138-183, learner.h:100-139): LPN lanes per
 // held-out edge; running average per edge in FP32 as the reference; the log
-// sum in FP64 with Kahan compensation, block partials, then k_ppx_final.
+// sum in FP64.  A block takes PpxPlan::per_block consecutive edges; their
+// averages go through shared memory so that the logarithms are taken by a
+// thread each (one lane's FP64 logarithm costs its warp as much as 32: with
+// the lane that formed the average taking it, 86,246 pairs of K = 1024 BF16
+// took 262 us, of which the rows are 53).  The block that finishes last adds
+// the blocks' partials, in a fixed order, so the result does not depend on
+// which it is; one thread adding a block's 256 values, and a second launch for
+// the partials, were 20 us of a small set's call.
 // ---------------------------------------------------------------------------
+struct PpxResult {
+  double value;
+  int32_t err;    // DevCounters::err when the call ran
+  uint32_t bad;   // a pair named a row outside pi
+  uint32_t done;  // blocks finished: zero between calls
+  uint32_t pad;
+};
+
+// Edges a block's lane groups take at a time (up to four each), and edges and
+// blocks of a call: at most kPpxMaxBlocks partials.
+constexpr int kPpxMaxBlocks = 16384;
+struct PpxPlan {
+  int per_block, blocks;
+};
+__host__ __device__ constexpr int ppx_chunk(int lpn) { return 4 * (256 / lpn) < 256 ? 4 * (256 / lpn) : 256; }
+inline PpxPlan ppx_plan(int lpn, int64_t H) {
+  const int64_t chunk = ppx_chunk(lpn), need = (H + kPpxMaxBlocks - 1) / kPpxMaxBlocks;
+  const int64_t per = (need < 1 ? 1 : (need + chunk - 1) / chunk) * chunk;
+  return PpxPlan{(int)per, (int)((H + per - 1) / per)};
+}
+
+// Sum of one value per thread of a 256-thread block (pairwise, fixed order),
+// in thread 0.
+__device__ __forceinline__ double block_sum_256(double v, double* s) {
+  const int tid = threadIdx.x;
+  s[tid] = v;
+  __syncthreads();
+#pragma unroll
+  for (int w = 128; w >= 32; w >>= 1) {
+    if (tid < w) s[tid] += s[tid + w];
+    __syncthreads();
+  }
+  if (tid >= 32) return 0.0;
+  v = s[tid];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+
 template <typename PiT, int LPN, int VPL>
 __global__ void __launch_bounds__(256) k_perplexity(Model m, const PiT* __restrict__ pi,
                                                     const float* __restrict__ beta,
                                                     const int32_t* __restrict__ ha,
                                                     const int32_t* __restrict__ hb,
-                                                    const uint8_t* __restrict__ hy, int64_t H,
+                                                    const uint8_t* __restrict__ hy, int64_t H, int per_block,
                                                     float* __restrict__ ppx, float count,
                                                     double* __restrict__ part, int64_t n_rows,
-                                                    unsigned int* __restrict__ bad) {
+                                                    const DevCounters* gc, PpxResult* res) {
   using TR = PiTraits<PiT>;
   constexpr int EV = TR::kPerVec;
   constexpr int EPL = VPL * EV;
-  constexpr int GPB = 256 / LPN;
+  constexpr int GPB = 256 / LPN, CH = ppx_chunk(LPN), J = CH / GPB;
+  __shared__ float s_avg[CH];
+  __shared__ double s_sum[256];
+  __shared__ int s_last;
   const int tid = threadIdx.x, grp = tid / LPN, l = tid % LPN, lane = tid & 31;
   const uint32_t gmask = group_mask<LPN>(lane);
   // rows are Kp apart; only the vectors that hold the K values are read,
@@ -1440,93 +1489,106 @@ __global__ void __launch_bounds__(256) k_perplexity(Model m, const PiT* __restri
       const int k = (l + LPN * v) * EV + e;
       bt[v * EV + e] = (k < K) ? beta[k] : 0.f;
     }
+  const int64_t e0 = (int64_t)blockIdx.x * per_block;
+  const int64_t e1 = e0 + per_block < H ? e0 + per_block : H;
   double sum = 0.0, comp = 0.0;
-  for (int64_t ed = (int64_t)blockIdx.x * GPB + grp; ed < H; ed += (int64_t)gridDim.x * GPB) {
-    const int32_t a = ha[ed], b = hb[ed];
-    // a pair naming a row outside pi is skipped (no row is read) and flagged
-    if ((uint64_t)(int64_t)a >= (uint64_t)n_rows || (uint64_t)(int64_t)b >= (uint64_t)n_rows) {
-      if (l == 0 && bad) atomicOr(bad, 1u);
-      continue;
+  for (int64_t c0 = e0; c0 < e1; c0 += CH) {
+    int32_t a[J], b[J];
+    bool y[J];
+    float old[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int64_t ed = c0 + grp + GPB * j;
+      const bool on = ed < e1;
+      a[j] = on ? ha[ed] : -1;
+      b[j] = on ? hb[ed] : -1;
+      y[j] = on && hy[ed] != 0;
+      old[j] = on ? ppx[ed] : 0.f;
     }
-    const PiT* ra = pi + (int64_t)a * Kp;
-    const PiT* rb = pi + (int64_t)b * Kp;
-    const bool y = hy[ed] != 0;
-    float s = 0.f, fs = 0.f;
 #pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      const int vi = l + LPN * v;
-      if (vi < nvec) {
-        float xa[EV], xb[EV];
-        TR::unpack(ldg_nc_v4(ra + vi * EV), xa);
-        TR::unpack(ldg_nc_v4(rb + vi * EV), xb);
+    for (int j = 0; j < J; ++j) {
+      const int64_t ed = c0 + grp + GPB * j;
+      if (ed >= e1) break;
+      // a pair naming a row outside pi is skipped (no row is read) and flagged
+      if ((uint64_t)(int64_t)a[j] >= (uint64_t)n_rows || (uint64_t)(int64_t)b[j] >= (uint64_t)n_rows) {
+        if (l == 0) {
+          atomicOr(&res->bad, 1u);
+          s_avg[grp + GPB * j] = 1.f;
+        }
+        continue;
+      }
+      const PiT* ra = pi + (int64_t)a[j] * Kp;
+      const PiT* rb = pi + (int64_t)b[j] * Kp;
+      uint4 va[VPL], vb[VPL];
 #pragma unroll
-        for (int e = 0; e < EV; ++e) {
-          if (vi * EV + e < K) {
-            const float f = xa[e] * xb[e];
-            fs += f;
-            s += f * (y ? bt[v * EV + e] : 1.0f - bt[v * EV + e]);
+      for (int v = 0; v < VPL; ++v) {
+        const int vi = l + LPN * v;
+        va[v] = vi < nvec ? ldg_nc_v4(ra + vi * EV) : make_uint4(0, 0, 0, 0);
+        vb[v] = vi < nvec ? ldg_nc_v4(rb + vi * EV) : make_uint4(0, 0, 0, 0);
+      }
+      float s = 0.f, fs = 0.f;
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        const int vi = l + LPN * v;
+        if (vi < nvec) {
+          float xa[EV], xb[EV];
+          TR::unpack(va[v], xa);
+          TR::unpack(vb[v], xb);
+#pragma unroll
+          for (int e = 0; e < EV; ++e) {
+            if (vi * EV + e < K) {
+              const float f = xa[e] * xb[e];
+              fs += f;
+              s += f * (y[j] ? bt[v * EV + e] : 1.0f - bt[v * EV + e]);
+            }
           }
         }
       }
-    }
 #pragma unroll
-    for (int o = LPN / 2; o > 0; o >>= 1) {
-      s += __shfl_xor_sync(gmask, s, o);
-      fs += __shfl_xor_sync(gmask, fs, o);
+      for (int o = LPN / 2; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(gmask, s, o);
+        fs += __shfl_xor_sync(gmask, fs, o);
+      }
+      if (l == 0) {
+        if (!y[j]) s += (1.0f - fs) * (1.0f - m.epsilon);
+        if (s < 1.0e-30f) s = 1.0e-30f;
+        const float avg = (old[j] * (count - 1.0f) + s) / count;
+        ppx[ed] = avg;
+        s_avg[grp + GPB * j] = avg;
+      }
     }
-    if (l == 0) {
-      if (!y) s += (1.0f - fs) * (1.0f - m.epsilon);
-      if (s < 1.0e-30f) s = 1.0e-30f;
-      const float avg = (ppx[ed] * (count - 1.0f) + s) / count;
-      ppx[ed] = avg;
-      const double term = log((double)avg) - comp;
+    __syncthreads();
+    if (tid < CH && c0 + tid < e1) {
+      const double term = log((double)s_avg[tid]) - comp;
       const double tsum = sum + term;
       comp = (tsum - sum) - term;
       sum = tsum;
     }
+    __syncthreads();
   }
-  // block reduction, compensated pairwise in fixed order
-  __shared__ double s_sum[256], s_comp[256];
-  s_sum[tid] = sum;
-  s_comp[tid] = comp;
-  __syncthreads();
+  double total = block_sum_256(sum - comp, s_sum);
   if (tid == 0) {
-    double t = 0.0, c = 0.0;
-    for (int q = 0; q < 256; q += LPN) {
-      const double term = (s_sum[q] - s_comp[q]) - c;
-      const double ts = t + term;
-      c = (ts - t) - term;
-      t = ts;
-    }
-    part[2 * blockIdx.x] = t;
-    part[2 * blockIdx.x + 1] = c;
+    part[blockIdx.x] = total;
+    __threadfence();
+    s_last = atomicAdd(&res->done, 1u) == gridDim.x - 1;
   }
-}
-
-// The blocks' compensated partials, summed by one block of kPpxFinalThreads:
-// thread j takes partials j, j + kPpxFinalThreads, ... in order (Kahan), then
-// a fixed pairwise tree adds the threads' sums (deterministic).  One thread
-// walking 1,216 partials in FP64 took ~230 us on GB300.
-constexpr int kPpxFinalThreads = 256;
-static __global__ void __launch_bounds__(kPpxFinalThreads) k_ppx_final(const double* part, int nblk, int64_t H,
-                                                                       double* out) {
-  __shared__ double s[kPpxFinalThreads];
-  const int tid = threadIdx.x;
-  double t = 0.0, c = 0.0;
-  for (int q = tid; q < nblk; q += kPpxFinalThreads) {
-    const double term = (part[2 * q] - part[2 * q + 1]) - c;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double t = 0.0, c = 0.0;  // each thread's partials in order (compensated), then a fixed tree
+  for (int q = tid; q < (int)gridDim.x; q += 256) {
+    const double term = __ldcg(part + q) - c;
     const double ts = t + term;
     c = (ts - t) - term;
     t = ts;
   }
-  s[tid] = t - c;
   __syncthreads();
-#pragma unroll
-  for (int w = kPpxFinalThreads / 2; w > 0; w >>= 1) {
-    if (tid < w) s[tid] += s[tid + w];
-    __syncthreads();
+  total = block_sum_256(t - c, s_sum);
+  if (tid == 0) {
+    res->value = -(total / (double)H);
+    res->err = gc ? gc->err : 0;
+    res->done = 0;
   }
-  if (tid == 0) out[0] = H ? -(s[0] / (double)H) : 0.0;
 }
 
 // ---------------------------------------------------------------------------

@@ -12,9 +12,8 @@
 // index-error flag) in a fixed file-scope __device__ array instead of
 // handle-owned memory.
 //
-// The array has room for kMaxBlocks partials and the kernel runs one block
-// per 256 held-out edges, so one call accepts at most kMaxBlocks * 256 =
-// 4,194,304 held-out edges and rejects more with AMMSB_E_CAPACITY (the
+// The array has room for kPpxMaxBlocks partials of up to kEdgesPerBlock
+// held-out edges, so one call accepts at most 4,194,304 held-out edges and rejects more with AMMSB_E_CAPACITY (the
 // message goes to stderr, as do those of the other rejected arguments).
 // The array lives in every GPU that loads the library, until the process
 // exits.  All calls on a device share it and it keeps the last call's
@@ -27,7 +26,6 @@
 #include <cuda_runtime.h>
 
 #include <cstdio>
-#include <cstring>
 #include <mutex>
 #include <string>
 
@@ -38,15 +36,11 @@ using namespace ammsb;
 
 namespace {
 
-constexpr int kMaxBlocks = 16384;
 constexpr int kEdgesPerBlock = 256;
 constexpr int kMaxDevices = 64;
 
-// partial (sum, compensation) per block, then the result (2 doubles), then
-// the index-error flag (one double's room)
-static __device__ __align__(256) double g_ppx_scratch[2 * kMaxBlocks + 3];
-constexpr int kResult = 2 * kMaxBlocks;
-constexpr int kFlag = 2 * kMaxBlocks + 2;
+// a partial sum per block, then the result with the index-error flag
+static __device__ __align__(256) double g_ppx_scratch[kPpxMaxBlocks + sizeof(PpxResult) / sizeof(double)];
 
 std::mutex g_mu;
 double* g_scratch_ptr[kMaxDevices] = {nullptr};
@@ -60,23 +54,20 @@ int next_pow2i(int v) {
 template <typename PiT, int LPN, int VPL>
 cudaError_t launch(const Model& m, const void* pi, const float* beta, const int32_t* ha,
                    const int32_t* hb, const uint8_t* hy, int64_t H, float* ppx, float count,
-                   double* scratch, int nblk, int64_t n_rows, cudaStream_t s) {
-  k_perplexity<PiT, LPN, VPL><<<nblk, 256, 0, s>>>(
-      m, reinterpret_cast<const PiT*>(pi), beta, ha, hb, hy, H, ppx, count, scratch, n_rows,
-      reinterpret_cast<unsigned int*>(scratch + kFlag));
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_ppx_final<<<1, kPpxFinalThreads, 0, s>>>(scratch, nblk, H, scratch + kResult);
+                   double* scratch, const PpxPlan& plan, int64_t n_rows, cudaStream_t s) {
+  k_perplexity<PiT, LPN, VPL><<<plan.blocks, 256, 0, s>>>(
+      m, reinterpret_cast<const PiT*>(pi), beta, ha, hb, hy, H, plan.per_block, ppx, count, scratch, n_rows, nullptr,
+      reinterpret_cast<PpxResult*>(scratch + kPpxMaxBlocks));
   return cudaGetLastError();
 }
 
 template <typename PiT>
 cudaError_t dispatch(int lpn, int vpl, const Model& m, const void* pi, const float* beta,
                      const int32_t* ha, const int32_t* hb, const uint8_t* hy, int64_t H, float* ppx,
-                     float count, double* scratch, int nblk, int64_t n_rows, cudaStream_t s) {
+                     float count, double* scratch, const PpxPlan& plan, int64_t n_rows, cudaStream_t s) {
 #define CASE(L, V) \
   if (lpn == L && vpl == V)  \
-    return launch<PiT, L, V>(m, pi, beta, ha, hb, hy, H, ppx, count, scratch, nblk, n_rows, s);
+    return launch<PiT, L, V>(m, pi, beta, ha, hb, hy, H, ppx, count, scratch, plan, n_rows, s);
   CASE(1, 1) CASE(2, 1) CASE(4, 1) CASE(8, 1) CASE(16, 1) CASE(32, 1) CASE(32, 2) CASE(32, 4) CASE(32, 8)
 #undef CASE
   return cudaErrorInvalidConfiguration;
@@ -107,7 +98,7 @@ int ammsb_perplexity_noalloc(const void* pi, int32_t pi_dtype, int64_t K, int64_
     return fail("pi must be 16-byte aligned", AMMSB_E_ARG);
   if (n_rows < 1 || n_rows > (int64_t)INT32_MAX + 1)
     return fail("n_rows must be in [1, 2^31]", AMMSB_E_ARG);
-  if (held_count < 0 || held_count > (int64_t)kMaxBlocks * kEdgesPerBlock)
+  if (held_count < 0 || held_count > (int64_t)kPpxMaxBlocks * kEdgesPerBlock)
     return fail("held_count exceeds the static scratch: at most 4,194,304 held-out edges",
                 AMMSB_E_CAPACITY);
   if (average_count < 1) return fail("average_count starts at 1", AMMSB_E_ARG);
@@ -145,26 +136,27 @@ int ammsb_perplexity_noalloc(const void* pi, int32_t pi_dtype, int64_t K, int64_
     vpl = next_pow2i((nvec + 31) / 32);
   }
   if (vpl > 8) return fail("row too wide", AMMSB_E_ARG);  // K <= 1024 keeps vpl <= 8
-  const int nblk = (int)((held_count + kEdgesPerBlock - 1) / kEdgesPerBlock);
+  const PpxPlan plan = ppx_plan(lpn, held_count);
   const float count = (float)average_count;
-  cudaError_t e = cudaMemsetAsync(scratch + kFlag, 0, sizeof(double), s);
+  // the flag, and the count of finished blocks (a call that raced with
+  // another may have left it anywhere)
+  PpxResult* result = reinterpret_cast<PpxResult*>(scratch + kPpxMaxBlocks);
+  cudaError_t e = cudaMemsetAsync(result, 0, sizeof(*result), s);
   if (e != cudaSuccess) return fail(std::string("flag clear: ") + cudaGetErrorString(e), AMMSB_E_CUDA);
   e = (pi_dtype == AMMSB_PI_BF16)
           ? dispatch<__nv_bfloat16>(lpn, vpl, m, pi, beta, held_a, held_b, held_y, held_count, ppx,
-                                    count, scratch, nblk, n_rows, s)
+                                    count, scratch, plan, n_rows, s)
           : dispatch<float>(lpn, vpl, m, pi, beta, held_a, held_b, held_y, held_count, ppx, count,
-                            scratch, nblk, n_rows, s);
+                            scratch, plan, n_rows, s);
   if (e != cudaSuccess) return fail(std::string("launch: ") + cudaGetErrorString(e), AMMSB_E_CUDA);
-  double res[3];  // result (2 doubles: value, compensation) and the flag
-  e = cudaMemcpyAsync(res, scratch + kResult, sizeof(res), cudaMemcpyDeviceToHost, s);
+  PpxResult res;
+  e = cudaMemcpyAsync(&res, result, sizeof(res), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(std::string("result copy: ") + cudaGetErrorString(e), AMMSB_E_CUDA);
-  unsigned int flag = 0;
-  std::memcpy(&flag, &res[2], sizeof(flag));
-  if (flag != 0)
+  if (res.bad != 0)
     return fail("a held-out pair names a row outside [0, n_rows): those pairs were skipped",
                 AMMSB_E_ARG);
-  *out = res[0];
+  *out = res.value;
   return AMMSB_OK;
 }
 
