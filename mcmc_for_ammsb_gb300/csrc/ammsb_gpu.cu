@@ -880,6 +880,7 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
   TRY(dev_alloc(h, &h->gc, 1));
   b.gc = h->gc;
   TRY(dev_alloc(h, &h->d_err_init, 1));
+  TRY(dev_alloc(h, &h->d_gamma, 1));
   TRY(dev_alloc(h, &h->d_fed_phi_noise, (size_t)m.max_nodes * K));
   TRY(dev_alloc(h, &h->d_fed_theta_noise, 2 * (size_t)K));
   b.fed_phi_noise = nullptr;
@@ -951,8 +952,9 @@ int ammsb_init_state(ammsb_handle* h) {
   CK(cudaMemcpyAsync(h->b.beta, beta.data(), sizeof(float) * h->m.Kp, cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemsetAsync(h->d_err_init, 0, sizeof(int32_t), h->stream));
   const int64_t total = h->m.N * (int64_t)h->m.Kp;
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 152 * 64));
-  k_init_phi<<<blocks, 256, 0, h->stream>>>(h->m, h->b.phi, 1.0, 1.0, h->d_err_init);  // cc:66
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 152 * 8));
+  k_gamma_tables<<<1, 256, 0, h->stream>>>(h->d_gamma);
+  k_init_phi<<<blocks, 256, 0, h->stream>>>(h->m, h->b.phi, h->d_gamma, h->d_err_init);  // cc:66
   CK(cudaGetLastError());
   CK(launch_normalize(h));
   int rc = reset_counters(h);

@@ -82,6 +82,7 @@ struct ammsb_handle {
   float* d_fed_phi_noise = nullptr;
   float* d_fed_theta_noise = nullptr;
   int32_t* d_err_init = nullptr;
+  GammaTables* d_gamma = nullptr;
   int ncommit = 1;
   bool star = false;  // drawn minibatches are stars
   int nbr_blocks = 1, phi_blocks = 1;

@@ -15,6 +15,7 @@
 //                        (cc:244-266), FP64
 #pragma once
 #include "ammsb_device.cuh"
+#include "ammsb_gamma.cuh"
 
 namespace ammsb {
 
@@ -1594,15 +1595,30 @@ __global__ void __launch_bounds__(256) k_perplexity(Model m, const PiT* __restri
 // ---------------------------------------------------------------------------
 // init: phi ~ Gamma(1,1) (cc:66), row normalisation into pi (cc:75)
 // ---------------------------------------------------------------------------
-static __global__ void k_init_phi(Model m, float* phi, double shape, double scale, int32_t* err) {
+static __global__ void __launch_bounds__(256) k_init_phi(Model m, float* phi, const GammaTables* tables,
+                                                         int32_t* err) {
+  __shared__ GammaTables s_t;
+  static_assert(sizeof(GammaTables) % sizeof(float2) == 0, "copied by pairs");
+  for (int i = threadIdx.x; i < (int)(sizeof(GammaTables) / sizeof(float2)); i += 256)
+    reinterpret_cast<float2*>(&s_t)[i] = reinterpret_cast<const float2*>(tables)[i];
+  __syncthreads();
   const Stream rs{m.seed, m.chain};
-  const int64_t total = m.N * (int64_t)m.Kp;
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < total;
-       x += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t v = x / m.Kp;
-    const int k = (int)(x - v * m.Kp);
-    phi[x] = (k < m.K) ? (float)gamma_draw(rs, kTagPhiInit, (uint32_t)v, (uint64_t)k, shape, scale, err)
-                       : 0.f;
+  // element x = v Kp + k, the grid's threads side by side: v and k follow
+  // without a division each
+  const int64_t total = m.N * (int64_t)m.Kp, stride = (int64_t)gridDim.x * 256;
+  const int64_t dv = stride / m.Kp;
+  const int dk = (int)(stride - dv * m.Kp);
+  int64_t x = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  int64_t v = x / m.Kp;
+  int k = (int)(x - v * m.Kp);
+  for (; x < total; x += stride) {
+    phi[x] = k < m.K ? gamma_one_draw(rs, kTagPhiInit, (uint32_t)v, (uint64_t)k, s_t, err) : 0.f;
+    v += dv;
+    k += dk;
+    if (k >= m.Kp) {
+      k -= m.Kp;
+      ++v;
+    }
   }
 }
 
