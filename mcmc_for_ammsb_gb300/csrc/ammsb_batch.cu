@@ -4,8 +4,8 @@
 // Each chain is an ammsb_handle of its own (its graph, held-out set, state,
 // options and update_phi configuration).  The batch launches every kernel
 // of the iteration once for all chains that share the kernel's compiled
-// shape: blockIdx.y selects the chain, whose model, graph and buffer sets
-// come from a device array of ChainArgs.  Chains of different row widths,
+// shape: a map from a block to its chain selects the chain, whose model, graph
+// and buffer sets come from a device array of ChainArgs.  Chains of different row widths,
 // minibatch sizes and graphs therefore run in a handful of launches per
 // iteration instead of five per chain, and a block of iterations of all
 // chains -- their updates and, on a second stream, one launch of all their
@@ -26,14 +26,23 @@
 
 namespace {
 
+// The blocks of one launch over many chains: each chain's own, in chain order.
+struct BlockMap {
+  std::vector<BlockOf> blocks;
+  BlockOf* d = nullptr;
+  void add(int chain, int n) {
+    for (int i = 0; i < n; ++i) blocks.push_back(BlockOf{chain, i, n, 0});
+  }
+  int grid() const { return (int)blocks.size(); }
+};
+
 // One launch of the update phase: the chains sharing a kernel shape.
 struct PhiGroup {
   int dtype;
   KernelCfg cfg;
   bool full;  // ring kernel: every lane's vectors inside the row
   std::vector<int> chains;
-  ChainArgs* d = nullptr;  // the group's chains, in order
-  int gx = 1;
+  BlockMap map, map_few;  // map_few: the ring kernel's launch for iterations of few nodes, where it has its own
   size_t smem = 0;      // ring kernel: per four-warp group
   size_t smem_few = 0;  // ring kernel: a 16-warp node
 };
@@ -41,64 +50,57 @@ struct PhiGroup {
 struct CommitGroup {
   int dtype, kq;
   int chunk;  // k_commit_star's edges per summing warp at once; 0: k_commit_beta
-  std::vector<int> chains;
-  ChainArgs* d = nullptr;
-  int gx = 1;
+  BlockMap map;
   size_t smem = 0;
 };
 
+// `all`: every chain's arguments; `pdl`: as for one chain.
 template <typename PiT, int L, int V, int S>
-cudaError_t phi_reg_chains(const PhiGroup& g, int p, cudaStream_t st) {
+cudaError_t phi_reg_chains(const PhiGroup& g, const ChainArgs* all, int p, cudaStream_t st, bool pdl) {
   constexpr int NPB = 128 / (L * S) > 0 ? 128 / (L * S) : 1;
-  k_update_phi_chains<PiT, L, V, S, NPB><<<dim3(g.gx, (unsigned)g.chains.size()), NPB * S * L, g.smem, st>>>(
-      g.d, p);
-  return cudaGetLastError();
+  return launch_k(k_update_phi_chains<PiT, L, V, S, NPB>, g.map.grid(), NPB * S * L, g.smem, st, pdl, all, g.map.d, p);
 }
 
 template <typename PiT, int V, int STAGES, bool FULL>
-cudaError_t phi_ring_chains(const PhiGroup& g, int p, cudaStream_t st, bool configure) {
-  // launched as for one chain; a CTA's groups for every node slot
+cudaError_t phi_ring_chains(const PhiGroup& g, const ChainArgs* all, int p, cudaStream_t st, bool pdl,
+                            bool configure) {
   auto kern = k_update_phi_ring_chains<PiT, V, STAGES, FULL>;
   const RingPlan r = ring_plan(g.cfg, g.smem, g.smem_few);
   if (configure) return ammsb_detail::raise_smem_limit(kern, r.smem());
-  const unsigned n = (unsigned)g.chains.size();
-  const dim3 grid(std::max((g.gx + r.groups - 1) / r.groups, r.few), n);
-  if (r.single) {
-    kern<<<grid, 512, r.smem(), st>>>(g.d, p, r.few, kPhiFew | kPhiMany);
-    return cudaGetLastError();
-  }
+  if (r.single)
+    return launch_k(kern, g.map.grid(), 512, r.smem(), st, pdl, all, g.map.d, p, r.few, kPhiFew | kPhiMany);
   if (r.few > 0) {
-    kern<<<dim3(r.few, n), 512, r.few_bytes, st>>>(g.d, p, r.few, kPhiFew);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_k(kern, g.map_few.grid(), 512, r.few_bytes, st, pdl, all, g.map_few.d, p, r.few, kPhiFew);
     if (e != cudaSuccess) return e;
   }
-  kern<<<grid, r.groups * kPhiGroup, r.groups * r.group_bytes, st>>>(g.d, p, r.few, kPhiMany);
-  return cudaGetLastError();
+  return launch_k(kern, g.map.grid(), r.groups * kPhiGroup, r.groups * r.group_bytes, st, pdl, all, g.map.d, p, r.few,
+                  kPhiMany);
 }
 
 template <typename PiT, int V>
-cudaError_t phi_ring_chains_v(const PhiGroup& g, int p, cudaStream_t st, bool configure) {
+cudaError_t phi_ring_chains_v(const PhiGroup& g, const ChainArgs* all, int p, cudaStream_t st, bool pdl,
+                              bool configure) {
 #define RING_CASE(S)                                                                           \
   if (g.cfg.ring_stages == S)                                                                  \
-    return g.full ? phi_ring_chains<PiT, V, S, true>(g, p, st, configure)                      \
-                  : phi_ring_chains<PiT, V, S, false>(g, p, st, configure);
+    return g.full ? phi_ring_chains<PiT, V, S, true>(g, all, p, st, pdl, configure)                      \
+                  : phi_ring_chains<PiT, V, S, false>(g, all, p, st, pdl, configure);
   AMMSB_PHI_RING_STAGES(RING_CASE)
 #undef RING_CASE
   return cudaErrorInvalidConfiguration;
 }
 
 template <typename PiT>
-cudaError_t phi_chains(const PhiGroup& g, int p, cudaStream_t st, bool configure) {
+cudaError_t phi_chains(const PhiGroup& g, const ChainArgs* all, int p, cudaStream_t st, bool pdl, bool configure) {
   const KernelCfg& c = g.cfg;
   if (c.ring) {
     switch (c.vpl) {
-      case 1: return phi_ring_chains_v<PiT, 1>(g, p, st, configure);
-      case 2: return phi_ring_chains_v<PiT, 2>(g, p, st, configure);
-      case 4: return phi_ring_chains_v<PiT, 4>(g, p, st, configure);
+      case 1: return phi_ring_chains_v<PiT, 1>(g, all, p, st, pdl, configure);
+      case 2: return phi_ring_chains_v<PiT, 2>(g, all, p, st, pdl, configure);
+      case 4: return phi_ring_chains_v<PiT, 4>(g, all, p, st, pdl, configure);
       default: break;
     }
     if constexpr (sizeof(PiT) == 4)
-      if (c.vpl == 8) return phi_ring_chains_v<PiT, 8>(g, p, st, configure);
+      if (c.vpl == 8) return phi_ring_chains_v<PiT, 8>(g, all, p, st, pdl, configure);
     return cudaErrorInvalidConfiguration;
   }
   if (configure) {
@@ -112,19 +114,18 @@ cudaError_t phi_chains(const PhiGroup& g, int p, cudaStream_t st, bool configure
     return cudaErrorInvalidConfiguration;
   }
 #define REG_CASE(L, V, S) \
-  if (c.lpn == L && c.vpl == V && c.split == S) return phi_reg_chains<PiT, L, V, S>(g, p, st);
+  if (c.lpn == L && c.vpl == V && c.split == S) return phi_reg_chains<PiT, L, V, S>(g, all, p, st, pdl);
   AMMSB_PHI_REG_SHAPES(REG_CASE)
 #undef REG_CASE
   return cudaErrorInvalidConfiguration;
 }
 
 template <typename PiT, int KQ>
-cudaError_t commit_chains_k(const CommitGroup& g, int p, cudaStream_t st, bool configure) {
-  const dim3 grid(g.gx, (unsigned)g.chains.size());
+cudaError_t commit_chains_k(const CommitGroup& g, const ChainArgs* all, int p, cudaStream_t st, bool pdl,
+                            bool configure) {
   auto go = [&](auto* kern, int threads) -> cudaError_t {
     if (configure) return ammsb_detail::raise_smem_limit(kern, g.smem);
-    kern<<<grid, threads, g.smem, st>>>(g.d, p);
-    return cudaGetLastError();
+    return launch_k(kern, g.map.grid(), threads, g.smem, st, pdl, all, g.map.d, p);
   };
   switch (g.chunk) {
     case 0: return go(k_commit_beta_chains<PiT, KQ>, 128);
@@ -133,12 +134,13 @@ cudaError_t commit_chains_k(const CommitGroup& g, int p, cudaStream_t st, bool c
   }
 }
 template <typename PiT>
-cudaError_t commit_chains(const CommitGroup& g, int p, cudaStream_t st, bool configure) {
+cudaError_t commit_chains(const CommitGroup& g, const ChainArgs* all, int p, cudaStream_t st, bool pdl,
+                          bool configure) {
   switch (g.kq) {
-    case 1: return commit_chains_k<PiT, 1>(g, p, st, configure);
-    case 2: return commit_chains_k<PiT, 2>(g, p, st, configure);
-    case 4: return commit_chains_k<PiT, 4>(g, p, st, configure);
-    case 8: return commit_chains_k<PiT, 8>(g, p, st, configure);
+    case 1: return commit_chains_k<PiT, 1>(g, all, p, st, pdl, configure);
+    case 2: return commit_chains_k<PiT, 2>(g, all, p, st, pdl, configure);
+    case 4: return commit_chains_k<PiT, 4>(g, all, p, st, pdl, configure);
+    case 8: return commit_chains_k<PiT, 8>(g, all, p, st, pdl, configure);
     default: return cudaErrorInvalidConfiguration;
   }
 }
@@ -158,8 +160,8 @@ struct ammsb_batch {
   std::vector<void*> allocs;
   std::vector<PhiGroup> phi;
   std::vector<CommitGroup> commit;
-  int theta_gx = 1;
-  int nbr_gx = 1;
+  BlockMap theta, nbr;
+  int pdl = 0;  // early starts (kPdl* bits), as for one chain
   size_t mb_smem = 0, nbr_smem = 0;
   // captured iterations, as for one chain (ammsb_handle): a block with the
   // other block's draws alongside, both in turn, runs of updates in a block
@@ -186,30 +188,39 @@ thread_local std::string g_batch_create_error;
     }                                                                  \
   } while (0)
 
-cudaError_t launch_update_chains(ammsb_batch* bt, int p) {
+// `pdl`: the theta step of the iteration before is the kernel ahead in the
+// stream and this iteration's draws are complete.
+cudaError_t launch_update_chains(ammsb_batch* bt, int p, bool pdl) {
   // the update_phi groups touch disjoint chains: they run concurrently
-  // (parallel branches of the captured graph), then join before the commits
+  // (parallel branches of the captured graph), then join before the commits.
+  // The first group, the commit and the theta step start early as for one
+  // chain; the other groups start when the theta step ahead has completed, and
+  // the commit when they have (every chain's update_phi and so its commit
+  // follow that step, as the rules for early starts ask).
   const size_t ng = bt->phi.size();
   cudaError_t e = cudaSuccess;
   if (ng > 1 && (e = cudaEventRecord(bt->ev_groups, bt->stream)) != cudaSuccess) return e;
   for (size_t gi = 0; gi < ng; ++gi) {
     const PhiGroup& g = bt->phi[gi];
     cudaStream_t st = gi == 0 ? bt->stream : bt->gstream[gi - 1];
+    const bool early = gi == 0 && pdl && (bt->pdl & kPdlPhi);
     if (gi > 0 && (e = cudaStreamWaitEvent(st, bt->ev_groups, 0)) != cudaSuccess) return e;
-    e = (g.dtype == AMMSB_PI_BF16) ? phi_chains<__nv_bfloat16>(g, p, st, false)
-                                   : phi_chains<float>(g, p, st, false);
+    e = (g.dtype == AMMSB_PI_BF16) ? phi_chains<__nv_bfloat16>(g, bt->d_all, p, st, early, false)
+                                   : phi_chains<float>(g, bt->d_all, p, st, early, false);
     if (e != cudaSuccess) return e;
     if (gi > 0 && (e = cudaEventRecord(bt->gevent[gi - 1], st)) != cudaSuccess) return e;
   }
   for (size_t gi = 1; gi < ng; ++gi)
     if ((e = cudaStreamWaitEvent(bt->stream, bt->gevent[gi - 1], 0)) != cudaSuccess) return e;
-  for (const CommitGroup& g : bt->commit) {
-    cudaError_t e = (g.dtype == AMMSB_PI_BF16) ? commit_chains<__nv_bfloat16>(g, p, bt->stream, false)
-                                               : commit_chains<float>(g, p, bt->stream, false);
+  for (size_t ci = 0; ci < bt->commit.size(); ++ci) {
+    const CommitGroup& g = bt->commit[ci];
+    const bool early = ci == 0 && (bt->pdl & kPdlCommit);
+    e = (g.dtype == AMMSB_PI_BF16) ? commit_chains<__nv_bfloat16>(g, bt->d_all, p, bt->stream, early, false)
+                                   : commit_chains<float>(g, bt->d_all, p, bt->stream, early, false);
     if (e != cudaSuccess) return e;
   }
-  k_theta_chains<<<dim3(bt->theta_gx, (unsigned)bt->h.size()), kThetaThreads, 0, bt->stream>>>(bt->d_all, p);
-  return cudaGetLastError();
+  return launch_k(k_theta_chains, bt->theta.grid(), kThetaThreads, 0, bt->stream, (bt->pdl & kPdlTheta) != 0,
+                  bt->d_all, bt->theta.d, p);
 }
 
 // Draws of one block of every chain, into the buffer sets from s0 on.
@@ -218,13 +229,13 @@ cudaError_t launch_sampling_chains(ammsb_batch* bt, int s0, cudaStream_t st) {
   k_sample_minibatch_chains<<<dim3(D, n), 1024, bt->mb_smem, st>>>(bt->d_all, s0);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_sample_neighbors_chains<8><<<dim3(bt->nbr_gx, n, D), 256, bt->nbr_smem, st>>>(bt->d_all, s0);
+  k_sample_neighbors_chains<8><<<dim3(bt->nbr.grid(), D), 256, bt->nbr_smem, st>>>(bt->d_all, bt->nbr.d, s0);
   return cudaGetLastError();
 }
 
-cudaError_t launch_updates_chains(ammsb_batch* bt, int s, int count) {
+cudaError_t launch_updates_chains(ammsb_batch* bt, int s, int count, bool first_pdl = false) {
   cudaError_t e = cudaSuccess;
-  for (int i = 0; i < count && e == cudaSuccess; ++i) e = launch_update_chains(bt, s + i);
+  for (int i = 0; i < count && e == cudaSuccess; ++i) e = launch_update_chains(bt, s + i, i > 0 || first_pdl);
   return e;
 }
 
@@ -238,10 +249,11 @@ cudaError_t fork_draws_chains(ammsb_batch* bt, int blk) {
   return cudaEventRecord(bt->ev_join, bt->side);
 }
 
-cudaError_t launch_block_chains(ammsb_batch* bt, int blk) {
+cudaError_t launch_block_chains(ammsb_batch* bt, int blk, bool first_pdl = false) {
   cudaError_t e = fork_draws_chains(bt, 1 - blk);
   if (e != cudaSuccess) return e;
-  if ((e = launch_updates_chains(bt, blk * bt->block, bt->block)) != cudaSuccess) return e;
+  if ((e = launch_updates_chains(bt, blk * bt->block, bt->block, first_pdl)) != cudaSuccess)
+    return e;
   return cudaStreamWaitEvent(bt->stream, bt->ev_join, 0);
 }
 
@@ -334,6 +346,7 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     bt->h.push_back(h);
   }
   bt->device = handles[0]->device;
+  bt->pdl = handles[0]->cfg.pdl;
   if (const char* env = std::getenv("AMMSB_BATCH_GRAPH_ITERS"))  // iterations of both blocks
     bt->block = std::max(1, std::min(kMaxBlock, std::atoi(env) / 2));
   int prio_lo = 0, prio_hi = 0;  // the draws ahead at the higher priority, as for one chain
@@ -360,8 +373,8 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     a.smem_hash = h->mb_smem > 0 ? 1 : 0;
     bt->mb_smem = std::max(bt->mb_smem, h->mb_smem);
     bt->nbr_smem = std::max(bt->nbr_smem, h->nbr_smem);
-    bt->nbr_gx = std::max(bt->nbr_gx, h->nbr_blocks);
-    bt->theta_gx = std::max(bt->theta_gx, (h->m.K + 31) / 32);
+    bt->nbr.add(i, h->nbr_blocks);
+    bt->theta.add(i, (h->m.K + 31) / 32);
   }
   if (dev_upload(bt, &bt->d_all, args) != cudaSuccess) {
     bt->err = "upload of the chain table failed";
@@ -389,12 +402,11 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     PhiGroup& g = bt->phi[it->second];
     g.chains.push_back(i);
     if (c.ring) {
-      g.gx = std::max(g.gx, h->m.max_nodes);
       g.smem = std::max(g.smem, h->phi_smem);
       g.smem_few = std::max(g.smem_few, h->phi_smem_few);
     } else {
       const int npb = std::max(1, 128 / (c.lpn * c.split));
-      g.gx = std::max(g.gx, std::max(1, std::min((h->m.max_nodes + npb - 1) / npb, 152 * 32)));
+      g.map.add(i, std::max(1, std::min((h->m.max_nodes + npb - 1) / npb, 152 * 32)));
       const size_t smem = ((size_t)npb * c.split * h->m.Kp + npb * c.split +
                            npb * std::max(1, c.split * c.lpn / 32)) * sizeof(float);
       g.smem = std::max(g.smem, smem);
@@ -411,20 +423,27 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
       bt->commit.push_back(g2);
     }
     CommitGroup& g2 = bt->commit[jt->second];
-    g2.chains.push_back(i);
-    g2.gx = std::max(g2.gx, (chunk ? 0 : h->ncommit) + h->m.nbb + (h->m.K + 31) / 32);
+    g2.map.add(i, (chunk ? 0 : h->ncommit) + h->m.nbb + (h->m.K + 31) / 32);
     if (chunk)
       g2.smem = std::max(g2.smem, chunk == 1 ? commit_star_smem<1>(h->m.Kp) : commit_star_smem<kStarChunk>(h->m.Kp));
   }
+  auto upload = [&](BlockMap& map) { return dev_upload(bt, &map.d, map.blocks) == cudaSuccess; };
   for (PhiGroup& g : bt->phi) {
-    std::vector<ChainArgs> a;
-    for (int i : g.chains) a.push_back(args[i]);
-    if (dev_upload(bt, &g.d, a) != cudaSuccess) {
+    if (g.cfg.ring) {  // a node per four-warp group, and a CTA per node of an iteration of few
+      const RingPlan r = ring_plan(g.cfg, g.smem, g.smem_few);
+      for (int i : g.chains) {
+        const int nodes = bt->h[i]->m.max_nodes, many = (nodes + r.groups - 1) / r.groups,
+                  few = std::min(r.few, nodes);
+        g.map.add(i, r.single ? std::max(many, few) : many);
+        if (!r.single && r.few > 0) g.map_few.add(i, few);
+      }
+    }
+    if (!upload(g.map) || !upload(g.map_few)) {
       bt->err = "upload of a group table failed";
       return bail(AMMSB_E_CUDA);
     }
-    cudaError_t e = (g.dtype == AMMSB_PI_BF16) ? phi_chains<__nv_bfloat16>(g, 0, bt->stream, true)
-                                               : phi_chains<float>(g, 0, bt->stream, true);
+    cudaError_t e = (g.dtype == AMMSB_PI_BF16) ? phi_chains<__nv_bfloat16>(g, bt->d_all, 0, bt->stream, false, true)
+                                               : phi_chains<float>(g, bt->d_all, 0, bt->stream, false, true);
     if (e != cudaSuccess) {
       bt->err = std::string("update_phi group configuration: ") + cudaGetErrorString(e);
       return bail(AMMSB_E_CUDA);
@@ -449,18 +468,21 @@ int ammsb_batch_create(ammsb_handle* const* handles, int32_t n, ammsb_batch** ou
     bt->gevent.push_back(ev);
   }
   for (CommitGroup& g : bt->commit) {
-    std::vector<ChainArgs> a;
-    for (int i : g.chains) a.push_back(args[i]);
-    if (dev_upload(bt, &g.d, a) != cudaSuccess) {
+    if (!upload(g.map)) {
       bt->err = "upload of a group table failed";
       return bail(AMMSB_E_CUDA);
     }
-    cudaError_t e = (g.dtype == AMMSB_PI_BF16) ? commit_chains<__nv_bfloat16>(g, 0, bt->stream, true)
-                                               : commit_chains<float>(g, 0, bt->stream, true);
+    cudaError_t e = (g.dtype == AMMSB_PI_BF16)
+                        ? commit_chains<__nv_bfloat16>(g, bt->d_all, 0, bt->stream, false, true)
+                        : commit_chains<float>(g, bt->d_all, 0, bt->stream, false, true);
     if (e != cudaSuccess) {
       bt->err = std::string("commit group configuration: ") + cudaGetErrorString(e);
       return bail(AMMSB_E_CUDA);
     }
+  }
+  if (!upload(bt->theta) || !upload(bt->nbr)) {
+    bt->err = "upload of a group table failed";
+    return bail(AMMSB_E_CUDA);
   }
   if ((bt->mb_smem > 48 * 1024 &&
        ammsb_detail::raise_smem_limit(k_sample_minibatch_chains, bt->mb_smem) != cudaSuccess) ||
@@ -521,7 +543,7 @@ int ammsb_batch_step(ammsb_batch* bt, int64_t n_iters) {
       n = both ? 2 * D : D;
       rc = launch_graph(bt, both ? bt->graphL[blk] : bt->graphB[blk], [&] {
         cudaError_t e = launch_block_chains(bt, blk);
-        return e == cudaSuccess && both ? launch_block_chains(bt, 1 - blk) : e;
+        return e == cudaSuccess && both ? launch_block_chains(bt, 1 - blk, true) : e;
       });
       drawn += (uint32_t)n;
     } else {

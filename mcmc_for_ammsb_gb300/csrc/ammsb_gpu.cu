@@ -74,32 +74,12 @@ int dev_alloc(ammsb_handle* h, T** p, size_t count) {
 
 // ---- kernel dispatch -------------------------------------------------------
 template <typename PiT, int LPN, int VPL, int SPLIT>
-cudaError_t launch_phi_t(ammsb_handle* h, const Buffers& b) {
+cudaError_t launch_phi_t(ammsb_handle* h, const Buffers& b, bool pdl) {
   constexpr int NPB = 128 / (LPN * SPLIT) > 0 ? 128 / (LPN * SPLIT) : 1;
   int blocks = (h->m.max_nodes + NPB - 1) / NPB;
   blocks = std::max(1, std::min(blocks, 152 * 32));
   size_t smem = ((size_t)NPB * SPLIT * h->m.Kp + NPB * SPLIT + NPB * std::max(1, SPLIT * LPN / 32)) * sizeof(float);
-  k_update_phi<PiT, LPN, VPL, SPLIT, NPB><<<blocks, NPB * SPLIT * LPN, smem, h->stream>>>(h->m, b);
-  return cudaGetLastError();
-}
-
-// Launches `k` on stream `s`; with `pdl` as a programmatic dependent launch
-// (it may start once every CTA of the kernel ahead of it in the stream has
-// triggered, and waits on the device before reading that kernel's results).
-template <typename... P, typename... A>
-cudaError_t launch_k(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, bool pdl,
-                     A&&... args) {
-  cudaLaunchConfig_t lc{};
-  lc.gridDim = dim3(grid);
-  lc.blockDim = dim3(block);
-  lc.dynamicSmemBytes = smem;
-  lc.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = at;
-  lc.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&lc, k, std::forward<A>(args)...);
+  return launch_k(k_update_phi<PiT, LPN, VPL, SPLIT, NPB>, blocks, NPB * SPLIT * LPN, smem, h->stream, pdl, h->m, b);
 }
 
 // `pdl`: the launch directly follows k_theta in the stream and its draws
@@ -162,9 +142,10 @@ cudaError_t launch_phi_ring(ammsb_handle* h, const Buffers& b, bool configure, b
 template <typename PiT>
 cudaError_t launch_phi(ammsb_handle* h, const Buffers& b, bool pdl = false) {
   const KernelCfg& c = h->cfg;
-  if (c.ring) return launch_phi_ring<PiT>(h, b, false, pdl && (c.pdl & kPdlPhi));
+  pdl = pdl && (c.pdl & kPdlPhi);
+  if (c.ring) return launch_phi_ring<PiT>(h, b, false, pdl);
 #define PHI_CASE(L, V, S) \
-  if (c.lpn == L && c.vpl == V && c.split == S) return launch_phi_t<PiT, L, V, S>(h, b);
+  if (c.lpn == L && c.vpl == V && c.split == S) return launch_phi_t<PiT, L, V, S>(h, b, pdl);
   AMMSB_PHI_REG_SHAPES(PHI_CASE)
 #undef PHI_CASE
   return cudaErrorInvalidConfiguration;
@@ -876,7 +857,7 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
     TRY(dev_alloc(h, &b.htab_idx, (size_t)h->block * hcap));
   }
   TRY(dev_alloc(h, &b.beta_part, (size_t)m.nbb * 2 * Kp));
-  TRY(dev_alloc(h, &b.theta_pre, 5 * (size_t)K));
+  TRY(dev_alloc(h, &b.theta_pre, kThetaPre * (size_t)K));
   TRY(dev_alloc(h, &h->gc, 1));
   b.gc = h->gc;
   TRY(dev_alloc(h, &h->d_err_init, 1));

@@ -8,6 +8,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/ammsb_gpu.h"
@@ -169,6 +170,25 @@ inline RingPlan ring_plan(const KernelCfg& c, size_t group_bytes, size_t few_byt
 
 // Ring depths the ring update_phi kernel is built for.
 #define AMMSB_PHI_RING_STAGES(X) X(3) X(4) X(6)
+
+// Launches `k` on stream `s`; with `pdl` as a programmatic dependent launch
+// (it may start once every CTA of the kernel ahead of it in the stream has
+// triggered, and waits on the device before reading that kernel's results).
+template <typename... P, typename... A>
+inline cudaError_t launch_k(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, bool pdl,
+                     A&&... args) {
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(grid);
+  lc.blockDim = dim3(block);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&lc, k, std::forward<A>(args)...);
+}
 
 namespace ammsb_detail {
 // Raises a kernel's dynamic shared memory limit to at least `bytes` and

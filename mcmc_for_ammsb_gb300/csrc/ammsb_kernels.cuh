@@ -29,6 +29,7 @@ constexpr int kMaxBetaBlocks = AMMSB_MAX_BETA_BLOCKS;
 constexpr int kThetaChains = 31, kThetaPerChain = 9;
 static_assert(kMaxBetaBlocks <= kThetaChains * kThetaPerChain, "k_theta reads the partials in one pass");
 constexpr int kThetaThreads = 256;
+constexpr int kThetaPre = 10;  // doubles per k of theta_pre_block
 
 struct Model {
   int32_t K;      // communities
@@ -72,7 +73,7 @@ struct Buffers {
   uint32_t* htab_idx;
   uint32_t hmask;
   float* beta_part;    // nbb x 2 x Kp
-  double* theta_pre;   // 5 x K: the theta step's parts that do not need the sums
+  double* theta_pre;   // kThetaPre x K: the theta step's parts that do not need the sums
   const float* fed_phi_noise;    // max_nodes x K or null
   const float* fed_theta_noise;  // K x 2 or null
   DevState* st;        // this buffer set's per-iteration scalars
@@ -98,9 +99,15 @@ __host__ __device__ __forceinline__ Buffers slot_buffers(const Model& m, const B
   return b;
 }
 
-// One chain of a multi-chain launch (blockIdx.y selects the chain): its
-// model, graph and buffer set 0 of its ring, plus the per-chain launch
-// parameters of the single-chain kernels.
+// One chain of a multi-chain launch: its model, graph and buffer set 0 of its
+// ring, plus the per-chain launch parameters of the single-chain kernels.  The
+// launch has the blocks that each chain's own launch would have, one after the
+// other, and a map from a block to its chain: with the largest chain's blocks
+// for every chain (a grid of chains x blocks) most blocks of a batch of unequal
+// chains started only to exit.
+struct BlockOf {
+  int32_t chain, block, blocks, pad;  // block `block` of the chain's `blocks`
+};
 struct ChainArgs {
   Model m;
   DevGraph g;
@@ -649,7 +656,7 @@ static __global__ void __launch_bounds__(1024) k_sample_minibatch_chains(const C
 // ---------------------------------------------------------------------------
 template <int WARPS>
 __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevGraph& g, const Buffers& b,
-                                                      int j0, int count0) {
+                                                      int j0, int count0, int block, int blocks) {
   // per warp: a set of the ids accepted so far (open addressing, capacity a
   // power of two >= 2 n_out, -1 empty) in dynamic shared memory
   extern __shared__ int32_t s_sets[];
@@ -668,13 +675,13 @@ __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevG
   // without a node (the grid has a warp more than the nodes) and which no
   // other warp waits for; in the single-CTA minibatch kernel its latency
   // delayed every block barrier (2.8 us of each minibatch)
-  if (blockIdx.x == gridDim.x - 1 && warp == WARPS - 1 && lane == 0) {
+  if (block == blocks - 1 && warp == WARPS - 1 && lane == 0) {
     b.st->eps = eps_schedule(m.a, m.b, m.c, step);
     // iteration 0 of the launch moves the counter past its `count0`
     // iterations: the minibatch launch ahead has read it, nothing here does
     if (j0 == 0) b.gc->next_step = step + (uint32_t)count0;
   }
-  for (int slot = blockIdx.x * WARPS + warp; slot < n_nodes; slot += gridDim.x * WARPS) {
+  for (int slot = block * WARPS + warp; slot < n_nodes; slot += blocks * WARPS) {
     const int32_t i = b.nodes[slot];
     const int64_t r0 = g.row_ptr[i], r1 = g.row_ptr[i + 1], x0 = g.xrow[i], x1 = g.xrow[i + 1];
     const StagedRow links = stage_row(g.col, r0, r1, s_rows[warp], kRowCap, lane, 32);
@@ -739,20 +746,30 @@ __device__ __forceinline__ void sample_neighbors_body(const Model& m, const DevG
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_sample_neighbors(Model m, DevGraph g, Buffers b0, int s0) {
   const int j = blockIdx.y;
-  sample_neighbors_body<WARPS>(m, g, slot_buffers(m, b0, (s0 + j) % m.ring), j, (int)gridDim.y);
+  sample_neighbors_body<WARPS>(m, g, slot_buffers(m, b0, (s0 + j) % m.ring), j, (int)gridDim.y, blockIdx.x,
+                               gridDim.x);
 }
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_sample_neighbors_chains(const ChainArgs* __restrict__ c,
-                                                                      int s0) {
-  const ChainArgs& a = c[blockIdx.y];
-  const int j = blockIdx.z;
-  sample_neighbors_body<WARPS>(a.m, a.g, slot_buffers(a.m, a.b, s0 + j), j, (int)gridDim.z);
+                                                                      const BlockOf* __restrict__ map, int s0) {
+  const BlockOf o = map[blockIdx.x];
+  const ChainArgs& a = c[o.chain];
+  const int j = blockIdx.y;
+  sample_neighbors_body<WARPS>(a.m, a.g, slot_buffers(a.m, a.b, s0 + j), j, (int)gridDim.y, o.block, o.blocks);
 }
 
 // ---------------------------------------------------------------------------
 // k_update_phi: update_phi (cc:269-313) for NPB minibatch nodes per CTA,
 // SPLIT sub-groups of LPN lanes per node, each lane holding VPL 16-byte
 // vectors of a pi row.  Sub-group s takes neighbours s, s+SPLIT, ...
+//
+// A minibatch of narrow rows is too small to hide latency by occupancy (500
+// nodes are three warps per SM), so the chain of each node is kept short: U
+// rows' warp sums side by side, the next U rows and the words after them in
+// flight, and all that beta is not needed for -- ids, words, first rows, phi and
+// its sum, the normals -- before the wait for the theta step.  With one row at a
+// time and no early start, an iteration of the 5k-node workload (K = 32 FP32)
+// took 15.1 us, now 9.0.
 //
 // Algebra (exact rewrite of the reference's per-k loop).  With
 // pi_ik = phi_ik / S, sigma_j = +1 for y=1 else -1, e_j = y ? eps : 1-eps,
@@ -769,11 +786,19 @@ __global__ void __launch_bounds__(WARPS * 32) k_sample_neighbors_chains(const Ch
 // buffer (pi itself is written after all nodes, by k_commit_beta).
 // ---------------------------------------------------------------------------
 template <typename PiT, int LPN, int VPL, int SPLIT, int NPB>
-__device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b) {
+__device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b, int block, int blocks) {
   using TR = PiTraits<PiT>;
   constexpr int EV = TR::kPerVec;
   constexpr int EPL = VPL * EV;
   constexpr int TPN = SPLIT * LPN;
+  // rows a sub-group takes together (their dot products' sums overlap), with
+  // the next ones in flight: as many as keep a lane at 8 floats of them
+  constexpr int U = EPL <= 4 ? 4 : EPL <= 8 ? 2 : 1;
+  // a thread's elements of the epilogue: each sub-group covers the whole row,
+  // Kp <= LPN * EPL = TPN * EPL / SPLIT; few enough of them draw their normals
+  // ahead of the rows
+  constexpr int NQ = (EPL + SPLIT - 1) / SPLIT;
+  constexpr bool kEarlyNoise = NQ <= 4;
   extern __shared__ float s_dyn[];
   float* s_A = s_dyn;                               // NPB x SPLIT x Kp
   float* s_B = s_A + (size_t)NPB * SPLIT * m.Kp;    // NPB x SPLIT
@@ -794,14 +819,42 @@ __device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b
   const PiT* __restrict__ pi = reinterpret_cast<const PiT*>(b.pi);
   const Stream rs{m.seed, m.chain};
 
-  for (int base = blockIdx.x * NPB; base < n_nodes; base += gridDim.x * NPB) {
+  const int first = block * NPB;
+  for (int base = first; base < n_nodes; base += blocks * NPB) {
     const int slot = base + ln;
     const bool active = slot < n_nodes;
     float S = 0.f, s_i = 0.f, Bsum = 0.f;
+    int32_t i = 0;
+    float w[EPL], A[EPL], noise[NQ];
+    const uint32_t* nb = b.nbr + (int64_t)slot * m.n_out;
+    uint32_t word[U], word_n[U];  // neighbour words of a chunk and the next
+    uint4 cur[U][VPL], nxt[U][VPL];
+    auto load_words = [&](int q, uint32_t* out) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) out[u] = q + u * SPLIT < m.n_out ? nb[q + u * SPLIT] : 0u;
+    };
+    auto load_rows = [&](int q, const uint32_t* words, uint4 (*out)[VPL]) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool on = q + u * SPLIT < m.n_out;
+        const PiT* row = pi + (int64_t)(words[u] & 0x7fffffffu) * Kp;
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          const int vi = l + LPN * v;
+          out[u][v] = (on && vi < nvec) ? ldg_nc_v4(row + vi * EV) : make_uint4(0, 0, 0, 0);
+        }
+      }
+    };
+    auto noise_at = [&](int k) {
+      return b.fed_phi_noise ? b.fed_phi_noise[(int64_t)slot * K + k]
+                             : normal_draw(rs, kTagPhiNoise, (uint32_t)i, step, (uint64_t)k);
+    };
     if (active) {
-      const int32_t i = b.nodes[slot];
+      i = b.nodes[slot];
+      load_words(sg, word);
+      load_words(sg + U * SPLIT, word_n);
       const float* phi_i = b.phi + (int64_t)i * Kp;
-      float w[EPL], A[EPL];
+      load_rows(sg, word, cur);
       // phi row -> S
 #pragma unroll
       for (int v = 0; v < VPL; ++v) {
@@ -815,6 +868,16 @@ __device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b
       }
 #pragma unroll
       for (int o = LPN / 2; o > 0; o >>= 1) S += __shfl_xor_sync(gmask, S, o);
+      if constexpr (kEarlyNoise) {
+#pragma unroll
+        for (int qq = 0; qq < NQ; ++qq) noise[qq] = r + TPN * qq < K ? noise_at(r + TPN * qq) : 0.f;
+      }
+    }
+    // beta, read from here on, is written by the theta step ahead of this
+    // launch; everything read before was complete before that step started
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (active) {
       // pi_i = phi_i / S, s_i = sum pi_i, w = pi_i * (beta - epsilon)
 #pragma unroll
       for (int v = 0; v < VPL; ++v) {
@@ -832,53 +895,47 @@ __device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b
 #pragma unroll
       for (int o = LPN / 2; o > 0; o >>= 1) s_i += __shfl_xor_sync(gmask, s_i, o);
       const float one_m_si = 1.0f - s_i;
-      const uint32_t* nb = b.nbr + (int64_t)slot * m.n_out;
 
-      // neighbour loop, one row prefetched ahead
-      uint4 cur[VPL], nxt[VPL];
-      uint32_t wcur = 0, wnxt = 0;
-      int q = sg;
-      if (q < m.n_out) {
-        wcur = nb[q];
-        const PiT* row = pi + (int64_t)(wcur & 0x7fffffffu) * Kp;
+      // neighbour loop, U rows at a time, the next U prefetched
+      for (int q = sg; q < m.n_out; q += U * SPLIT) {
+        const int qn = q + U * SPLIT;
+        uint32_t word_f[U];
+        load_words(qn + U * SPLIT, word_f);
+        load_rows(qn, word_n, nxt);
+        float x[U][EPL], D[U];
 #pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          const int vi = l + LPN * v;
-          cur[v] = (vi < nvec) ? ldg_nc_v4(row + vi * EV) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) TR::unpack(cur[u][v], x[u] + v * EV);
+          float d4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) d4[e & 3] = fmaf(w[e], x[u][e], d4[e & 3]);
+          D[u] = (d4[0] + d4[1]) + (d4[2] + d4[3]);
         }
-      }
-      for (; q < m.n_out; q += SPLIT) {
-        const int qn = q + SPLIT;
-        if (qn < m.n_out) {
-          wnxt = nb[qn];
-          const PiT* row = pi + (int64_t)(wnxt & 0x7fffffffu) * Kp;
 #pragma unroll
-          for (int v = 0; v < VPL; ++v) {
-            const int vi = l + LPN * v;
-            nxt[v] = (vi < nvec) ? ldg_nc_v4(row + vi * EV) : make_uint4(0, 0, 0, 0);
-          }
+        for (int o = LPN / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int u = 0; u < U; ++u) D[u] += __shfl_xor_sync(gmask, D[u], o);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (u > 0 && q + u * SPLIT >= m.n_out) break;
+          const bool y = (word[u] >> 31) != 0;
+          const float sg_ = y ? 1.f : -1.f;
+          const float ej = y ? m.epsilon : 1.0f - m.epsilon;
+          const float P = fmaf(sg_, D[u], ej * s_i);
+          const float invP = rcp_approx(P);
+          const float cj = sg_ * invP;
+          Bsum += (ej * one_m_si - sg_ * D[u]) * invP;
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) A[e] = fmaf(cj, x[u][e], A[e]);
         }
-        float x[EPL];
 #pragma unroll
-        for (int v = 0; v < VPL; ++v) TR::unpack(cur[v], x + v * EV);
-        float d4[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int u = 0; u < U; ++u) {
+          word[u] = word_n[u];
+          word_n[u] = word_f[u];
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) d4[e & 3] = fmaf(w[e], x[e], d4[e & 3]);
-        float D = (d4[0] + d4[1]) + (d4[2] + d4[3]);
-#pragma unroll
-        for (int o = LPN / 2; o > 0; o >>= 1) D += __shfl_xor_sync(gmask, D, o);
-        const bool y = (wcur >> 31) != 0;
-        const float sg_ = y ? 1.f : -1.f;
-        const float ej = y ? m.epsilon : 1.0f - m.epsilon;
-        const float P = fmaf(sg_, D, ej * s_i);
-        const float invP = rcp_approx(P);
-        const float cj = sg_ * invP;
-        Bsum += (ej * one_m_si - sg_ * D) * invP;
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) A[e] = fmaf(cj, x[e], A[e]);
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) cur[v] = nxt[v];
-        wcur = wnxt;
+          for (int v = 0; v < VPL; ++v) cur[u][v] = nxt[u][v];
+        }
       }
       // publish A and B of this sub-group
       float* sA = s_A + ((size_t)ln * SPLIT + sg) * Kp;
@@ -894,13 +951,9 @@ __device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b
     }
     __syncthreads();
     // epilogue: TPN threads per node, element k = r + TPN * q
-    // each sub-group covers the whole row: Kp <= LPN * EPL = TPN * EPL / SPLIT
-    constexpr int NQ = (EPL + SPLIT - 1) / SPLIT;
     float pnew[NQ];
     float Snew = 0.f;
-    int32_t i = 0;
     if (active) {
-      i = b.nodes[slot];
       float Bt = 0.f;
 #pragma unroll
       for (int s = 0; s < SPLIT; ++s) Bt += s_B[ln * SPLIT + s];
@@ -917,11 +970,9 @@ __device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b
           for (int s = 0; s < SPLIT; ++s) Ak += s_A[((size_t)ln * SPLIT + s) * Kp + k];
           const float bk = b.beta[k] - m.epsilon;
           const float grad = (bk * Ak + Bt) * invS;
-          const float noise = b.fed_phi_noise
-                                  ? b.fed_phi_noise[(int64_t)slot * K + k]
-                                  : normal_draw(rs, kTagPhiNoise, (uint32_t)i, step, (uint64_t)k);
+          const float nz = kEarlyNoise ? noise[qq] : noise_at(k);
           const float ph = phi_i[k];
-          val = fabsf((ph + half_eps * (m.alpha - ph + m.Nn * grad)) + sqrtf(eps_t * ph) * noise);
+          val = fabsf((ph + half_eps * (m.alpha - ph + m.Nn * grad)) + sqrtf(eps_t * ph) * nz);
           if (val < 1.0e-24f) val = 1.0e-24f;
           phi_i[k] = val;
         }
@@ -952,16 +1003,19 @@ __device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b
     }
     __syncthreads();
   }
+  // CTAs with no work wait before they exit
+  if (first >= n_nodes) grid_dependency_wait();
 }
 template <typename PiT, int LPN, int VPL, int SPLIT, int NPB>
 __global__ void __launch_bounds__(NPB * SPLIT * LPN) k_update_phi(Model m, Buffers b) {
-  update_phi_body<PiT, LPN, VPL, SPLIT, NPB>(m, b);
+  update_phi_body<PiT, LPN, VPL, SPLIT, NPB>(m, b, blockIdx.x, gridDim.x);
 }
 template <typename PiT, int LPN, int VPL, int SPLIT, int NPB>
 __global__ void __launch_bounds__(NPB * SPLIT * LPN) k_update_phi_chains(const ChainArgs* __restrict__ c,
-                                                                         int p) {
-  const ChainArgs& a = c[blockIdx.y];
-  update_phi_body<PiT, LPN, VPL, SPLIT, NPB>(a.m, slot_buffers(a.m, a.b, p));
+                                                                         const BlockOf* __restrict__ map, int p) {
+  const BlockOf o = map[blockIdx.x];
+  const ChainArgs& a = c[o.chain];
+  update_phi_body<PiT, LPN, VPL, SPLIT, NPB>(a.m, slot_buffers(a.m, a.b, p), o.block, o.blocks);
 }
 
 // ---------------------------------------------------------------------------
@@ -974,15 +1028,18 @@ __global__ void __launch_bounds__(NPB * SPLIT * LPN) k_update_phi_chains(const C
 // theta factors), accumulated per warp in registers, then per block.
 // ---------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
-// The parts of k's theta step that do not depend on the sums:
-// 1/(theta0+theta1), the two gradient factors 1/theta_kc - 1/ts, and the two
-// noise terms sqrt(eps theta_kc) n_kc -- three FP64 divisions and two square
-// roots, about 2.5 us at GB300's FP64 rate.  They are formed by blocks of one
-// working warp (32 values of k) beside the commit's own, because nothing of
-// them waits for update_phi: in the theta kernel they were the longest part
-// between the commit's end and the step.
+// The parts of k's theta step that do not depend on the sums: theta and beta
+// themselves, eta_c - theta_kc, the noise terms sqrt(eps theta_kc) n_kc,
+// 1/(theta0+theta1) and the two gradient factors 1/theta_kc - 1/ts -- three FP64
+// divisions and two square roots, about 2.5 us at GB300's FP64 rate.  They are
+// formed by blocks of one working warp (32 values of k) beside the commit's
+// own, because nothing of them waits for update_phi: in the theta kernel they
+// were the longest part between the commit's end and the step.  (Folding the
+// step into one multiply-add per class and side saves six more dependent FP64
+// operations but rounds theta differently: the sum is kept as it was.)
 // ---------------------------------------------------------------------------
 static __device__ __forceinline__ void theta_pre_block(const Model& m, const Buffers& b, int block) {
+  grid_launch_dependents();
   const int k = block * 32 + (int)threadIdx.x;
   if (threadIdx.x < 32 && k < m.K) {
     const double eps_t = (double)b.st->eps;
@@ -997,11 +1054,17 @@ static __device__ __forceinline__ void theta_pre_block(const Model& m, const Buf
       n0 = normal_draw(rs, kTagThetaNoise, 0, b.st->step, 2ull * k);
       n1 = normal_draw(rs, kTagThetaNoise, 0, b.st->step, 2ull * k + 1);
     }
-    b.theta_pre[k] = ts_inv;
-    b.theta_pre[m.K + k] = 1.0 / th0 - ts_inv;
-    b.theta_pre[2 * m.K + k] = 1.0 / th1 - ts_inv;
-    b.theta_pre[3 * m.K + k] = sqrt(eps_t * th0) * n0;
-    b.theta_pre[4 * m.K + k] = sqrt(eps_t * th1) * n1;
+    double* out = b.theta_pre + k;
+    out[0] = th0;
+    out[m.K] = th1;
+    out[2 * m.K] = (double)m.eta0 - th0;
+    out[3 * m.K] = (double)m.eta1 - th1;
+    out[4 * m.K] = sqrt(eps_t * th0) * n0;
+    out[5 * m.K] = sqrt(eps_t * th1) * n1;
+    out[6 * m.K] = ts_inv;
+    out[7 * m.K] = 1.0 / th0 - ts_inv;
+    out[8 * m.K] = 1.0 / th1 - ts_inv;
+    out[9 * m.K] = (double)b.beta[k];
   }
   grid_dependency_wait();
 }
@@ -1028,15 +1091,16 @@ __device__ __forceinline__ float edge_inv_prob(float fsum, float psum, bool y, f
 }
 
 template <typename PiT, int KQ>
-__device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& b, int ncommit) {
+__device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& b, int ncommit, int block) {
   using TR = PiTraits<PiT>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int Kp = m.Kp, K = m.K;
-  if ((int)blockIdx.x >= ncommit + m.nbb) {
-    theta_pre_block(m, b, (int)blockIdx.x - ncommit - m.nbb);
+  if (block >= ncommit + m.nbb) {
+    theta_pre_block(m, b, block - ncommit - m.nbb);
     return;
   }
-  if ((int)blockIdx.x < ncommit) {
+  grid_launch_dependents();
+  if (block < ncommit) {
     const int n_nodes = b.st->n_nodes;
     constexpr int EV = TR::kPerVec;
     PiT* pi = reinterpret_cast<PiT*>(b.pi);
@@ -1044,8 +1108,7 @@ __device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& 
     // the staged rows come from update_phi, the launch ahead of this one,
     // which also still reads the pi rows written here
     grid_dependency_wait();
-    grid_launch_dependents();
-    for (int slot = blockIdx.x * 4 + warp; slot < n_nodes; slot += ncommit * 4) {
+    for (int slot = block * 4 + warp; slot < n_nodes; slot += ncommit * 4) {
       const int32_t i = b.nodes[slot];
       const float* src = b.stage + (int64_t)slot * Kp;
       PiT* dst = pi + (int64_t)i * Kp;
@@ -1067,7 +1130,7 @@ __device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& 
     return;
   }
   __shared__ float s_part[4][2][KQ * 128];
-  const int bb = blockIdx.x - ncommit;
+  const int bb = block - ncommit;
   const int n_edges = b.st->n_edges;
   if (bb * 4 >= n_edges) {  // no edges for this block: k_theta skips its partial
     grid_dependency_wait();
@@ -1084,7 +1147,6 @@ __device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& 
       bt[q * 4 + e] = (k < K) ? b.beta[k] : 0.f;
     }
   grid_dependency_wait();  // the staged rows (update_phi)
-  grid_launch_dependents();
   for (int ed = bb * 4 + warp; ed < n_edges; ed += m.nbb * 4) {
     const float* pa = b.stage + (int64_t)b.ea[ed] * Kp;
     const float* pb = b.stage + (int64_t)b.eb[ed] * Kp;
@@ -1134,12 +1196,14 @@ __device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& 
 }
 template <typename PiT, int KQ>
 __global__ void __launch_bounds__(128) k_commit_beta(Model m, Buffers b, int ncommit) {
-  commit_beta_body<PiT, KQ>(m, b, ncommit);
+  commit_beta_body<PiT, KQ>(m, b, ncommit, blockIdx.x);
 }
 template <typename PiT, int KQ>
-__global__ void __launch_bounds__(128) k_commit_beta_chains(const ChainArgs* __restrict__ c, int p) {
-  const ChainArgs& a = c[blockIdx.y];
-  commit_beta_body<PiT, KQ>(a.m, slot_buffers(a.m, a.b, p), a.ncommit);
+__global__ void __launch_bounds__(128) k_commit_beta_chains(const ChainArgs* __restrict__ c,
+                                                            const BlockOf* __restrict__ map, int p) {
+  const BlockOf o = map[blockIdx.x];
+  const ChainArgs& a = c[o.chain];
+  commit_beta_body<PiT, KQ>(a.m, slot_buffers(a.m, a.b, p), a.ncommit, o.block);
 }
 
 // ---------------------------------------------------------------------------
@@ -1171,7 +1235,7 @@ constexpr size_t commit_star_smem(int Kp) {  // f, the source's row, w, 1 / P
 }
 
 template <typename PiT, int KQ, int JC>
-__device__ __forceinline__ void commit_star_body(const Model& m, const Buffers& b) {
+__device__ __forceinline__ void commit_star_body(const Model& m, const Buffers& b, int block) {
   constexpr int NT = 128 * JC;
   constexpr int NIT = (KQ * 64 + NT - 1) / NT;  // float pairs of k per thread
   extern __shared__ __align__(16) float s_star[];
@@ -1181,11 +1245,12 @@ __device__ __forceinline__ void commit_star_body(const Model& m, const Buffers& 
   float* s_w = s_xa + Kp;            // beta or 1 - beta
   float* s_inv = s_w + Kp;           // 4*JC
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int bb = blockIdx.x, n_edges = b.st->n_edges, per = m.nbb * 4;
+  const int bb = block, n_edges = b.st->n_edges, per = m.nbb * 4;
   if (bb >= m.nbb) {
     theta_pre_block(m, b, bb - m.nbb);
     return;
   }
+  grid_launch_dependents();
   if (bb * 4 >= n_edges) {
     grid_dependency_wait();
     return;
@@ -1204,7 +1269,6 @@ __device__ __forceinline__ void commit_star_body(const Model& m, const Buffers& 
   // the staged rows come from update_phi, the launch ahead of this one,
   // which also still reads the pi rows written here
   grid_dependency_wait();
-  grid_launch_dependents();
   for (int k = 4 * tid; k < Kp; k += 4 * NT) {
     const float4 x = *reinterpret_cast<const float4*>(b.stage + k);
     *reinterpret_cast<float4*>(s_xa + k) = x;
@@ -1268,12 +1332,15 @@ __device__ __forceinline__ void commit_star_body(const Model& m, const Buffers& 
 }
 template <typename PiT, int KQ, int JC>
 __global__ void __launch_bounds__(128 * JC, JC == 1 ? 4 : 2) k_commit_star(Model m, Buffers b) {
-  commit_star_body<PiT, KQ, JC>(m, b);
+  commit_star_body<PiT, KQ, JC>(m, b, blockIdx.x);
 }
 template <typename PiT, int KQ, int JC>
-__global__ void __launch_bounds__(128 * JC, JC == 1 ? 4 : 2) k_commit_star_chains(const ChainArgs* __restrict__ c, int p) {
-  const ChainArgs& a = c[blockIdx.y];
-  commit_star_body<PiT, KQ, JC>(a.m, slot_buffers(a.m, a.b, p));
+__global__ void __launch_bounds__(128 * JC, JC == 1 ? 4 : 2) k_commit_star_chains(const ChainArgs* __restrict__ c,
+                                                                              const BlockOf* __restrict__ map,
+                                                                              int p) {
+  const BlockOf o = map[blockIdx.x];
+  const ChainArgs& a = c[o.chain];
+  commit_star_body<PiT, KQ, JC>(a.m, slot_buffers(a.m, a.b, p), o.block);
 }
 
 // ---------------------------------------------------------------------------
@@ -1288,11 +1355,10 @@ __global__ void __launch_bounds__(128 * JC, JC == 1 ? 4 : 2) k_commit_star_chain
 // partials are k_commit_star's, of the minibatch's y alone.
 //
 // A latency chain (partial loads, compensated sums, FP64 at 1/64 of the FP32
-// rate), so what does not need the partials is done elsewhere: the divisions,
-// square roots and normals beside the commit (theta_pre_block), the scalars,
-// theta, beta and the counters before the wait.  256 threads rather than
-// 1,024, so that the CTA fits an SM that still holds commit CTAs.
-static __device__ __forceinline__ void theta_body(const Model& m, const Buffers& b, int star,
+// rate), so what does not need the partials is done beside the commit
+// (theta_pre_block) and two FMA chains and a division are left.  256 threads
+// rather than 1,024, so that the CTA fits an SM that still holds commit CTAs.
+static __device__ __forceinline__ void theta_body(const Model& m, const Buffers& b, int star, int block,
                                                   const double* R_given = nullptr,
                                                   double* R_out = nullptr) {
   // 32 consecutive k per CTA (lane = k).  31 chains add the partials of the
@@ -1302,20 +1368,13 @@ static __device__ __forceinline__ void theta_body(const Model& m, const Buffers&
   constexpr int C = kThetaChains, P = kThetaPerChain, W = kThetaThreads / 32, CW = (C + W - 1) / W;
   __shared__ float s_r[2][C][33], s_c[2][C][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k = blockIdx.x * 32 + lane;
+  const int k = block * 32 + lane;
   const int Kp = m.Kp;
   const int active = min(m.nbb, (b.st->n_edges + 3) / 4);  // blocks that saw edges
-  const double eps_t = (double)b.st->eps;
-  const double scale = (double)b.st->scale;
+  const double half_eps = (double)b.st->eps / 2.0, scale = (double)b.st->scale;
   const bool kin = k < m.K;
   const int only = star && active > 0 ? (b.ey[0] ? 1 : 0) : -1;  // the class with partials
-  double th0 = 1.0, th1 = 1.0, bt = 0.0;
-  if (warp == 0 && kin && !R_out) {
-    th0 = b.theta[2 * k];
-    th1 = b.theta[2 * k + 1];
-    bt = (double)b.beta[k];
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 32 && !R_out) {
+  if (block == 0 && threadIdx.x == 32 && !R_out) {
     // the iteration's edge evaluations and errors, counted as it is applied
     if (b.st->err) atomicOr(&b.gc->err, b.st->err);
     b.gc->evals += (unsigned long long)b.st->n_nodes * (unsigned long long)m.n_out;
@@ -1323,9 +1382,9 @@ static __device__ __forceinline__ void theta_body(const Model& m, const Buffers&
   }
   grid_dependency_wait();  // the beta partials and theta_pre: the commit, the launch ahead
   grid_launch_dependents();
-  double pre[5];
+  double pre[kThetaPre];
 #pragma unroll
-  for (int i = 0; i < 5; ++i) pre[i] = (warp == 0 && kin && !R_out) ? b.theta_pre[i * m.K + k] : 0.0;
+  for (int i = 0; i < kThetaPre; ++i) pre[i] = (warp == 0 && kin && !R_out) ? b.theta_pre[i * m.K + k] : 0.0;
   double R[2] = {0.0, 0.0};
   if (R_given) {
     if (warp != 0 || !kin) return;
@@ -1382,12 +1441,18 @@ static __device__ __forceinline__ void theta_body(const Model& m, const Buffers&
       return;
     }
   }
-  const double R0 = R[0], R1 = R[1];
-  const double ts_inv = pre[0], f0 = pre[1], f1 = pre[2], nz0 = pre[3], nz1 = pre[4];
-  const double G0 = bt * R1 * (-ts_inv) + (1.0 - bt) * R0 * f0;
-  const double G1 = bt * R1 * f1 + (1.0 - bt) * R0 * (-ts_inv);
-  double t0 = fabs(th0 + eps_t / 2.0 * ((double)m.eta0 - th0 + scale * G0) + nz0);
-  double t1 = fabs(th1 + eps_t / 2.0 * ((double)m.eta1 - th1 + scale * G1) + nz1);
+  const double th0 = pre[0], th1 = pre[1], ts_inv = pre[6], f0 = pre[7], f1 = pre[8], bt = pre[9];
+  double G0, G1;
+  if (only >= 0) {  // one of the sums is zero, and its products
+    const double g = only ? bt * R[1] : (1.0 - bt) * R[0];
+    G0 = g * (only ? -ts_inv : f0);
+    G1 = g * (only ? f1 : -ts_inv);
+  } else {
+    G0 = bt * R[1] * (-ts_inv) + (1.0 - bt) * R[0] * f0;
+    G1 = bt * R[1] * f1 + (1.0 - bt) * R[0] * (-ts_inv);
+  }
+  double t0 = fabs(th0 + half_eps * (pre[2] + scale * G0) + pre[4]);
+  double t1 = fabs(th1 + half_eps * (pre[3] + scale * G1) + pre[5]);
   if (t0 < 1.0e-24) t0 = 1.0e-24;
   if (t1 < 1.0e-24) t1 = 1.0e-24;
   b.theta[2 * k] = t0;
@@ -1395,19 +1460,21 @@ static __device__ __forceinline__ void theta_body(const Model& m, const Buffers&
   b.beta[k] = (float)(t1 / (t0 + t1));
 }
 static __global__ void __launch_bounds__(kThetaThreads) k_theta(Model m, Buffers b, int star) {
-  theta_body(m, b, star);
+  theta_body(m, b, star, blockIdx.x);
 }
 // the per-k sums R0, R1 of the beta partials, without the step
 static __global__ void __launch_bounds__(kThetaThreads) k_beta_sums(Model m, Buffers b, double* R_out) {
-  theta_body(m, b, 0, nullptr, R_out);
+  theta_body(m, b, 0, blockIdx.x, nullptr, R_out);
 }
 // the theta step from given sums
 static __global__ void __launch_bounds__(kThetaThreads) k_theta_given(Model m, Buffers b, const double* R) {
-  theta_body(m, b, 0, R, nullptr);
+  theta_body(m, b, 0, blockIdx.x, R, nullptr);
 }
-static __global__ void __launch_bounds__(kThetaThreads) k_theta_chains(const ChainArgs* __restrict__ c, int p) {
-  const ChainArgs& a = c[blockIdx.y];
-  theta_body(a.m, slot_buffers(a.m, a.b, p), a.star);
+static __global__ void __launch_bounds__(kThetaThreads) k_theta_chains(const ChainArgs* __restrict__ c,
+                                                                       const BlockOf* __restrict__ map, int p) {
+  const BlockOf o = map[blockIdx.x];
+  const ChainArgs& a = c[o.chain];
+  theta_body(a.m, slot_buffers(a.m, a.b, p), a.star, o.block);
 }
 
 // ---------------------------------------------------------------------------

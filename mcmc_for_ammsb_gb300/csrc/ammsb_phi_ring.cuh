@@ -516,19 +516,19 @@ template <typename PiT>
 __host__ __device__ constexpr int ring_few_stages() { return sizeof(PiT) == 2 ? 4 : 2; }
 
 template <typename PiT, int VPL, int STAGES, bool FULL>
-__device__ __forceinline__ void update_phi_ring_any(const Model& m, const Buffers& b, int few, int parts) {
+__device__ __forceinline__ void update_phi_ring_any(const Model& m, const Buffers& b, int few, int parts, int block,
+                                                    int blocks) {
   extern __shared__ __align__(128) unsigned char s_ring[];
   const int n_nodes = b.st->n_nodes;
   if (n_nodes <= few) {
     if (parts & kPhiFew)
-      update_phi_ring_body<PiT, VPL, 16, ring_few_stages<PiT>(), FULL, false>(m, b, s_ring, 0, blockIdx.x,
-                                                                              gridDim.x);
+      update_phi_ring_body<PiT, VPL, 16, ring_few_stages<PiT>(), FULL, false>(m, b, s_ring, 0, block, blocks);
   } else if (parts & kPhiMany) {
     const int per = blockDim.x / kPhiGroup, group = threadIdx.x / kPhiGroup;
     const int Kp = FULL ? 32 * VPL * PiTraits<PiT>::kPerVec : m.Kp;
     update_phi_ring_body<PiT, VPL, 4, STAGES, FULL, true>(
         m, b, s_ring + group * PhiRingSmem<PiT, VPL, 4, STAGES>::bytes(Kp, m.n_out), group,
-        blockIdx.x * per + group, gridDim.x * per);
+        block * per + group, blocks * per);
   }
   // CTAs with no work wait for the kernel ahead before they exit, so that
   // this launch completes after it
@@ -536,13 +536,15 @@ __device__ __forceinline__ void update_phi_ring_any(const Model& m, const Buffer
 }
 template <typename PiT, int VPL, int STAGES, bool FULL>
 __global__ void __launch_bounds__(512, 1) k_update_phi_ring(Model m, Buffers b, int few, int parts) {
-  update_phi_ring_any<PiT, VPL, STAGES, FULL>(m, b, few, parts);
+  update_phi_ring_any<PiT, VPL, STAGES, FULL>(m, b, few, parts, blockIdx.x, gridDim.x);
 }
 template <typename PiT, int VPL, int STAGES, bool FULL>
-__global__ void __launch_bounds__(512, 1) k_update_phi_ring_chains(const ChainArgs* __restrict__ c, int p, int few,
+__global__ void __launch_bounds__(512, 1) k_update_phi_ring_chains(const ChainArgs* __restrict__ c,
+                                                                   const BlockOf* __restrict__ map, int p, int few,
                                                                    int parts) {
-  const ChainArgs& a = c[blockIdx.y];
-  update_phi_ring_any<PiT, VPL, STAGES, FULL>(a.m, slot_buffers(a.m, a.b, p), few, parts);
+  const BlockOf o = map[blockIdx.x];
+  const ChainArgs& a = c[o.chain];
+  update_phi_ring_any<PiT, VPL, STAGES, FULL>(a.m, slot_buffers(a.m, a.b, p), few, parts, o.block, o.blocks);
 }
 
 }  // namespace ammsb
