@@ -1480,14 +1480,14 @@ static __global__ void __launch_bounds__(kThetaThreads) k_theta_chains(const Cha
 // ---------------------------------------------------------------------------
 // Held-out perplexity (learner.cc:138-183, learner.h:100-139): LPN lanes per
 // held-out edge; running average per edge in FP32 as the reference; the log
-// sum in FP64.  A block takes PpxPlan::per_block consecutive edges; their
-// averages go through shared memory so that the logarithms are taken by a
-// thread each (one lane's FP64 logarithm costs its warp as much as 32: with
-// the lane that formed the average taking it, 86,246 pairs of K = 1024 BF16
-// took 262 us, of which the rows are 53).  The block that finishes last adds
-// the blocks' partials, in a fixed order, so the result does not depend on
-// which it is; one thread adding a block's 256 values, and a second launch for
-// the partials, were 20 us of a small set's call.
+// sum in FP64.  A block takes PpxPlan::per_block consecutive edges.  A lane
+// group keeps its edges' averages a lane each, and the lanes then take the
+// logarithms side by side (one lane's FP64 logarithm costs its warp as much as
+// 32: with the lane that formed an average taking its logarithm, 86,246 pairs of
+// K = 1024 BF16 took 262 us, of which the rows are 53).  The block that finishes
+// last adds the blocks' partials, in a fixed order, so the result does not
+// depend on which it is; one thread adding a block's 256 values, and a second
+// launch for the partials, were 20 us of a small set's call.
 // ---------------------------------------------------------------------------
 struct PpxResult {
   double value;
@@ -1497,13 +1497,14 @@ struct PpxResult {
   uint32_t pad;
 };
 
-// Edges a block's lane groups take at a time (up to four each), and edges and
-// blocks of a call: at most kPpxMaxBlocks partials.
+// Edges a lane group takes at a time, eight of them or a lane each; the edges
+// and blocks of a call: at most kPpxMaxBlocks partials.
 constexpr int kPpxMaxBlocks = 16384;
 struct PpxPlan {
   int per_block, blocks;
 };
-__host__ __device__ constexpr int ppx_chunk(int lpn) { return 4 * (256 / lpn) < 256 ? 4 * (256 / lpn) : 256; }
+__host__ __device__ constexpr int ppx_edges(int lpn) { return lpn < 8 ? lpn : 8; }
+__host__ __device__ constexpr int ppx_chunk(int lpn) { return ppx_edges(lpn) * (256 / lpn); }
 inline PpxPlan ppx_plan(int lpn, int64_t H) {
   const int64_t chunk = ppx_chunk(lpn), need = (H + kPpxMaxBlocks - 1) / kPpxMaxBlocks;
   const int64_t per = (need < 1 ? 1 : (need + chunk - 1) / chunk) * chunk;
@@ -1529,7 +1530,7 @@ __device__ __forceinline__ double block_sum_256(double v, double* s) {
 }
 
 template <typename PiT, int LPN, int VPL>
-__global__ void __launch_bounds__(256) k_perplexity(Model m, const PiT* __restrict__ pi,
+__global__ void __launch_bounds__(256, VPL >= 8 ? 2 : VPL >= 4 ? 3 : 4) k_perplexity(Model m, const PiT* __restrict__ pi,
                                                     const float* __restrict__ beta,
                                                     const int32_t* __restrict__ ha,
                                                     const int32_t* __restrict__ hb,
@@ -1540,8 +1541,10 @@ __global__ void __launch_bounds__(256) k_perplexity(Model m, const PiT* __restri
   using TR = PiTraits<PiT>;
   constexpr int EV = TR::kPerVec;
   constexpr int EPL = VPL * EV;
-  constexpr int GPB = 256 / LPN, CH = ppx_chunk(LPN), J = CH / GPB;
-  __shared__ float s_avg[CH];
+  constexpr int GPB = 256 / LPN, CH = ppx_chunk(LPN), J = ppx_edges(LPN);
+  // beta in shared memory, not registers: 32 of them a lane left an SM with two
+  // blocks instead of three (four measured no better)
+  __shared__ __align__(16) float s_beta[LPN * EPL];
   __shared__ double s_sum[256];
   __shared__ int s_last;
   const int tid = threadIdx.x, grp = tid / LPN, l = tid % LPN, lane = tid & 31;
@@ -1549,44 +1552,31 @@ __global__ void __launch_bounds__(256) k_perplexity(Model m, const PiT* __restri
   // rows are Kp apart; only the vectors that hold the K values are read,
   // and elements past K (row padding) take no part in either sum
   const int Kp = m.Kp, K = m.K, nvec = (K + EV - 1) / EV;
-  float bt[EPL];
-#pragma unroll
-  for (int v = 0; v < VPL; ++v)
-#pragma unroll
-    for (int e = 0; e < EV; ++e) {
-      const int k = (l + LPN * v) * EV + e;
-      bt[v * EV + e] = (k < K) ? beta[k] : 0.f;
-    }
+  for (int k = tid; k < LPN * EPL; k += 256) s_beta[k] = (k < K) ? beta[k] : 0.f;
+  __syncthreads();
   const int64_t e0 = (int64_t)blockIdx.x * per_block;
   const int64_t e1 = e0 + per_block < H ? e0 + per_block : H;
   double sum = 0.0, comp = 0.0;
   for (int64_t c0 = e0; c0 < e1; c0 += CH) {
-    int32_t a[J], b[J];
-    bool y[J];
-    float old[J];
-#pragma unroll
+    float mine = 1.f;  // the average of the lane's edge (logarithm 0: none)
+    // lane j reads edge j's words and passes them on
+    const int64_t own = c0 + grp + GPB * l;
+    const bool on = l < J && own < e1;
+    const int32_t own_a = on ? ha[own] : -1, own_b = on ? hb[own] : -1;
+    const int own_y = on && hy[own] != 0;
+    const float old = on ? ppx[own] : 0.f;
+#pragma unroll 2
     for (int j = 0; j < J; ++j) {
-      const int64_t ed = c0 + grp + GPB * j;
-      const bool on = ed < e1;
-      a[j] = on ? ha[ed] : -1;
-      b[j] = on ? hb[ed] : -1;
-      y[j] = on && hy[ed] != 0;
-      old[j] = on ? ppx[ed] : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const int64_t ed = c0 + grp + GPB * j;
-      if (ed >= e1) break;
+      if (c0 + grp + GPB * j >= e1) break;
+      const int32_t a = __shfl_sync(gmask, own_a, j, LPN), b = __shfl_sync(gmask, own_b, j, LPN);
+      const bool y = __shfl_sync(gmask, own_y, j, LPN) != 0;
       // a pair naming a row outside pi is skipped (no row is read) and flagged
-      if ((uint64_t)(int64_t)a[j] >= (uint64_t)n_rows || (uint64_t)(int64_t)b[j] >= (uint64_t)n_rows) {
-        if (l == 0) {
-          atomicOr(&res->bad, 1u);
-          s_avg[grp + GPB * j] = 1.f;
-        }
+      if ((uint64_t)(int64_t)a >= (uint64_t)n_rows || (uint64_t)(int64_t)b >= (uint64_t)n_rows) {
+        if (l == 0) atomicOr(&res->bad, 1u);
         continue;
       }
-      const PiT* ra = pi + (int64_t)a[j] * Kp;
-      const PiT* rb = pi + (int64_t)b[j] * Kp;
+      const PiT* ra = pi + (int64_t)a * Kp;
+      const PiT* rb = pi + (int64_t)b * Kp;
       uint4 va[VPL], vb[VPL];
 #pragma unroll
       for (int v = 0; v < VPL; ++v) {
@@ -1599,15 +1589,18 @@ __global__ void __launch_bounds__(256) k_perplexity(Model m, const PiT* __restri
       for (int v = 0; v < VPL; ++v) {
         const int vi = l + LPN * v;
         if (vi < nvec) {
-          float xa[EV], xb[EV];
+          float xa[EV], xb[EV], bt[EV];
           TR::unpack(va[v], xa);
           TR::unpack(vb[v], xb);
+#pragma unroll
+          for (int e = 0; e < EV; e += 4)
+            *reinterpret_cast<float4*>(bt + e) = *reinterpret_cast<const float4*>(s_beta + vi * EV + e);
 #pragma unroll
           for (int e = 0; e < EV; ++e) {
             if (vi * EV + e < K) {
               const float f = xa[e] * xb[e];
               fs += f;
-              s += f * (y[j] ? bt[v * EV + e] : 1.0f - bt[v * EV + e]);
+              s += f * (y ? bt[e] : 1.0f - bt[e]);
             }
           }
         }
@@ -1617,22 +1610,17 @@ __global__ void __launch_bounds__(256) k_perplexity(Model m, const PiT* __restri
         s += __shfl_xor_sync(gmask, s, o);
         fs += __shfl_xor_sync(gmask, fs, o);
       }
-      if (l == 0) {
-        if (!y[j]) s += (1.0f - fs) * (1.0f - m.epsilon);
+      if (l == j) {
+        if (!y) s += (1.0f - fs) * (1.0f - m.epsilon);
         if (s < 1.0e-30f) s = 1.0e-30f;
-        const float avg = (old[j] * (count - 1.0f) + s) / count;
-        ppx[ed] = avg;
-        s_avg[grp + GPB * j] = avg;
+        mine = (old * (count - 1.0f) + s) / count;
+        ppx[own] = mine;
       }
     }
-    __syncthreads();
-    if (tid < CH && c0 + tid < e1) {
-      const double term = log((double)s_avg[tid]) - comp;
-      const double tsum = sum + term;
-      comp = (tsum - sum) - term;
-      sum = tsum;
-    }
-    __syncthreads();
+    const double term = log((double)mine) - comp;
+    const double tsum = sum + term;
+    comp = (tsum - sum) - term;
+    sum = tsum;
   }
   double total = block_sum_256(sum - comp, s_sum);
   if (tid == 0) {
