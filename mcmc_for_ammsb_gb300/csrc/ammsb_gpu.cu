@@ -443,6 +443,41 @@ int check_draw_err(ammsb_handle* h, int slot) {
   return rc ? rc : device_err_status(h, st.err);
 }
 
+// Rows of pi or phi into a host array of N x K floats.  FP32 rows are copied;
+// BF16 rows are widened on the device, a staging buffer at a time (a kernel and
+// a copy each: widening them on the host was 0.9 of the 1.05 ms that 5M values
+// took), after their host pages have been touched, as the host loop did: a copy
+// into pages of a fresh array has the GPU fault them in (4 ms for 20 MB, not 1).
+constexpr size_t kReadBytes = 8u << 20;
+template <typename T>
+int get_rows(ammsb_handle* h, const T* rows, float* dst) {
+  const int64_t N = h->m.N, K = h->m.K, Kp = h->m.Kp;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (K == Kp)
+      CK(cudaMemcpyAsync(dst, rows, sizeof(float) * (size_t)N * K, cudaMemcpyDeviceToHost, h->stream));
+    else
+      CK(cudaMemcpy2DAsync(dst, sizeof(float) * K, rows, sizeof(float) * Kp, sizeof(float) * K, N,
+                           cudaMemcpyDeviceToHost, h->stream));
+  } else {
+    const int64_t per = std::min<int64_t>(N, std::max<int64_t>(1, (int64_t)(kReadBytes / sizeof(float)) / K));
+    if (!h->d_read) {
+      int rc = dev_alloc(h, &h->d_read, (size_t)(per * K));
+      if (rc) return rc;
+    }
+    volatile char* page = reinterpret_cast<volatile char*>(dst);
+    for (size_t x = 0; x < sizeof(float) * (size_t)(N * K); x += 4096) page[x] = 0;
+    for (int64_t r = 0; r < N; r += per) {
+      const int64_t n = std::min(per, N - r);
+      k_widen_rows<<<(int)std::min<int64_t>((n * K + 255) / 256, 152 * 16), 256, 0, h->stream>>>(
+          rows + r * Kp, (int)K, (int)Kp, n, h->d_read);
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(dst + r * K, h->d_read, sizeof(float) * (size_t)(n * K), cudaMemcpyDeviceToHost, h->stream));
+    }
+  }
+  CK(cudaStreamSynchronize(h->stream));
+  return AMMSB_OK;
+}
+
 // Drops draws made ahead of time (their step no longer follows, or their
 // buffer sets are about to be written).
 void invalidate_prefetch(ammsb_handle* h) {
@@ -769,11 +804,12 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
           f(s->b[i], s->a[i]);
         }
     };
-    each([&](int32_t a, int32_t) { ++xrow[(size_t)a + 1]; });
-    for (int64_t v = 0; v < N; ++v) xrow[v + 1] += xrow[v];
+    // counts, their running sums (each row's end), then every entry placed
+    // below its row's end, which leaves the row's start
+    each([&](int32_t a, int32_t) { ++xrow[a]; });
+    for (int64_t v = 1; v <= N; ++v) xrow[v] += xrow[v - 1];
     std::vector<int32_t> xcol((size_t)std::max<int64_t>(xrow[N], 1));
-    std::vector<int64_t> at(xrow.begin(), xrow.end() - 1);
-    each([&](int32_t a, int32_t b) { xcol[at[a]++] = b; });
+    each([&](int32_t a, int32_t b) { xcol[--xrow[a]] = b; });
     for (int64_t v = 0; v < N; ++v)
       if (xrow[v + 1] - xrow[v] > 1) std::sort(xcol.begin() + xrow[v], xcol.begin() + xrow[v + 1]);
     int64_t* d_xrow = nullptr;
@@ -1273,32 +1309,14 @@ int ammsb_run(ammsb_handle* h, double* last) {
 int ammsb_get_pi(ammsb_handle* h, float* dst) {
   if (!h || !dst) return AMMSB_E_ARG;
   CK(cudaSetDevice(h->device));
-  const int K = h->m.K, Kp = h->m.Kp;
-  const int64_t N = h->m.N;
-  if (h->opt.pi_dtype == AMMSB_PI_F32) {
-    CK(cudaMemcpy2DAsync(dst, sizeof(float) * K, h->b.pi, sizeof(float) * Kp, sizeof(float) * K, N,
-                         cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-  } else {
-    std::vector<uint16_t> tmp((size_t)N * K);
-    CK(cudaMemcpy2DAsync(tmp.data(), 2 * K, h->b.pi, 2 * Kp, 2 * K, N, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    for (size_t x = 0; x < tmp.size(); ++x) {
-      uint32_t u = (uint32_t)tmp[x] << 16;
-      std::memcpy(dst + x, &u, 4);
-    }
-  }
-  return AMMSB_OK;
+  return h->opt.pi_dtype == AMMSB_PI_BF16 ? get_rows(h, static_cast<const __nv_bfloat16*>(h->b.pi), dst)
+                                          : get_rows(h, static_cast<const float*>(h->b.pi), dst);
 }
 
 int ammsb_get_phi(ammsb_handle* h, float* dst) {
   if (!h || !dst) return AMMSB_E_ARG;
   CK(cudaSetDevice(h->device));
-  const int K = h->m.K, Kp = h->m.Kp;
-  CK(cudaMemcpy2DAsync(dst, sizeof(float) * K, h->b.phi, sizeof(float) * Kp, sizeof(float) * K, h->m.N,
-                       cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
-  return AMMSB_OK;
+  return get_rows(h, h->b.phi, dst);
 }
 
 int ammsb_get_theta(ammsb_handle* h, double* dst) {

@@ -79,6 +79,7 @@ struct ammsb_handle {
   uint8_t* d_hy = nullptr;
   float* d_ppx = nullptr;
   double* d_ppx_part = nullptr;
+  float* d_read = nullptr;  // staging of get_rows, allocated with the first read that needs it
   PpxResult* d_ppx_res = nullptr;
   float* d_fed_phi_noise = nullptr;
   float* d_fed_theta_noise = nullptr;

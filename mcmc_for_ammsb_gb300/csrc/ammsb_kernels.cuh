@@ -1702,4 +1702,25 @@ __global__ void k_normalize_rows(Model m, const float* phi, PiT* pi) {
   }
 }
 
+// n rows of K elements (stride Kp) as packed floats.
+template <typename T>
+__global__ void __launch_bounds__(256) k_widen_rows(const T* __restrict__ rows, int K, int Kp, int64_t n,
+                                                   float* __restrict__ out) {
+  const int64_t total = n * K, stride = (int64_t)gridDim.x * 256;
+  const int64_t dr = stride / K;
+  const int dk = (int)(stride - dr * K);
+  int64_t x = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  int64_t r = x / K;
+  int k = (int)(x - r * K);
+  for (; x < total; x += stride) {
+    out[x] = (float)rows[r * Kp + k];
+    r += dr;
+    k += dk;
+    if (k >= K) {
+      k -= K;
+      ++r;
+    }
+  }
+}
+
 }  // namespace ammsb
