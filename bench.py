@@ -274,9 +274,9 @@ def ours_arm(args, net, opts, rank, world, local):
     torch.cuda.synchronize()
     if world > 1:
         torch.distributed.barrier()
-    # kernels per iteration: minibatch, neighbour sets, update_phi (the ring
-    # kernel launches its many-node and few-node variants), commit/beta, theta
-    launches_per_iter = 6 if s.kernel_config()["ring"] else 5
+    # kernels: update_phi, commit/beta and theta of every iteration, and the
+    # minibatch and neighbour draws of each block of eight
+    launches = 3 * args.steps + 2 * (args.steps // 8)
     e0, i0 = s.counters()
     clocks = ClockSampler(local)
     clocks.start()
@@ -389,7 +389,7 @@ def ours_arm(args, net, opts, rank, world, local):
                                       int(net.held_out[0].shape[0])),
             "parallelism": "replicas" if world > 1 else "single",
             "iterations_per_s": (i1 - i0) / secs if world == 1 else None,
-            "gpu_launches": launches_per_iter * args.steps,
+            "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": achieved,
                          "peak": peaks.get("hbm_gbs", PEAKS_FALLBACK["hbm_gbs"]),
                          "unit": "GB/s", "frac": achieved / peaks.get("hbm_gbs", 6800.0),

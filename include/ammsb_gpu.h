@@ -249,11 +249,11 @@ int ammsb_get_kernel_config(ammsb_handle *h, int32_t *out);
 
 /* Batches of independent chains (no reference counterpart): the
  * iterations of many handles -- each with its own graph, held-out set,
- * state, options and update_phi configuration -- advanced together, one
- * CUDA graph launch per iteration for all of them.  Each kernel of the
- * iteration runs once for all chains sharing its compiled shape (the chain
- * is the grid's y index), so chains of different sizes and row widths take
- * a handful of launches per iteration instead of five each.  A chain goes
+ * state, options and update_phi configuration -- advanced together by
+ * CUDA graphs of up to 16 iterations of all of them.  Each kernel of the
+ * iteration runs once for all chains sharing its compiled shape (a map
+ * gives each block its chain), so chains of different sizes and row widths
+ * take a handful of launches per iteration instead of three each.  A chain goes
  * through exactly the states it goes through when stepped on its own (same
  * kernels, same draws); its step counter advances with the batch.  The
  * handles must outlive the batch and must not be stepped concurrently with

@@ -429,6 +429,7 @@ int ammsb_group_pairs(const int64_t* src, const int64_t* nbr, const uint8_t* y, 
   const int src_bits = bits_below(src_keys), nbr_bits = bits_below(nbr_keys);
   cudaError_t e = cudaSuccess;
   // one block also fills the pointers, a binary search each: 512 a few times
+  // (1,600 pairs 15 us; the general path's launches are some 40 us of host time)
   if (n_pairs <= kTile && n_src + n_nbr <= 16384) {
     k_group_tile<<<1, kThreads, 0, s>>>(g, src_bits, nbr_bits);
     e = cudaGetLastError();

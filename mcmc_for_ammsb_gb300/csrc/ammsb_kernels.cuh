@@ -8,11 +8,15 @@
 //   k_update_phi         update_phi (cc:269-313), fused with the noise draw
 //                        and the normalisation pi_i = phi_i / sum(phi_i)
 //                        into a staging buffer (Jacobi: pi is not touched)
-//   k_commit_beta        pi[nodes] = staged rows (cc:162-166) and the
-//                        per-edge update_beta gradient (cc:212-240) as a
-//                        segmented block reduction
+//   k_commit_star        pi[nodes] = staged rows (cc:162-166) and the
+//   k_commit_beta        per-edge update_beta gradient (cc:212-240) as a
+//                        segmented block reduction: for minibatches of one
+//                        source, and for any
 //   k_theta              sum of block partials + SGRLD theta step + beta
 //                        (cc:244-266), FP64
+// The draws (the first two) depend on the step alone, so a launch of either
+// makes those of eight iterations: one CTA per iteration's minibatch took 17 us
+// of each of a 100,000-node chain's 20 us iterations; eight at once 4.
 #pragma once
 #include "ammsb_device.cuh"
 #include "ammsb_gamma.cuh"
@@ -1219,7 +1223,9 @@ __global__ void __launch_bounds__(128) k_commit_beta_chains(const ChainArgs* __r
 // (kept in shared memory) and 1 / P_e, then the CTA's threads, one float pair
 // of k each, add the JC terms of the four w in that order.
 // Bound by latency, not bytes: one round of row loads and one warp sum per
-// JC*4 edges where k_commit_beta made a round per edge and warp.
+// JC*4 edges where k_commit_beta made a round per edge and warp.  4,096 edges of
+// K = 1024 BF16: 15.5 and 11.3 us (cold, alone), 13 and 5 us in an iteration; a
+// link stratum's few edges 5.2 us alone either way.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void store_pi4(float* dst, const float4& x) {
   *reinterpret_cast<float4*>(dst) = x;
@@ -1356,8 +1362,9 @@ __global__ void __launch_bounds__(128 * JC, JC == 1 ? 4 : 2) k_commit_star_chain
 //
 // A latency chain (partial loads, compensated sums, FP64 at 1/64 of the FP32
 // rate), so what does not need the partials is done beside the commit
-// (theta_pre_block) and two FMA chains and a division are left.  256 threads
-// rather than 1,024, so that the CTA fits an SM that still holds commit CTAs.
+// (theta_pre_block) and two FMA chains and a division are left: 6.6 and 3 us
+// behind the commit of a K = 1024 iteration.  256 threads rather than 1,024, so
+// that the CTA fits an SM that still holds commit CTAs.
 static __device__ __forceinline__ void theta_body(const Model& m, const Buffers& b, int star, int block,
                                                   const double* R_given = nullptr,
                                                   double* R_out = nullptr) {
@@ -1648,7 +1655,8 @@ __global__ void __launch_bounds__(256, VPL >= 8 ? 2 : VPL >= 4 ? 3 : 4) k_perple
 }
 
 // ---------------------------------------------------------------------------
-// init: phi ~ Gamma(1,1) (cc:66), row normalisation into pi (cc:75)
+// init: phi ~ Gamma(1,1) (cc:66), row normalisation into pi (cc:75).  Bound by
+// FP32 issue (ammsb_gamma.cuh): 30,000 x 256, 3.28 ms of FP64 draws and 0.2.
 // ---------------------------------------------------------------------------
 static __global__ void __launch_bounds__(256) k_init_phi(Model m, float* phi, const GammaTables* tables,
                                                          int32_t* err) {
@@ -1702,7 +1710,9 @@ __global__ void k_normalize_rows(Model m, const float* phi, PiT* pi) {
   }
 }
 
-// n rows of K elements (stride Kp) as packed floats.
+// n rows of K elements (stride Kp) as packed floats: a read-out of BF16 pi.
+// Bound by the copy to the host behind it (5M values 1,054 us when the host
+// widened them one by one, now 235).
 template <typename T>
 __global__ void __launch_bounds__(256) k_widen_rows(const T* __restrict__ rows, int K, int Kp, int64_t n,
                                                    float* __restrict__ out) {

@@ -76,6 +76,8 @@ struct PairLoad<__nv_bfloat16> {
 // shuffles each, some 150 cycles) then overlap.  As many as keep a lane at 32
 // floats of rows or fewer beside its w and A; rows of 32 floats a lane (K =
 // 1024 BF16) are bound by HBM with 16 warps per SM and take one at a time.
+// 100,000 x 256 BF16, 32 neighbours: 6.66 ms per 500 iterations with one row at
+// a time and a launch per kind, now 5.60; 400,000 x 1024 BF16 10.30 and 10.12 per 100.
 template <typename PiT, int VPL>
 __host__ __device__ constexpr int ring_rows() {
   constexpr int EPL = VPL * PiTraits<PiT>::kPerVec;
