@@ -1488,10 +1488,13 @@ static __global__ void __launch_bounds__(kThetaThreads) k_theta_chains(const Cha
 // Held-out perplexity (learner.cc:138-183, learner.h:100-139): LPN lanes per
 // held-out edge; running average per edge in FP32 as the reference; the log
 // sum in FP64.  A block takes PpxPlan::per_block consecutive edges.  A lane
-// group keeps its edges' averages a lane each, and the lanes then take the
-// logarithms side by side (one lane's FP64 logarithm costs its warp as much as
-// 32: with the lane that formed an average taking its logarithm, 86,246 pairs of
-// K = 1024 BF16 took 262 us, of which the rows are 53).  The block that finishes
+// group keeps its edges' averages a lane each; they meet in shared memory, and
+// a warp or two take the logarithms of products of four (an FP64 instruction
+// holds the SM's FP64 pipe 16 cycles however few of its lanes are on: 86,246
+// pairs of K = 1024 BF16, of which the rows are 53 us, took 262 us with a
+// logarithm per edge and warp, 82 with one per warp and 8 edges, 70 with
+// one per block and 64).  The product's roundings are within those of the sum
+// of four logarithms.  The block that finishes
 // last adds the blocks' partials, in a fixed order, so the result does not
 // depend on which it is; one thread adding a block's 256 values, and a second
 // launch for the partials, were 20 us of a small set's call.
@@ -1549,9 +1552,11 @@ __global__ void __launch_bounds__(256, VPL >= 8 ? 2 : VPL >= 4 ? 3 : 4) k_perple
   constexpr int EV = TR::kPerVec;
   constexpr int EPL = VPL * EV;
   constexpr int GPB = 256 / LPN, CH = ppx_chunk(LPN), J = ppx_edges(LPN);
+  constexpr int LOGS = CH / 4;  // threads that take logarithms, 16 to 64
   // beta in shared memory, not registers: 32 of them a lane left an SM with two
   // blocks instead of three (four measured no better)
   __shared__ __align__(16) float s_beta[LPN * EPL];
+  __shared__ __align__(16) float s_avg[CH];
   __shared__ double s_sum[256];
   __shared__ int s_last;
   const int tid = threadIdx.x, grp = tid / LPN, l = tid % LPN, lane = tid & 31;
@@ -1624,12 +1629,32 @@ __global__ void __launch_bounds__(256, VPL >= 8 ? 2 : VPL >= 4 ? 3 : 4) k_perple
         ppx[own] = mine;
       }
     }
-    const double term = log((double)mine) - comp;
-    const double tsum = sum + term;
-    comp = (tsum - sum) - term;
-    sum = tsum;
+    if (l < J) s_avg[grp * J + l] = mine;
+    __syncthreads();
+    if (tid < LOGS) {
+      // NaN for a negative average (of a caller's array), as its logarithm
+      // has it; a product of four floats neither overflows nor underflows
+      const float4 q = *reinterpret_cast<const float4*>(s_avg + 4 * tid);
+      double x = ((double)q.x * q.y) * ((double)q.z * q.w);
+      if (fminf(fminf(q.x, q.y), fminf(q.z, q.w)) < 0.f) x = nan("");
+      const double term = log(x) - comp;
+      const double tsum = sum + term;
+      comp = (tsum - sum) - term;
+      sum = tsum;
+    }
+    if (c0 + CH < e1) __syncthreads();  // s_avg is written again
   }
-  double total = block_sum_256(sum - comp, s_sum);
+  // the sum over the LOGS threads
+  double total = tid < LOGS ? sum - comp : 0.0;
+  if (tid < 64) {
+#pragma unroll
+    for (int o = (LOGS < 32 ? LOGS : 32) / 2; o > 0; o >>= 1) total += __shfl_down_sync(0xffffffffu, total, o);
+  }
+  if (LOGS > 32) {
+    if (tid == 32) s_sum[0] = total;
+    __syncthreads();
+    if (tid == 0) total += s_sum[0];
+  }
   if (tid == 0) {
     part[blockIdx.x] = total;
     __threadfence();

@@ -3,6 +3,7 @@ remainders, through ammsb_perplexity_noalloc on the caller's memory: each
 running average and the result against the plain expression in FP64, within
 the 1e-5 of test_gpu_parity."""
 import ctypes
+import math
 
 import pytest
 
@@ -42,3 +43,31 @@ def test_perplexity_at_block_remainders(native_lib, K, bf16, pairs):
         assert rc == 0
         assert float(((ppx.double() - p) / p).abs().max()) < 1e-5
         assert out.value == pytest.approx(float(-p.log().mean()), rel=1e-5, abs=1e-5)
+
+
+# the logarithms are taken of products of four averages: of the smallest ones
+# (a link between disjoint rows has p = 1e-30), and with a negative average in
+# the caller's array, whose logarithm is NaN
+@pytest.mark.parametrize("K", [2, 32, 128])
+def test_perplexity_of_the_smallest_averages(native_lib, K):
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    pairs = 100
+    pi = torch.zeros(2, -(-K // 4) * 4, device="cuda")
+    pi[0, 0], pi[1, 1] = 1.0, 1.0
+    beta = torch.full((K,), 0.5, device="cuda")
+    a = torch.zeros(pairs, dtype=torch.int32, device="cuda")
+    b, y = torch.ones_like(a), torch.ones(pairs, dtype=torch.uint8, device="cuda")
+    ppx = torch.zeros(pairs, device="cuda")
+
+    def call(count):
+        out = ctypes.c_double()
+        assert native_lib.ammsb_perplexity_noalloc(
+            pi.data_ptr(), _native.PI_F32, K, pi.shape[1], 2, beta.data_ptr(), 1e-7, a.data_ptr(), b.data_ptr(),
+            y.data_ptr(), pairs, ppx.data_ptr(), count, 0, ctypes.byref(out)) == 0
+        return out.value
+
+    tiny = float(torch.tensor(1e-30))
+    assert call(1) == pytest.approx(-math.log(tiny), rel=1e-12)
+    ppx[7] = ppx[10] = -1.0
+    assert math.isnan(call(2))
