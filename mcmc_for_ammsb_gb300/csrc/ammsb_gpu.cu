@@ -857,14 +857,13 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
   TRY(dev_alloc(h, &b.stage, (size_t)m.max_nodes * Kp));
   TRY(dev_alloc(h, &b.beta, (size_t)Kp));
   TRY(dev_alloc(h, &b.theta, 2 * (size_t)K));
-  // a minibatch round examines up to max(remaining, 4096) candidates while
-  // the dedup hash stays at most half full
-  m.slot_cand = std::max<int64_t>(o.mini_batch_size, 4096);
-  // ... and numbers the nodes of a general edge list (random-edge, several
-  // link sources) in the same table: at most max_nodes distinct vertices
+  // a minibatch round keeps the dedup hash at most half full; the nodes of a
+  // general edge list (random-edge, several link sources) are numbered in the
+  // same table: at most max_nodes distinct vertices
   int64_t hneed = std::max<int64_t>(8192, 2 * o.mini_batch_size);
   if (multi_src || rand_edge) hneed = std::max<int64_t>(hneed, 2 * (int64_t)m.max_nodes);
   const int hcap = next_pow2(hneed);
+  m.slot_cand = candidate_slots(o.mini_batch_size, hcap);
   b.hmask = (uint32_t)(hcap - 1);
   // the dedup hash lives in shared memory when it fits (up to 16Ki entries)
   if (hcap <= 16384 &&

@@ -20,6 +20,7 @@
 #pragma once
 #include "ammsb_device.cuh"
 #include "ammsb_gamma.cuh"
+#include "ammsb_plan.h"
 
 namespace ammsb {
 
@@ -72,7 +73,7 @@ struct Buffers {
   int32_t* eb;         // slot of second endpoint
   uint8_t* ey;         // y of each minibatch edge
   uint32_t* nbr;       // max_nodes x n_out: id | y << 31
-  int32_t* cand;       // mini_batch_size: candidate scratch
+  int32_t* cand;       // slot_cand: candidate scratch
   uint32_t* htab_key;  // minibatch dedup hash
   uint32_t* htab_idx;
   uint32_t hmask;
@@ -354,9 +355,8 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
     uint64_t t = 0;
     // the spec scans candidates t = 0, 1, ... until mb are kept, giving up
     // at `cap`; a round examines R >= need of them in parallel and keeps the
-    // first new valid ones, in order, up to mb.  R is what the rounds so far
-    // say `need` new ones take (need at first), plus an eighth and 64, while
-    // the dedup hash stays at most half full: a round's cost grows with R
+    // first new valid ones, in order, up to mb.  R (nonlink_round) follows the
+    // acceptance of the rounds so far: a round's cost grows with R
     // (a first round of up to 4,096 whatever the need took the 100k-node
     // workload's non-link minibatch from 16 to 44 us), and small populations
     // with many repeats still finish in two or three rounds.
@@ -369,9 +369,7 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
         err |= kErrMinibatchCap;
         break;
       }
-      const int64_t est = seen == 0 ? need : (kept > 0 ? (need * seen + kept - 1) / kept : half);
-      const int want = (int)min(est + est / 8 + 64, (int64_t)half);
-      const int R = (int)min((uint64_t)max(need, min(half - count, want)), cap - t);
+      const int R = (int)min((uint64_t)nonlink_round(need, count, half, seen, kept), cap - t);
       const int count0 = count;
       // pass A: validity and first-occurrence index per value; both of the
       // source's rows are in shared memory
@@ -480,7 +478,7 @@ static __device__ __forceinline__ void sample_minibatch_body(const Model& m, con
           err |= kErrMinibatchCap;
           break;
         }
-        const int R = (int)min((uint64_t)max(need, min(half - count, 4096)), cap - t);
+        const int R = (int)min((uint64_t)edge_round(need, count, half), cap - t);
         for (int c = tid; c < R; c += blockDim.x) {
           const int64_t q = (int64_t)uniform_below(rs.draw_u64(kTagMbCand, 0, step, t + (uint64_t)c),
                                                    (uint64_t)m.n_entries);

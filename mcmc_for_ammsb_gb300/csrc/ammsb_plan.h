@@ -1,0 +1,38 @@
+// ammsb_plan.h -- sizes that a kernel and the buffers it writes have to agree
+// on, in plain C++.
+#pragma once
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define AMMSB_HD __host__ __device__ __forceinline__
+#else
+#define AMMSB_HD inline
+#endif
+
+namespace ammsb {
+
+AMMSB_HD int64_t plan_min(int64_t a, int64_t b) { return a < b ? a : b; }
+AMMSB_HD int64_t plan_max(int64_t a, int64_t b) { return a > b ? a : b; }
+
+// Candidates that a round of a non-link minibatch examines, to find the `need`
+// of m that it lacks with `count` kept: what the rounds so far (`kept` of `seen`)
+// say they take (need at first), plus an eighth and 64, while the dedup hash
+// stays at most half full (`half` keys) -- and never fewer than need.
+AMMSB_HD int64_t nonlink_round(int64_t need, int64_t count, int64_t half, int64_t seen, int64_t kept) {
+  const int64_t est = seen == 0 ? need : (kept > 0 ? (need * seen + kept - 1) / kept : half);
+  const int64_t want = plan_min(est + est / 8 + 64, half);
+  return plan_max(need, plan_min(half - count, want));
+}
+
+// ... and a round of a random-edge one.
+constexpr int64_t kEdgeRound = 4096;
+AMMSB_HD int64_t edge_round(int64_t need, int64_t count, int64_t half) {
+  return plan_max(need, plan_min(half - count, kEdgeRound));
+}
+
+// Candidate words of one iteration's minibatch: the most that either round
+// writes, for minibatches of m with a hash of hcap slots (a round is need <= m,
+// or at most half the hash).
+AMMSB_HD int64_t candidate_slots(int64_t m, int64_t hcap) { return plan_max(m, hcap / 2); }
+
+}  // namespace ammsb
