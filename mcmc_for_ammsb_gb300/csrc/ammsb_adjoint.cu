@@ -192,12 +192,13 @@ __global__ void __launch_bounds__(kThreads) k_ll_forward(Args g) {
   for (int64_t qb = q0 + grp; qb < q1; qb += NG * U) {
     T x[U][EPL], D[U];
     int32_t nb[U];
-    bool y[U];
+    bool on[U], y[U];  // on: not past the source's pairs
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t q = qb + (int64_t)u * NG;
-      nb[u] = q < q1 ? g.pair_nbr[q] : -2;  // -2: past the source's pairs
-      y[u] = q < q1 && g.pair_y[q] != 0;
+      on[u] = q < q1;
+      nb[u] = on[u] ? g.pair_nbr[q] : -1;
+      y[u] = on[u] && g.pair_y[q] != 0;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(kThreads) k_ll_forward(Args g) {
       for (int u = 0; u < U; ++u) D[u] += __shfl_xor_sync(mask, D[u], o);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (nb[u] == -2) continue;
+      if (!on[u]) continue;
       const int64_t q = qb + (int64_t)u * NG;
       if (nb[u] < 0 || nb[u] >= g.n_nbr) {
         if (l == 0) {

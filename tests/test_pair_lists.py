@@ -1,0 +1,53 @@
+"""Pair lists as callers may pass them to the edge log-likelihood."""
+import ctypes
+
+import pytest
+
+from mcmc_for_ammsb_gb300 import _native
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def gpu(native_lib):
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+
+
+# every index outside the rows is skipped and flagged, whatever its value: the
+# loss is that of the other pairs (their sum in another order, hence the
+# tolerances of test_adjoint), and no word of the workspace is read unwritten
+@pytest.mark.parametrize("bad", [-1, -2, -3, -2**31, 90, 2**31 - 1])
+@pytest.mark.parametrize("K,dtype,tol", [(16, torch.float64, 1e-11), (17, torch.float32, 1e-4),
+                                         (256, torch.float32, 1e-4)])
+def test_any_index_out_of_range_is_flagged(native_lib, bad, K, dtype, tol):
+    n_src, n_nbr, per = 5, 90, 40
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    phi, pi = (torch.rand(n, K, device="cuda", generator=gen, dtype=dtype) + 0.1 for n in (n_src, n_nbr))
+    pi /= pi.sum(1, keepdim=True)
+    theta = torch.rand(K, 2, device="cuda", generator=gen, dtype=dtype) + 0.5
+    nbr = torch.randint(n_nbr, (n_src * per,), device="cuda", generator=gen, dtype=torch.int32)
+    y = (torch.rand(n_src * per, device="cuda", generator=gen) < 0.3).to(torch.uint8)
+    code = _native.REAL_F64 if dtype == torch.float64 else _native.REAL_F32
+
+    def forward(nbr, y, per):
+        ptr = torch.arange(n_src + 1, device="cuda") * per
+        size = native_lib.ammsb_edge_loglik_workspace_size(code, K, n_src, len(nbr))
+        ws = torch.full((size // phi.element_size(),), float("nan"), device="cuda", dtype=dtype)
+        loss, flags = torch.zeros((), device="cuda", dtype=dtype), ctypes.c_int32()
+        p = [ctypes.c_void_p(t.data_ptr()) for t in (phi, pi, theta, ptr, nbr, y, loss, ws)]
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert native_lib.ammsb_edge_loglik_forward(code, K, p[0], K, p[1], K, n_nbr, p[2], 1e-7, p[3], n_src,
+                                                    p[4], p[5], len(nbr), p[6], p[7], stream) == 0
+        assert native_lib.ammsb_edge_loglik_status(p[7], stream, ctypes.byref(flags)) == 0
+        return float(loss), flags.value
+
+    marked = nbr.clone().view(n_src, per)
+    marked[:, [0, 7, per - 1]] = bad
+    keep = torch.ones(per, dtype=torch.bool, device="cuda")
+    keep[[0, 7, per - 1]] = False
+    want, clean = forward(nbr.view(n_src, per)[:, keep].reshape(-1), y.view(n_src, per)[:, keep].reshape(-1), per - 3)
+    got, flags = forward(marked.reshape(-1), y, per)
+    assert clean == 0 and flags == 1
+    assert got == pytest.approx(want, rel=tol)
