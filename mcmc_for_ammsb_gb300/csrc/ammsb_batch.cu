@@ -188,9 +188,10 @@ thread_local std::string g_batch_create_error;
     }                                                                  \
   } while (0)
 
-// `pdl`: the theta step of the iteration before is the kernel ahead in the
-// stream and this iteration's draws are complete.
-cudaError_t launch_update_chains(ammsb_batch* bt, int p, bool pdl) {
+// The update in two parts, as for one chain.  `pdl`: the theta step of the
+// iteration before is the kernel ahead in the stream and this iteration's draws
+// were complete before that step ended.
+cudaError_t launch_rows_chains(ammsb_batch* bt, int p, bool pdl) {
   // the update_phi groups touch disjoint chains: they run concurrently
   // (parallel branches of the captured graph), then join before the commits.
   // The first group, the commit and the theta step start early as for one
@@ -219,6 +220,9 @@ cudaError_t launch_update_chains(ammsb_batch* bt, int p, bool pdl) {
                                    : commit_chains<float>(g, bt->d_all, p, bt->stream, early, false);
     if (e != cudaSuccess) return e;
   }
+  return cudaSuccess;
+}
+cudaError_t launch_theta_chains(ammsb_batch* bt, int p) {
   return launch_k(k_theta_chains, bt->theta.grid(), kThetaThreads, 0, bt->stream, (bt->pdl & kPdlTheta) != 0,
                   bt->d_all, bt->theta.d, p);
 }
@@ -233,9 +237,12 @@ cudaError_t launch_sampling_chains(ammsb_batch* bt, int s0, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_updates_chains(ammsb_batch* bt, int s, int count, bool first_pdl = false) {
+cudaError_t launch_updates_chains(ammsb_batch* bt, int s, int count) {
   cudaError_t e = cudaSuccess;
-  for (int i = 0; i < count && e == cudaSuccess; ++i) e = launch_update_chains(bt, s + i, i > 0 || first_pdl);
+  for (int i = 0; i < count && e == cudaSuccess; ++i) {
+    e = launch_rows_chains(bt, s + i, i > 0);
+    if (e == cudaSuccess) e = launch_theta_chains(bt, s + i);
+  }
   return e;
 }
 
@@ -249,12 +256,16 @@ cudaError_t fork_draws_chains(ammsb_batch* bt, int blk) {
   return cudaEventRecord(bt->ev_join, bt->side);
 }
 
-cudaError_t launch_block_chains(ammsb_batch* bt, int blk, bool first_pdl = false) {
-  cudaError_t e = fork_draws_chains(bt, 1 - blk);
-  if (e != cudaSuccess) return e;
-  if ((e = launch_updates_chains(bt, blk * bt->block, bt->block, first_pdl)) != cudaSuccess)
-    return e;
-  return cudaStreamWaitEvent(bt->stream, bt->ev_join, 0);
+cudaError_t launch_block_chains(ammsb_batch* bt, int blk, bool first_early, bool early_follows) {
+  struct Launches {
+    ammsb_batch* bt;
+    int blk;
+    cudaError_t fork() { return fork_draws_chains(bt, 1 - blk); }
+    cudaError_t rows(int i, bool early) { return launch_rows_chains(bt, blk * bt->block + i, early); }
+    cudaError_t theta(int i) { return launch_theta_chains(bt, blk * bt->block + i); }
+    cudaError_t join() { return cudaStreamWaitEvent(bt->stream, bt->ev_join, 0); }
+  };
+  return launch_block_order(Launches{bt, blk}, bt->block, first_early, early_follows);
 }
 
 // Launches `work` as a captured graph kept in g.
@@ -542,8 +553,8 @@ int ammsb_batch_step(ammsb_batch* bt, int64_t n_iters) {
       const bool both = left >= 2 * (int64_t)D;
       n = both ? 2 * D : D;
       rc = launch_graph(bt, both ? bt->graphL[blk] : bt->graphB[blk], [&] {
-        cudaError_t e = launch_block_chains(bt, blk);
-        return e == cudaSuccess && both ? launch_block_chains(bt, 1 - blk, true) : e;
+        cudaError_t e = launch_block_chains(bt, blk, false, both);
+        return e == cudaSuccess && both ? launch_block_chains(bt, 1 - blk, true, false) : e;
       });
       drawn += (uint32_t)n;
     } else {

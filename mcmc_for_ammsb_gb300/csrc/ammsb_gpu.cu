@@ -83,7 +83,7 @@ cudaError_t launch_phi_t(ammsb_handle* h, const Buffers& b, bool pdl) {
 }
 
 // `pdl`: the launch directly follows k_theta in the stream and its draws
-// were complete before that kernel started; it then starts as a programmatic
+// were complete before that kernel's wait ended; it then starts as a programmatic
 // dependent launch, which overlaps its first row copies and node prologues
 // with the theta step.
 template <typename PiT, int VPL, int STAGES, bool FULL>
@@ -233,25 +233,25 @@ inline cudaError_t mark(cudaEvent_t ev, cudaStream_t s) {
                                                                              : cudaEventRecordDefault);
 }
 
-// The iteration's kernels in order; `b` carries the fed-noise pointers when
-// called from ammsb_step_fed (which skips the two sampling kernels).  With
-// `ev`, events are recorded after update_phi, the commit and theta, and
-// every kernel waits for the one ahead to finish; without, the commit and
-// theta step start as programmatic dependent launches (cfg.pdl).  `pdl`:
+// The iteration's kernels in order, in two parts; `b` carries the fed-noise
+// pointers when called from ammsb_step_fed (which skips the two sampling
+// kernels).  With `ev`, events are recorded after update_phi, the commit and
+// theta, and every kernel waits for the one ahead to finish; without, the commit
+// and theta step start as programmatic dependent launches (cfg.pdl).  `pdl`:
 // the previous iteration's theta step is the kernel ahead in the stream and
-// this iteration's draws are complete (update_phi may then start early).
-// `star`: the minibatch is one.
-cudaError_t launch_update_phase(ammsb_handle* h, const Buffers& b, bool star, const cudaEvent_t* ev = nullptr,
-                                bool pdl = false) {
-  const int early = ev ? 0 : h->cfg.pdl;
+// this iteration's draws were complete before that step ended (update_phi may
+// then start early).  `star`: the minibatch is one.
+cudaError_t launch_rows(ammsb_handle* h, const Buffers& b, bool star, const cudaEvent_t* ev, bool pdl) {
   cudaError_t e = (h->opt.pi_dtype == AMMSB_PI_BF16) ? launch_phi<__nv_bfloat16>(h, b, pdl)
                                                       : launch_phi<float>(h, b, pdl);
   if (e != cudaSuccess || (e = mark(ev ? ev[0] : nullptr, h->stream)) != cudaSuccess) return e;
-  e = launch_commits(h, b, star, early & kPdlCommit);
-  if (e != cudaSuccess || (e = mark(ev ? ev[1] : nullptr, h->stream)) != cudaSuccess) return e;
-  e = launch_k(k_theta, (h->m.K + 31) / 32, kThetaThreads, 0, h->stream, early & kPdlTheta, h->m, b, (int)star);
-  if (e != cudaSuccess) return e;
-  return mark(ev ? ev[2] : nullptr, h->stream);
+  e = launch_commits(h, b, star, !ev && (h->cfg.pdl & kPdlCommit));
+  return e != cudaSuccess ? e : mark(ev ? ev[1] : nullptr, h->stream);
+}
+cudaError_t launch_theta(ammsb_handle* h, const Buffers& b, bool star, const cudaEvent_t* ev) {
+  cudaError_t e = launch_k(k_theta, (h->m.K + 31) / 32, kThetaThreads, 0, h->stream, !ev && (h->cfg.pdl & kPdlTheta),
+                           h->m, b, (int)star);
+  return e != cudaSuccess ? e : mark(ev ? ev[2] : nullptr, h->stream);
 }
 
 // Buffer set `slot` of the handle's ring.
@@ -271,19 +271,24 @@ cudaError_t launch_sampling_phase(ammsb_handle* h, int s0, int count, cudaStream
   return mark(ev ? ev[2] : nullptr, s);
 }
 
-// `count` updates from ring slot s on; `first_pdl`: the theta step of the
-// iteration before is the kernel ahead of the first one in the stream.  With
-// `timed`, each records its buffer set's events.
-cudaError_t launch_updates(ammsb_handle* h, int s, int count, bool timed, bool first_pdl = false) {
+// The update of ring slot s in its two parts; with `timed`, it records its
+// buffer set's events.
+cudaError_t launch_slot_rows(ammsb_handle* h, int s, bool timed, bool pdl) {
+  const cudaEvent_t* ev = timed ? h->ev_upd[s] : nullptr;
+  cudaError_t e = mark(ev ? ev[0] : nullptr, h->stream);
+  return e != cudaSuccess ? e : launch_rows(h, ring_set(h, s), h->star, ev ? ev + 1 : nullptr, pdl && !ev);
+}
+cudaError_t launch_slot_theta(ammsb_handle* h, int s, bool timed) {
+  return launch_theta(h, ring_set(h, s), h->star, timed ? h->ev_upd[s] + 1 : nullptr);
+}
+
+// `count` updates from ring slot s on, inside a block: an update after another
+// follows its theta step directly (its draws were joined before this launch).
+cudaError_t launch_updates(ammsb_handle* h, int s, int count, bool timed) {
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < count && e == cudaSuccess; ++i) {
-    const cudaEvent_t* ev = timed ? h->ev_upd[(s + i) % h->m.ring] : nullptr;
-    e = mark(ev ? ev[0] : nullptr, h->stream);
-    // an update after another follows its theta step directly (its draws
-    // were joined before this launch)
-    if (e == cudaSuccess)
-      e = launch_update_phase(h, ring_set(h, (s + i) % h->m.ring), h->star, ev ? ev + 1 : nullptr,
-                              (i > 0 || first_pdl) && !ev);
+    e = launch_slot_rows(h, s + i, timed, i > 0);
+    if (e == cudaSuccess) e = launch_slot_theta(h, s + i, timed);
   }
   return e;
 }
@@ -310,11 +315,17 @@ cudaError_t join_draws(ammsb_handle* h) { return cudaStreamWaitEvent(h->stream, 
 // which eight iterations side by side pay once; with a launch per iteration
 // the draws were the longer branch of every small chain and of every
 // link-stratum iteration.
-cudaError_t launch_block(ammsb_handle* h, int blk, bool timed, bool first_pdl = false) {
-  cudaError_t e = fork_draws(h, 1 - blk, timed);
-  if (e != cudaSuccess) return e;
-  if ((e = launch_updates(h, blk * h->block, h->block, timed, first_pdl)) != cudaSuccess) return e;
-  return join_draws(h);
+cudaError_t launch_block(ammsb_handle* h, int blk, bool timed, bool first_early = false, bool early_follows = false) {
+  struct Launches {
+    ammsb_handle* h;
+    int blk;
+    bool timed;
+    cudaError_t fork() { return fork_draws(h, 1 - blk, timed); }
+    cudaError_t rows(int i, bool early) { return launch_slot_rows(h, blk * h->block + i, timed, early); }
+    cudaError_t theta(int i) { return launch_slot_theta(h, blk * h->block + i, timed); }
+    cudaError_t join() { return join_draws(h); }
+  };
+  return launch_block_order(Launches{h, blk, timed}, h->block, first_early, early_follows);
 }
 
 // One iteration at ring slot s in run()'s loop order on the handle's
@@ -1095,7 +1106,7 @@ int ammsb_step(ammsb_handle* h, int64_t n_iters) {
       if (timed && (rc = take_phase_events(h, s, D, (1 - blk) * D))) return rc;
       if (both)
         rc = launch(h->graphL[blk], [&] {
-          cudaError_t e = launch_block(h, blk, false);
+          cudaError_t e = launch_block(h, blk, false, false, true);
           return e != cudaSuccess ? e : launch_block(h, 1 - blk, false, true);
         });
       else
@@ -1196,7 +1207,8 @@ int ammsb_step_fed(ammsb_handle* h, uint32_t step, int32_t n_edges, const int32_
   bool star = n_edges > 0 && n_nodes == n_edges + 1;
   for (int32_t e = 0; e < n_edges && star; ++e)
     star = edge_slot_a[e] == 0 && edge_slot_b[e] == e + 1 && !edge_y[e] == !edge_y[0];
-  CK(launch_update_phase(h, fb, star));
+  CK(launch_rows(h, fb, star, nullptr, false));
+  CK(launch_theta(h, fb, star, nullptr));
   h->last = h->slot;
   return check_device_err(h);
 }

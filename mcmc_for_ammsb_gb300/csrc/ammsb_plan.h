@@ -1,5 +1,5 @@
 // ammsb_plan.h -- sizes that a kernel and the buffers it writes have to agree
-// on, in plain C++.
+// on, and the order of a block's launches, in plain C++.
 #pragma once
 #include <stdint.h>
 
@@ -34,5 +34,26 @@ AMMSB_HD int64_t edge_round(int64_t need, int64_t count, int64_t half) {
 // writes, for minibatches of m with a hash of hcap slots (a round is need <= m,
 // or at most half the hash).
 AMMSB_HD int64_t candidate_slots(int64_t m, int64_t hcap) { return plan_max(m, hcap / 2); }
+
+// The launches of a block of `count` iterations, with the other block's draws
+// forked alongside: per iteration the rows (update_phi and the commit, update_phi
+// early unless the launch ahead is no theta step), then the theta step.
+// `early_follows`: the other block's first update is launched next and starts
+// early.  Its dependence on the draws is then no more than on the theta step
+// (a programmatic launch that follows a joined stream takes a programmatic edge
+// from that stream's kernel too, as the edges of such a capture say), so the
+// draws are joined ahead of the block's last theta step, whose own wait they end
+// before; else behind it, where the theta step does not wait for them.
+template <class Launches>
+auto launch_block_order(Launches&& l, int count, bool first_early, bool early_follows) {
+  auto e = l.fork();
+  for (int i = 0; !e && i < count; ++i) {
+    e = l.rows(i, i > 0 || first_early);
+    if (!e && early_follows && i == count - 1) e = l.join();
+    if (!e) e = l.theta(i);
+  }
+  if (!e && !early_follows) e = l.join();
+  return e;
+}
 
 }  // namespace ammsb

@@ -1,6 +1,6 @@
-"""Sizes that kernels and their buffers agree on (csrc/ammsb_plan.h), compiled
-for the host: no round of a minibatch examines more candidates than an
-iteration's scratch area holds."""
+"""What csrc/ammsb_plan.h holds, compiled for the host: no round of a minibatch
+examines more candidates than an iteration's scratch area holds, and an update
+that starts early finds its draws joined ahead of the theta step before it."""
 import os
 import subprocess
 
@@ -38,9 +38,47 @@ int main() {
 """
 
 
-def test_a_round_fits_its_scratch_area(tmp_path):
-    src, exe = tmp_path / "rounds.cc", str(tmp_path / "rounds")
-    src.write_text(ROUNDS)
+ORDER = r"""
+#include <cstdio>
+#include <initializer_list>
+#include <string>
+#include "ammsb_plan.h"
+struct Recorder {  // F fork, J join, R and r rows (r early), T theta, X the launch that fails
+  std::string* log;
+  int fail;
+  int put(char c) { return log->push_back((int)log->size() == fail ? 'X' : c), (int)log->size() - 1 == fail; }
+  int fork() { return put('F'); }
+  int rows(int, bool early) { return put(early ? 'r' : 'R'); }
+  int theta(int) { return put('T'); }
+  int join() { return put('J'); }
+};
+int main() {
+  for (int count : {1, 3}) {
+    std::string pair, failed;
+    ammsb::launch_block_order(Recorder{&pair, -1}, count, false, true);
+    ammsb::launch_block_order(Recorder{&pair, -1}, count, true, false);
+    const int e = ammsb::launch_block_order(Recorder{&failed, count + 1}, count, false, false);
+    std::printf("%s %s %d\n", pair.c_str(), failed.c_str(), e);
+  }
+}
+"""
+
+
+def compiled_output(tmp_path, program):
+    src, exe = tmp_path / "program.cc", str(tmp_path / "program")
+    src.write_text(program)
     subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-I", build.CSRC, str(src), "-o", exe], check=True)
     r = subprocess.run([exe], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+    return r.stdout
+
+
+def test_a_round_fits_its_scratch_area(tmp_path):
+    assert "rounds checked" in compiled_output(tmp_path, ROUNDS)
+
+
+def test_draws_are_joined_before_the_theta_step_ahead(tmp_path):
+    one, three = compiled_output(tmp_path, ORDER).splitlines()
+    # a block whose end the next block's first update (r) overlaps, and that block
+    assert one == "FRJT" "FrTJ" " FRX 1"
+    assert three == "FRTrTrJT" "FrTrTrTJ" " FRTrX 1"
