@@ -1471,8 +1471,11 @@ static __global__ void __launch_bounds__(kThetaThreads) k_theta(Model m, Buffers
 static __global__ void __launch_bounds__(kThetaThreads) k_beta_sums(Model m, Buffers b, double* R_out) {
   theta_body(m, b, 0, blockIdx.x, nullptr, R_out);
 }
-// the theta step from given sums
+// the theta step from given sums: a call of its own, so its other parts are
+// formed here too, from the theta and beta of now (not those of the commit)
 static __global__ void __launch_bounds__(kThetaThreads) k_theta_given(Model m, Buffers b, const double* R) {
+  theta_pre_block(m, b, blockIdx.x);
+  __syncthreads();
   theta_body(m, b, 0, blockIdx.x, R, nullptr);
 }
 static __global__ void __launch_bounds__(kThetaThreads) k_theta_chains(const ChainArgs* __restrict__ c,
