@@ -139,6 +139,12 @@ def _group_cuda(src, nbr, y, n_src, n_nbr, src_keys, nbr_keys, ws):
 
 
 def _as_lists(src, nbr, y):
+    # the kernels get bare pointers: what they read is checked here
+    if not src.device == nbr.device == y.device:
+        raise RuntimeError("pair lists on different devices: %s, %s, %s"
+                           % (src.device, nbr.device, y.device))
+    if src.dim() > 1 or nbr.dim() > 1:
+        raise RuntimeError("pair lists must be 1-D")
     return (src.to(torch.int64).contiguous(), nbr.to(torch.int64).contiguous(),
             y.to(torch.uint8).contiguous())
 

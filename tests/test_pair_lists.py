@@ -6,22 +6,58 @@ import pytest
 from mcmc_for_ammsb_gb300 import _native
 
 torch = pytest.importorskip("torch")
-pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module", autouse=True)
+@pytest.fixture
 def gpu(native_lib):
     if not torch.cuda.is_available():
         pytest.skip("no GPU")
 
 
+def lists(device="cpu"):
+    return [torch.tensor(x, device=device) for x in ([0, 1, 1], [2, 0, 1], [1, 0, 0])]
+
+
+# no pointer of another device, and no list of other than one dimension, gets
+# as far as a kernel (the meta device stands for any other one)
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_lists_of_another_device_are_refused(which):
+    from mcmc_for_ammsb_gb300.autograd import _as_lists
+    mixed = lists()
+    mixed[which] = mixed[which].to("meta")
+    with pytest.raises(RuntimeError):
+        _as_lists(*mixed)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_mixed_lists_are_refused(gpu, which):
+    from mcmc_for_ammsb_gb300.autograd import edge_log_likelihood, group_pairs
+    phi, theta = torch.ones(3, 4, device="cuda"), torch.ones(4, 2, device="cuda")
+    mixed = lists("cuda")
+    mixed[which] = mixed[which].cpu()
+    with pytest.raises(RuntimeError):
+        edge_log_likelihood(phi, phi / 4, theta, *mixed, 1e-7)
+    if which:  # lists led by a CPU one are grouped by torch
+        with pytest.raises(RuntimeError):
+            group_pairs(*mixed, 3, 3)
+    flat = lists("cuda")
+    if which < 2:
+        flat[which] = flat[which][:, None]
+        with pytest.raises(RuntimeError):
+            group_pairs(*flat, 3, 3)
+        with pytest.raises(RuntimeError):
+            edge_log_likelihood(phi, phi / 4, theta, *flat, 1e-7)
+
+
 # every index outside the rows is skipped and flagged, whatever its value: the
 # loss is that of the other pairs (their sum in another order, hence the
 # tolerances of test_adjoint), and no word of the workspace is read unwritten
+@pytest.mark.gpu
 @pytest.mark.parametrize("bad", [-1, -2, -3, -2**31, 90, 2**31 - 1])
 @pytest.mark.parametrize("K,dtype,tol", [(16, torch.float64, 1e-11), (17, torch.float32, 1e-4),
                                          (256, torch.float32, 1e-4)])
-def test_any_index_out_of_range_is_flagged(native_lib, bad, K, dtype, tol):
+def test_any_index_out_of_range_is_flagged(gpu, native_lib, bad, K, dtype, tol):
     n_src, n_nbr, per = 5, 90, 40
     gen = torch.Generator(device="cuda").manual_seed(K)
     phi, pi = (torch.rand(n, K, device="cuda", generator=gen, dtype=dtype) + 0.1 for n in (n_src, n_nbr))
