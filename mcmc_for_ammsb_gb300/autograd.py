@@ -203,6 +203,10 @@ def edge_log_likelihood(phi_src, pi_nbr, theta, src, nbr, y, epsilon):
         raise IndexError("pair lists of different lengths")
     if src.shape[0] and (n_src == 0 or n_nbr == 0):
         raise IndexError("pair indices out of range")
+    if nbr.shape[0] > src.shape[0] > 0:  # its tail is in no pair, but has to be in range
+        tail = nbr[src.shape[0]:]
+        if int(tail.min()) < 0 or int(tail.max()) >= n_nbr:
+            raise IndexError("pair indices out of range")
     # an index out of range marks its pair, which the forward flags: the
     # status it reads anyway raises the IndexError
     groups = _group_cuda(src, nbr, y, n_src, n_nbr, n_src, n_nbr, _pair_workspace(src))

@@ -87,3 +87,19 @@ def test_any_index_out_of_range_is_flagged(gpu, native_lib, bad, K, dtype, tol):
     got, flags = forward(marked.reshape(-1), y, per)
     assert clean == 0 and flags == 1
     assert got == pytest.approx(want, rel=tol)
+
+
+# a neighbour list longer than the source list: its tail takes no part, but
+# has to be in range
+@pytest.mark.gpu
+def test_a_longer_neighbour_list_is_checked_to_its_end(gpu):
+    from mcmc_for_ammsb_gb300.autograd import edge_log_likelihood
+    phi, theta = torch.ones(3, 4, device="cuda"), torch.ones(4, 2, device="cuda")
+    src, nbr, y = lists("cuda")
+    want = edge_log_likelihood(phi, phi / 4, theta, src, nbr, y, 1e-7)
+    longer = torch.cat([nbr, nbr])
+    assert torch.equal(edge_log_likelihood(phi, phi / 4, theta, src, longer, y, 1e-7), want)
+    for bad in (-1, 3):
+        longer[-1] = bad
+        with pytest.raises(IndexError):
+            edge_log_likelihood(phi, phi / 4, theta, src, longer, y, 1e-7)
