@@ -376,8 +376,8 @@ int ammsb_edge_loglik_status(const void *workspace, void *stream,
  * nbr_ptr its row pointers (n_nbr + 1).  Device arrays.  src_keys >= n_src and
  * nbr_keys >= n_nbr bound the indices (ammsb_check_pairs gives the largest);
  * pairs at or above n_src or n_nbr come last and under no row.  A pair with an
- * index below zero or past its bound is put under some row with pair_nbr = -1,
- * which the forward skips and flags.  Kernels are queued on `stream`; workspace
+ * index below zero, past its bound or past 2^31 - 1 is put under some row with
+ * pair_nbr = -1, which the forward skips and flags.  Kernels are queued on `stream`; workspace
  * is caller-owned device memory of ammsb_group_pairs_workspace_size bytes. */
 size_t ammsb_group_pairs_workspace_size(int64_t n_pairs);
 int ammsb_group_pairs(const int64_t *src, const int64_t *nbr,

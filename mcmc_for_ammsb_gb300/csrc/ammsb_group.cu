@@ -27,6 +27,7 @@ constexpr int kThreads = 512, kWarps = kThreads / 32;
 constexpr int kRounds = 4;                  // pairs per thread
 constexpr int kTile = kThreads * kRounds;   // pairs per block
 constexpr int kMaxDigit = 9, kMaxBins = 1 << kMaxDigit;
+constexpr int64_t kNamed = 1ll << 31;       // indices that an int32 holds
 constexpr int kCheckWords = 4;  // max and ~min of the sources, of the neighbours
 
 __device__ __forceinline__ uint32_t lanes_below() {
@@ -418,8 +419,11 @@ int ammsb_group_pairs(const int64_t* src, const int64_t* nbr, const uint8_t* y, 
                       void* stream) {
   const char* fn = "ammsb_group_pairs";
   if (n_pairs < 0 || n_pairs > INT32_MAX || n_src < 0 || n_nbr < 0 || src_keys < n_src || nbr_keys < n_nbr ||
-      src_keys > (1ll << 31) || nbr_keys > (1ll << 31) || (n_pairs > 0 && (src_keys < 1 || nbr_keys < 1)))
+      (n_pairs > 0 && (src_keys < 1 || nbr_keys < 1)))
     return fail(fn, "sizes out of range", AMMSB_E_ARG);
+  // there may be more rows than the int32 arrays can name: pairs of those are marked
+  src_keys = src_keys < kNamed ? src_keys : kNamed;
+  nbr_keys = nbr_keys < kNamed ? nbr_keys : kNamed;
   if (!src_ptr || !nbr_ptr || !workspace ||
       (n_pairs > 0 && (!src || !nbr || !y || !pair_nbr || !pair_y || !pair_src || !nbr_pairs)))
     return fail(fn, "null argument", AMMSB_E_ARG);

@@ -103,3 +103,20 @@ def test_a_longer_neighbour_list_is_checked_to_its_end(gpu):
         longer[-1] = bad
         with pytest.raises(IndexError):
             edge_log_likelihood(phi, phi / 4, theta, src, longer, y, 1e-7)
+
+
+# more rows than an int32 can name, of which the pairs name the first and the
+# last that it can: the pointers are those of the sorted list (exact)
+@pytest.mark.gpu
+def test_more_rows_than_an_int32_names(gpu):
+    from mcmc_for_ammsb_gb300.autograd import group_pairs
+    n_src, last = 2**31 + 5, 2**31 - 1
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs 40 GB of device memory")
+    src = torch.tensor([last, 0, last, 7], device="cuda")
+    src_ptr, pair_nbr, _, pair_src, _, _ = group_pairs(src, torch.tensor([2, 0, 1, 1], device="cuda"),
+                                                       torch.zeros_like(src), n_src, 3)
+    assert pair_src.tolist() == [0, 7, last, last] and pair_nbr.tolist() == [0, 1, 2, 1]
+    assert src_ptr.shape[0] == n_src + 1
+    for at, want in ((0, 0), (1, 1), (7, 1), (8, 2), (last, 2), (last + 1, 4), (n_src, 4)):
+        assert int(src_ptr[at]) == want, at
