@@ -122,6 +122,14 @@ struct Args {
   __host__ __device__ T* at(size_t off) const { return reinterpret_cast<T*>(ws + off); }
 };
 
+// A grid of any number of blocks: in rows of 2^30 where they are more than its
+// x dimension holds (kernels return from blocks past their rows).
+constexpr int64_t kGridRow = 1ll << 30;
+dim3 grid_of(int64_t blocks) {
+  return blocks <= kGridRow ? dim3((unsigned)blocks) : dim3((unsigned)kGridRow, (unsigned)((blocks - 1) / kGridRow + 1));
+}
+__device__ __forceinline__ int64_t block_of_grid() { return blockIdx.x + (int64_t)blockIdx.y * kGridRow; }
+
 // VEC elements of a row as one load or store (VEC * sizeof(T) bytes, aligned).
 template <typename T, int VEC>
 struct alignas(sizeof(T) * VEC) Vec {
@@ -162,7 +170,8 @@ __global__ void __launch_bounds__(kThreads) k_ll_forward(Args g) {
   __shared__ T s_B[NG], s_ll[kThreads / 32];
   const int tid = threadIdx.x, l = tid % LPR, grp = tid / LPR;
   const uint32_t mask = lane_group_mask<LPR>();
-  const int64_t a = blockIdx.x;
+  const int64_t a = block_of_grid();
+  if (a >= g.n_src) return;
   const int K = g.K, nvec = K / VEC;
   const T eps = (T)g.eps;
   const T* pin = static_cast<const T*>(g.pin);
@@ -359,7 +368,7 @@ __global__ void __launch_bounds__(kThreads) k_ll_backward_nbr(Args g) {
   constexpr int EPL = VPL * VEC, U = rows_ahead<EPL>();
   const int l = threadIdx.x % LPR;
   const uint32_t mask = lane_group_mask<LPR>();
-  const int64_t b = ((int64_t)blockIdx.x * kThreads + threadIdx.x) / LPR;
+  const int64_t b = (block_of_grid() * kThreads + threadIdx.x) / LPR;
   if (b >= g.n_nbr) return;
   const int K = g.K, nvec = K / VEC;
   const T* phi = static_cast<const T*>(g.phi);
@@ -428,9 +437,9 @@ unsigned blocks_of(int64_t n, int64_t per) { return (unsigned)((n + per - 1) / p
 template <typename T, int VEC, int LPR, int VPL>
 cudaError_t launch_rows(bool fwd, const Args& g, cudaStream_t s) {
   if (fwd) {
-    if (g.n_src) k_ll_forward<T, VEC, LPR, VPL><<<(unsigned)g.n_src, kThreads, 0, s>>>(g);
+    if (g.n_src) k_ll_forward<T, VEC, LPR, VPL><<<grid_of(g.n_src), kThreads, 0, s>>>(g);
   } else if (g.n_nbr) {
-    k_ll_backward_nbr<T, VEC, LPR, VPL><<<blocks_of(g.n_nbr, kThreads / LPR), kThreads, 0, s>>>(g);
+    k_ll_backward_nbr<T, VEC, LPR, VPL><<<grid_of((g.n_nbr - 1) / (kThreads / LPR) + 1), kThreads, 0, s>>>(g);
   }
   return cudaGetLastError();
 }

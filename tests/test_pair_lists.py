@@ -120,3 +120,28 @@ def test_more_rows_than_an_int32_names(gpu):
     assert src_ptr.shape[0] == n_src + 1
     for at, want in ((0, 0), (1, 1), (7, 1), (8, 2), (last, 2), (last + 1, 4), (n_src, 4)):
         assert int(src_ptr[at]) == want, at
+
+
+# so many source rows that the forward's blocks do not fit one grid dimension:
+# K = 1, phi = 1 and theta = (1, 1) give every pair p = eps + (1/2 - eps) pi for
+# a link and dL/dphi = 0 of every row (a row's pi is 1 whatever phi); FP32's
+# roundings of p and its logarithm allow 1e-6
+@pytest.mark.gpu
+def test_more_sources_than_a_grid_dimension(gpu):
+    import math
+    from mcmc_for_ammsb_gb300.autograd import edge_log_likelihood
+    n_src, last = 2**31 + 5, 2**31 - 1
+    if torch.cuda.mem_get_info()[0] < 120 << 30:
+        pytest.skip("needs 120 GB of device memory")
+    phi = torch.ones(n_src, 1, device="cuda").requires_grad_()
+    pi = torch.tensor([[0.25], [0.5]], device="cuda").requires_grad_()
+    theta = torch.ones(1, 2, device="cuda").requires_grad_()
+    src = torch.tensor([0, last, last], device="cuda")
+    loss = edge_log_likelihood(phi, pi, theta, src, torch.tensor([0, 1, 0], device="cuda"),
+                               torch.ones(3, dtype=torch.uint8, device="cuda"), 1e-3)
+    p = [1e-3 + (0.5 - 1e-3) * x for x in (0.25, 0.5)]
+    assert float(loss.detach()) == pytest.approx(2 * math.log(p[0]) + math.log(p[1]), rel=1e-6)
+    dphi, dpi, _ = torch.autograd.grad(loss, [phi, pi, theta])
+    assert float(dphi[1:8].abs().max()) == 0.0 and float(dphi[last + 1:].abs().max()) == 0.0
+    assert float(dphi[[0, last]].abs().max()) <= 1e-6
+    assert dpi[:, 0].tolist() == pytest.approx([2 * 0.499 / p[0], 0.499 / p[1]], rel=1e-6)
