@@ -457,8 +457,10 @@ int check_draw_err(ammsb_handle* h, int slot) {
 // Rows of pi or phi into a host array of N x K floats.  FP32 rows are copied;
 // BF16 rows are widened on the device, a staging buffer at a time (a kernel and
 // a copy each: widening them on the host was 0.9 of the 1.05 ms that 5M values
-// took), after their host pages have been touched, as the host loop did: a copy
+// took), after their host pages have been touched, as the host loop does: a copy
 // into pages of a fresh array has the GPU fault them in (4 ms for 20 MB, not 1).
+// A few values, and any number on a device without room for the buffer, are
+// widened on the host (widen_on_device).
 constexpr size_t kReadBytes = 8u << 20;
 template <typename T>
 int get_rows(ammsb_handle* h, const T* rows, float* dst) {
@@ -471,9 +473,22 @@ int get_rows(ammsb_handle* h, const T* rows, float* dst) {
                            cudaMemcpyDeviceToHost, h->stream));
   } else {
     const int64_t per = std::min<int64_t>(N, std::max<int64_t>(1, (int64_t)(kReadBytes / sizeof(float)) / K));
-    if (!h->d_read) {
-      int rc = dev_alloc(h, &h->d_read, (size_t)(per * K));
-      if (rc) return rc;
+    auto stage = [&] {
+      if (h->d_read || dev_alloc(h, &h->d_read, (size_t)(per * K)) == AMMSB_OK) return true;
+      cudaGetLastError();  // no room: not this call's error
+      h->err.clear();
+      return false;
+    };
+    if (!widen_on_device(N * K, stage)) {
+      std::vector<uint16_t> bits((size_t)(N * K));
+      CK(cudaMemcpy2DAsync(bits.data(), sizeof(T) * K, rows, sizeof(T) * Kp, sizeof(T) * K, N, cudaMemcpyDeviceToHost,
+                           h->stream));
+      CK(cudaStreamSynchronize(h->stream));
+      for (size_t x = 0; x < bits.size(); ++x) {
+        const uint32_t word = (uint32_t)bits[x] << 16;
+        std::memcpy(dst + x, &word, sizeof(word));
+      }
+      return AMMSB_OK;
     }
     volatile char* page = reinterpret_cast<volatile char*>(dst);
     for (size_t x = 0; x < sizeof(float) * (size_t)(N * K); x += 4096) page[x] = 0;

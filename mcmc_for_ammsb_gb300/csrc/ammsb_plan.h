@@ -1,6 +1,6 @@
 // ammsb_plan.h -- sizes that a kernel and the buffers it writes have to agree
-// on, the order of a block's launches, and the rows that the samplers search, in
-// plain C++.
+// on, the order of a block's launches, the rows that the samplers search, and
+// choices between two ways of a call, in plain C++.
 #pragma once
 #include <stdint.h>
 
@@ -57,6 +57,16 @@ auto launch_block_order(Launches&& l, int count, bool first_early, bool early_fo
   }
   if (!e && !early_follows) e = l.join();
   return e;
+}
+
+// Whether BF16 rows are widened on the device for a read-out, with a staging
+// buffer that stage() allocates with the first read that wants it: reads of more
+// than 16,384 values, if it can be had.  2,000 values take the host's loop 22 us
+// and a kernel with its copy 28, 32,000 either 28, 140,000 the host 62 and the
+// kernel 35.
+template <class Stage>
+bool widen_on_device(int64_t values, Stage&& stage) {
+  return values > 16384 && stage();
 }
 
 // Pairs of n nodes (each(f) calls f(a, b) for every one) as a symmetric CSR with

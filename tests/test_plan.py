@@ -1,7 +1,8 @@
 """What csrc/ammsb_plan.h holds, compiled for the host: no round of a minibatch
 examines more candidates than an iteration's scratch area holds, an update that
-starts early finds its draws joined ahead of the theta step before it, and the
-pairs that the samplers leave out are rows in order."""
+starts early finds its draws joined ahead of the theta step before it, the pairs
+that the samplers leave out are rows in order, and a read-out that finds no room
+on the device is made without it."""
 import os
 import subprocess
 
@@ -85,6 +86,21 @@ int main(int argc, char** argv) {  // n, then the pairs
 """
 
 
+READS = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "ammsb_plan.h"
+int main() {
+  for (bool room : {true, false})
+    for (long long values : {1ll, 16384ll, 16385ll, 1ll << 40}) {
+      int asked = 0;
+      const bool on = ammsb::widen_on_device(values, [&] { return ++asked, room; });
+      std::printf("%d%d ", asked, (int)on);
+    }
+}
+"""
+
+
 def compiled_output(tmp_path, program, *args):
     src, exe = tmp_path / "program.cc", str(tmp_path / "program")
     src.write_text(program)
@@ -111,3 +127,8 @@ def test_left_out_pairs_are_rows_in_order(tmp_path):
         rows = [sorted([b for a, b in pairs if a == v] + [a for a, b in pairs if b == v]) for v in range(n)]
         out = compiled_output(tmp_path, ROWS, n, *(x for p in pairs for x in p))
         assert [[int(x) for x in line.split()] for line in out.split("\n")[:n]] == rows  # repeated pairs stay
+
+
+def test_a_read_without_room_for_its_staging_goes_on_on_the_host(tmp_path):
+    # (asked for the buffer, widened on the device) with room, then without
+    assert compiled_output(tmp_path, READS).split() == ["00", "00", "11", "11", "00", "00", "10", "10"]
