@@ -895,19 +895,6 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
   const int64_t set_bytes = 4 * (m.slot_nodes + m.slot_nbr) + 9 * m.slot_edges + 2 * m.slot_cand +
                             (h->mb_smem ? 0 : 4ll * hcap);
   if (2 * h->block * set_bytes > kRingBytes) h->block = std::min(h->block, 2);
-  m.ring = 2 * h->block;
-  const size_t nring = (size_t)m.ring;
-  TRY(dev_alloc(h, &b.nodes, nring * m.slot_nodes));
-  TRY(dev_alloc(h, &b.ea, nring * m.slot_edges));
-  TRY(dev_alloc(h, &b.eb, nring * m.slot_edges));
-  TRY(dev_alloc(h, &b.ey, nring * m.slot_edges));
-  TRY(dev_alloc(h, &b.nbr, nring * m.slot_nbr));
-  TRY(dev_alloc(h, &b.st, nring));
-  TRY(dev_alloc(h, &b.cand, (size_t)h->block * m.slot_cand));
-  if (!h->mb_smem) {
-    TRY(dev_alloc(h, &b.htab_key, (size_t)h->block * hcap));
-    TRY(dev_alloc(h, &b.htab_idx, (size_t)h->block * hcap));
-  }
   TRY(dev_alloc(h, &b.beta_part, (size_t)m.nbb * 2 * Kp));
   TRY(dev_alloc(h, &b.theta_pre, kThetaPre * (size_t)K));
   TRY(dev_alloc(h, &h->gc, 1));
@@ -918,6 +905,28 @@ int ammsb_create(const ammsb_options* opt_in, const ammsb_graph* graph,
   TRY(dev_alloc(h, &h->d_fed_theta_noise, 2 * (size_t)K));
   b.fed_phi_noise = nullptr;
   b.fed_theta_noise = nullptr;
+  // the ring last, so that a device with little room keeps its smaller one for it
+  const size_t before_ring = h->allocs.size();
+  auto alloc_ring = [&](int block) {
+    m.ring = 2 * block;
+    const size_t n = (size_t)m.ring;
+    rc = dev_alloc(h, &b.nodes, n * m.slot_nodes);
+    if (!rc) rc = dev_alloc(h, &b.ea, n * m.slot_edges);
+    if (!rc) rc = dev_alloc(h, &b.eb, n * m.slot_edges);
+    if (!rc) rc = dev_alloc(h, &b.ey, n * m.slot_edges);
+    if (!rc) rc = dev_alloc(h, &b.nbr, n * m.slot_nbr);
+    if (!rc) rc = dev_alloc(h, &b.st, n);
+    if (!rc) rc = dev_alloc(h, &b.cand, (size_t)block * m.slot_cand);
+    if (!rc && !h->mb_smem) rc = dev_alloc(h, &b.htab_key, (size_t)block * hcap);
+    if (!rc && !h->mb_smem) rc = dev_alloc(h, &b.htab_idx, (size_t)block * hcap);
+    if (rc) {
+      cudaGetLastError();
+      for (; h->allocs.size() > before_ring; h->allocs.pop_back()) cudaFree(h->allocs.back());
+    }
+    return rc == AMMSB_OK;
+  };
+  if (!(h->block = block_with_room(h->block, alloc_ring))) return bail(rc);
+  h->err.clear();
 #undef TRY
   // commit blocks (4 rows each, grid-strided): two per SM, so an iteration
   // of few nodes does not launch a thousand idle blocks

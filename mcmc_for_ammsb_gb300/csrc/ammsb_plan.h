@@ -59,6 +59,16 @@ auto launch_block_order(Launches&& l, int count, bool first_early, bool early_fo
   return e;
 }
 
+// The iterations of a draws launch: `want`, or as few as alloc(block), which gives
+// back what it got when it fails, finds room for (a ring of two blocks' buffer
+// sets: sixteen for eight iterations, four for two, two for one).  0: none.
+template <class Alloc>
+int block_with_room(int want, Alloc&& alloc) {
+  for (int block = want; block > 0; block = block > 2 ? 2 : block - 1)
+    if (alloc(block)) return block;
+  return 0;
+}
+
 // Whether BF16 rows are widened on the device for a read-out, with a staging
 // buffer that stage() allocates with the first read that wants it: reads of more
 // than 16,384 values, if it can be had.  2,000 values take the host's loop 22 us

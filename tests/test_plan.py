@@ -1,8 +1,8 @@
 """What csrc/ammsb_plan.h holds, compiled for the host: no round of a minibatch
 examines more candidates than an iteration's scratch area holds, an update that
 starts early finds its draws joined ahead of the theta step before it, the pairs
-that the samplers leave out are rows in order, and a read-out that finds no room
-on the device is made without it."""
+that the samplers leave out are rows in order, and a read-out or a ring
+of draws that finds no room on the device makes do with less."""
 import os
 import subprocess
 
@@ -101,6 +101,18 @@ int main() {
 """
 
 
+ROOM = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "ammsb_plan.h"
+int main() {
+  for (int want : {16, 8, 3, 2, 1})
+    for (int room : {32, 16, 4, 3, 2, 1})  // buffer sets that fit
+      std::printf("%d ", ammsb::block_with_room(want, [&](int block) { return 2 * block <= room; }));
+}
+"""
+
+
 def compiled_output(tmp_path, program, *args):
     src, exe = tmp_path / "program.cc", str(tmp_path / "program")
     src.write_text(program)
@@ -132,3 +144,8 @@ def test_left_out_pairs_are_rows_in_order(tmp_path):
 def test_a_read_without_room_for_its_staging_goes_on_on_the_host(tmp_path):
     # (asked for the buffer, widened on the device) with room, then without
     assert compiled_output(tmp_path, READS).split() == ["00", "00", "11", "11", "00", "00", "10", "10"]
+
+
+def test_a_ring_without_room_takes_smaller_blocks(tmp_path):
+    assert compiled_output(tmp_path, ROOM).split() == \
+        "16 2 2 1 1 0  8 8 2 1 1 0  3 3 2 1 1 0  2 2 2 1 1 0  1 1 1 1 1 0".split()
