@@ -547,27 +547,25 @@ int ammsb_batch_step(ammsb_batch* bt, int64_t n_iters) {
   bool forked = false;
   int64_t left = n_iters;
   while (left > 0) {  // as ammsb_step
-    const int s = bt->slot, pos = s % D, blk = s / D;
-    int n, rc;
-    if (pos == 0 && left >= D) {
-      const bool both = left >= 2 * (int64_t)D;
-      n = both ? 2 * D : D;
-      rc = launch_graph(bt, both ? bt->graphL[blk] : bt->graphB[blk], [&] {
-        cudaError_t e = launch_block_chains(bt, blk, false, both);
-        return e == cudaSuccess && both ? launch_block_chains(bt, 1 - blk, true, false) : e;
+    const int s = bt->slot, blk = s / D;
+    const NextLaunch next = next_launch(D, s, bt->ahead, left, !in_sync, true, false);
+    const int n = next.n;
+    int rc;
+    if (next.whole) {
+      rc = launch_graph(bt, next.both ? bt->graphL[blk] : bt->graphB[blk], [&] {
+        cudaError_t e = launch_block_chains(bt, blk, false, next.both);
+        return e == cudaSuccess && next.both ? launch_block_chains(bt, 1 - blk, true, false) : e;
       });
       drawn += (uint32_t)n;
     } else {
-      if (pos == 0) {
+      if (next.fork) {
         BK(fork_draws_chains(bt, 1 - blk));
         forked = true;
         drawn += (uint32_t)D;
         bt->ahead += D;
       }
-      const int most = (int)std::min<int64_t>(left, D - pos);
       int lg = 0;
-      while (lg < 3 && (2 << lg) <= most) ++lg;
-      n = 1 << lg;
+      while ((1 << lg) < n) ++lg;
       rc = launch_graph(bt, bt->graphU[s][lg], [&] { return launch_updates_chains(bt, s, n); });
       bt->ahead -= n;
       if (forked && (s + n) % D == 0) {

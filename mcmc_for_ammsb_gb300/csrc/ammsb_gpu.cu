@@ -1099,7 +1099,8 @@ int ammsb_step(ammsb_handle* h, int64_t n_iters) {
     h->step_count += (uint64_t)n_iters;
     return AMMSB_OK;
   }
-  if (h->ahead == 0) {  // the first block's draws
+  const bool fresh = h->ahead == 0;
+  if (fresh) {  // the first block's draws
     ++h->ring_gen;
     h->slot = 0;
     if ((rc = point_draws(h, h->step_count, h->stream))) return rc;
@@ -1110,16 +1111,14 @@ int ammsb_step(ammsb_handle* h, int64_t n_iters) {
   bool forked = false;  // draws on the side stream that this stream has not joined
   int64_t left = n_iters;
   while (left > 0) {
-    const int s = h->slot, pos = s % D, blk = s / D;
-    int n;
-    if (pos == 0 && left >= D) {
-      // whole blocks; both in turn in one launch, so that every update but
-      // the launch's first follows a theta step inside the graph (and may
-      // start early)
-      const bool both = h->opt.use_graph && !timed && left >= 2 * (int64_t)D;
-      n = both ? 2 * D : D;
+    const int s = h->slot, blk = s / D;
+    const NextLaunch next = next_launch(D, s, h->ahead, left, fresh, h->opt.use_graph && !timed, timed);
+    const int n = next.n;
+    if (next.whole) {
+      // both blocks in turn in one launch, so that every update but the
+      // launch's first follows a theta step inside the graph (and may start early)
       if (timed && (rc = take_phase_events(h, s, D, (1 - blk) * D))) return rc;
-      if (both)
+      if (next.both)
         rc = launch(h->graphL[blk], [&] {
           cudaError_t e = launch_block(h, blk, false, false, true);
           return e != cudaSuccess ? e : launch_block(h, 1 - blk, false, true);
@@ -1129,20 +1128,16 @@ int ammsb_step(ammsb_handle* h, int64_t n_iters) {
       if (rc) return rc;
       h->dev_next += (uint32_t)n;
     } else {
-      // part of a block: the other block's draws go out with its first
-      // iteration, as they do in a whole one
-      if (pos == 0) {
+      if (next.fork) {
         if (timed && (rc = take_phase_events(h, 0, 0, (1 - blk) * D))) return rc;
         CK(fork_draws(h, 1 - blk, timed));
         forked = true;
         h->dev_next += (uint32_t)D;
         h->ahead += D;
       }
-      const int most = (int)std::min<int64_t>(left, D - pos);
-      int lg = 0;  // runs of a power of two of them, so that few graphs are kept
-      while (!timed && lg < 3 && (2 << lg) <= most) ++lg;
-      n = 1 << lg;
       if (timed && (rc = take_phase_events(h, s, 1, -1))) return rc;
+      int lg = 0;
+      while ((1 << lg) < n) ++lg;
       if ((rc = launch(timed ? h->graphUt[s] : h->graphU[s][lg], [&] { return launch_updates(h, s, n, timed); })))
         return rc;
       h->ahead -= n;

@@ -59,6 +59,33 @@ auto launch_block_order(Launches&& l, int count, bool first_early, bool early_fo
   return e;
 }
 
+// What a call launches next with `left` iterations to go, at ring slot `slot` of
+// two blocks of D with `ahead` iterations drawn from there on: n updates -- one
+// whole block with the other's draws alongside, both in turn (`both`, where
+// `pairs` allows it), or a run of n (a power of two, so that few graphs are kept;
+// one with `single`) inside a block, with the other block's draws forked ahead of
+// it (`fork`): with a block's first launch, so that they overlap all of the call
+// that is left; but a `fresh` call, which had to make its first block's draws
+// itself, forks them only if it reaches the block's end.  Short calls that each
+// follow a change of state or step, which drops the draws, then make eight
+// iterations' draws rather than sixteen (set_step and step(1) of the 400,000-node
+// workload: 198 us, now 120).
+struct NextLaunch {
+  int n;
+  bool whole, both, fork;
+};
+inline NextLaunch next_launch(int D, int slot, int ahead, int64_t left, bool fresh, bool pairs, bool single) {
+  const int pos = slot % D, rest = D - pos;
+  if (pos == 0 && left >= D) {
+    const bool both = pairs && left >= 2 * (int64_t)D;
+    return {both ? 2 * D : D, true, both, false};
+  }
+  const int most = (int)plan_min(left, rest);
+  int n = 1;
+  while (!single && n < 8 && 2 * n <= most) n *= 2;
+  return {n, false, false, ahead == rest && (left >= rest || (pos == 0 && !fresh))};
+}
+
 // The iterations of a draws launch: `want`, or as few as alloc(block), which gives
 // back what it got when it fails, finds room for (a ring of two blocks' buffer
 // sets: sixteen for eight iterations, four for two, two for one).  0: none.

@@ -113,6 +113,42 @@ int main() {
 """
 
 
+CALLS = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "ammsb_plan.h"
+int main() {
+  unsigned seed = 1;
+  long long bad = 0;
+  for (int D : {1, 2, 3, 8, 16})
+    for (bool pairs : {true, false})
+      for (bool single : {true, false})
+        for (int chain = 0; chain < 200; ++chain) {
+          long long drawn = D, done = 0;  // of this chain's iterations
+          for (int call = 0, slot = 0, ahead = D; call < 12; ++call) {
+            seed = seed * 1664525u + 1013904223u;
+            const long long count = 1 + (seed >> 8) % (chain % 2 ? 3 * D + 2 : D);
+            for (long long left = count; left > 0;) {
+              const auto next = ammsb::next_launch(D, slot, ahead, left, call == 0, pairs, single);
+              if (next.fork) drawn += D, ahead += D;
+              bad += next.n < 1 || next.n > left || next.n > ahead + (next.whole ? next.n : 0);
+              bad += next.whole ? slot % D != 0 || ahead != D || next.n != (next.both ? 2 * D : D) || (next.both && !pairs)
+                                : slot % D + next.n > D || (next.n & (next.n - 1)) != 0 || (single && next.n > 1);
+              if (next.whole) drawn += next.n; else ahead -= next.n;
+              slot = (slot + next.n) % (2 * D);
+              done += next.n, left -= next.n;
+              bad += drawn - done != ahead || ahead < 1 || ahead > 2 * D || drawn % D != 0;
+              // the first call, after its own draws, makes those of blocks that it reaches; a
+              // later one also those of the block after the one where it ends
+              bad += drawn > ((done + left) / D + (call == 0 ? 1 : 2)) * D;
+            }
+          }
+        }
+  std::printf("%lld", bad);
+}
+"""
+
+
 def compiled_output(tmp_path, program, *args):
     src, exe = tmp_path / "program.cc", str(tmp_path / "program")
     src.write_text(program)
@@ -149,3 +185,7 @@ def test_a_read_without_room_for_its_staging_goes_on_on_the_host(tmp_path):
 def test_a_ring_without_room_takes_smaller_blocks(tmp_path):
     assert compiled_output(tmp_path, ROOM).split() == \
         "16 2 2 1 1 0  8 8 2 1 1 0  3 3 2 1 1 0  2 2 2 1 1 0  1 1 1 1 1 0".split()
+
+
+def test_a_call_draws_no_block_that_it_does_not_reach(tmp_path):
+    assert compiled_output(tmp_path, CALLS) == "0"
