@@ -1,5 +1,5 @@
-// ammsb_batch.cu -- many independent chains advanced together, one CUDA
-// graph launch per iteration for all of them.
+// ammsb_batch.cu -- many independent chains advanced together, up to sixteen
+// iterations of all of them per CUDA graph launch.
 //
 // Each chain is an ammsb_handle of its own (its graph, held-out set, state,
 // options and update_phi configuration).  The batch launches every kernel

@@ -25,7 +25,8 @@ constexpr int kMaxRing = 2 * kMaxBlock;
 // A ring of at most this many bytes takes the full block (16 sets of the
 // 4,096-edge, 128-neighbour minibatch are 35 MB); larger buffer sets
 // (random-edge over the whole training set, where an iteration lasts so long
-// that its draws' launches do not show) take blocks of two.
+// that its draws' launches do not show) take blocks of two, as does a ring for
+// which the device has no room (block_with_room).
 constexpr int64_t kRingBytes = 1ll << 30;
 
 // Launches of the iteration that may start before the kernel ahead of them
@@ -91,7 +92,7 @@ struct ammsb_handle {
   GammaTables* d_gamma = nullptr;
   int ncommit = 1;
   bool star = false;  // drawn minibatches are stars
-  int nbr_blocks = 1, phi_blocks = 1;
+  int nbr_blocks = 1;
   size_t phi_smem = 0, phi_smem_few = 0, nbr_smem = 0, mb_smem = 0;
   // host mirrors
   uint64_t step_count = 1;     // learner.cc:37

@@ -25,7 +25,7 @@
 namespace ammsb {
 
 // Upper bound of Model::nbb, the blocks of k_commit_beta that write beta
-// gradient partials (k_theta reads them back, up to 9 per warp).
+// gradient partials (k_theta reads them back, up to 36 per warp: four chains of 9).
 #ifndef AMMSB_MAX_BETA_BLOCKS
 #define AMMSB_MAX_BETA_BLOCKS 256
 #endif
@@ -1021,15 +1021,6 @@ __global__ void __launch_bounds__(NPB * SPLIT * LPN) k_update_phi_chains(const C
 }
 
 // ---------------------------------------------------------------------------
-// k_commit_beta: blocks [0, ncommit) copy the staged rows into pi (the
-// reference's update_pi loop, cc:162-166); blocks [ncommit, ncommit+nbb)
-// evaluate update_beta's per-edge terms (cc:212-240) on the staged (new) pi
-// and reduce them per block.  With f_k = pi_ak pi_bk, P_e = sum_k
-// (y ? beta_k : 1-beta_k) f_k + (y ? eps : 1-eps)(1 - sum_k f_k) the
-// gradient only needs R_yk = sum_{e: y_e = y} f_ek / P_e (k_theta applies the
-// theta factors), accumulated per warp in registers, then per block.
-// ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // The parts of k's theta step that do not depend on the sums: theta and beta
 // themselves, eta_c - theta_kc, the noise terms sqrt(eps theta_kc) n_kc,
 // 1/(theta0+theta1) and the two gradient factors 1/theta_kc - 1/ts -- three FP64
@@ -1092,6 +1083,15 @@ __device__ __forceinline__ float edge_inv_prob(float fsum, float psum, bool y, f
   return 1.0f / __fmaf_rn(y ? epsilon : 1.0f - epsilon, 1.0f - fsum, psum);
 }
 
+// ---------------------------------------------------------------------------
+// k_commit_beta: blocks [0, ncommit) copy the staged rows into pi (the
+// reference's update_pi loop, cc:162-166); blocks [ncommit, ncommit+nbb)
+// evaluate update_beta's per-edge terms (cc:212-240) on the staged (new) pi
+// and reduce them per block.  With f_k = pi_ak pi_bk, P_e = sum_k
+// (y ? beta_k : 1-beta_k) f_k + (y ? eps : 1-eps)(1 - sum_k f_k) the
+// gradient only needs R_yk = sum_{e: y_e = y} f_ek / P_e (k_theta applies the
+// theta factors), accumulated per warp in registers, then per block.
+// ---------------------------------------------------------------------------
 template <typename PiT, int KQ>
 __device__ __forceinline__ void commit_beta_body(const Model& m, const Buffers& b, int ncommit, int block) {
   using TR = PiTraits<PiT>;

@@ -280,8 +280,8 @@ class MCMCSamplerStochastic:
 
 
 class ChainBatch:
-    """Independent chains advanced together, one CUDA graph launch per
-    iteration for all of them (ammsb_batch_*).  Every sampler keeps its own
+    """Independent chains advanced together, up to sixteen iterations of
+    all of them per CUDA graph launch (ammsb_batch_*).  Every sampler keeps its own
     graph, state and step counter; step(n) advances all of them by n."""
 
     def __init__(self, samplers):
