@@ -190,7 +190,7 @@ thread_local std::string g_batch_create_error;
 
 // The update in two parts, as for one chain.  `pdl`: the theta step of the
 // iteration before is the kernel ahead in the stream and this iteration's draws
-// were complete before that step ended.
+// were complete before that step started.
 cudaError_t launch_rows_chains(ammsb_batch* bt, int p, bool pdl) {
   // the update_phi groups touch disjoint chains: they run concurrently
   // (parallel branches of the captured graph), then join before the commits.
@@ -256,7 +256,7 @@ cudaError_t fork_draws_chains(ammsb_batch* bt, int blk) {
   return cudaEventRecord(bt->ev_join, bt->side);
 }
 
-cudaError_t launch_block_chains(ammsb_batch* bt, int blk, bool first_early, bool early_follows) {
+cudaError_t launch_block_chains(ammsb_batch* bt, int blk) {
   struct Launches {
     ammsb_batch* bt;
     int blk;
@@ -265,7 +265,7 @@ cudaError_t launch_block_chains(ammsb_batch* bt, int blk, bool first_early, bool
     cudaError_t theta(int i) { return launch_theta_chains(bt, blk * bt->block + i); }
     cudaError_t join() { return cudaStreamWaitEvent(bt->stream, bt->ev_join, 0); }
   };
-  return launch_block_order(Launches{bt, blk}, bt->block, first_early, early_follows);
+  return launch_block_order(Launches{bt, blk}, bt->block);
 }
 
 // Launches `work` as a captured graph kept in g.
@@ -553,8 +553,8 @@ int ammsb_batch_step(ammsb_batch* bt, int64_t n_iters) {
     int rc;
     if (next.whole) {
       rc = launch_graph(bt, next.both ? bt->graphL[blk] : bt->graphB[blk], [&] {
-        cudaError_t e = launch_block_chains(bt, blk, false, next.both);
-        return e == cudaSuccess && next.both ? launch_block_chains(bt, 1 - blk, true, false) : e;
+        cudaError_t e = launch_block_chains(bt, blk);
+        return e == cudaSuccess && next.both ? launch_block_chains(bt, 1 - blk) : e;
       });
       drawn += (uint32_t)n;
     } else {

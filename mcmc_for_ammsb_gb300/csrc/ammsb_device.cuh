@@ -31,8 +31,8 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // counts as triggered); (2) in every launch at least one CTA waits before it
 // exits (every CTA, where the launch has no work); (3) before its wait a kernel
 // reads only what kernels at least two launches ahead in the stream wrote (or
-// draws joined before the launch ahead: an edge of the launch itself from the
-// joined stream would be a programmatic one too).  By (1) and (2) a launch completes
+// draws joined before the launch ahead: a launch that follows a joined stream
+// itself has a programmatic edge from there too, and is no early one).  By (1) and (2) a launch completes
 // after the kernel ahead of it, and update_phi and the commit start only once
 // the kernel two ahead has completed.  The commit triggers at its start, so
 // that the theta step's launch (some 2 us) is over when the commit ends: the

@@ -83,7 +83,7 @@ cudaError_t launch_phi_t(ammsb_handle* h, const Buffers& b, bool pdl) {
 }
 
 // `pdl`: the launch directly follows k_theta in the stream and its draws
-// were complete before that kernel's wait ended; it then starts as a programmatic
+// were complete before that kernel started; it then starts as a programmatic
 // dependent launch, which overlaps its first row copies and node prologues
 // with the theta step.
 template <typename PiT, int VPL, int STAGES, bool FULL>
@@ -239,7 +239,7 @@ inline cudaError_t mark(cudaEvent_t ev, cudaStream_t s) {
 // theta, and every kernel waits for the one ahead to finish; without, the commit
 // and theta step start as programmatic dependent launches (cfg.pdl).  `pdl`:
 // the previous iteration's theta step is the kernel ahead in the stream and
-// this iteration's draws were complete before that step ended (update_phi may
+// this iteration's draws were complete before that step started (update_phi may
 // then start early).  `star`: the minibatch is one.
 cudaError_t launch_rows(ammsb_handle* h, const Buffers& b, bool star, const cudaEvent_t* ev, bool pdl) {
   cudaError_t e = (h->opt.pi_dtype == AMMSB_PI_BF16) ? launch_phi<__nv_bfloat16>(h, b, pdl)
@@ -315,7 +315,7 @@ cudaError_t join_draws(ammsb_handle* h) { return cudaStreamWaitEvent(h->stream, 
 // which eight iterations side by side pay once; with a launch per iteration
 // the draws were the longer branch of every small chain and of every
 // link-stratum iteration.
-cudaError_t launch_block(ammsb_handle* h, int blk, bool timed, bool first_early = false, bool early_follows = false) {
+cudaError_t launch_block(ammsb_handle* h, int blk, bool timed) {
   struct Launches {
     ammsb_handle* h;
     int blk;
@@ -325,7 +325,7 @@ cudaError_t launch_block(ammsb_handle* h, int blk, bool timed, bool first_early 
     cudaError_t theta(int i) { return launch_slot_theta(h, blk * h->block + i, timed); }
     cudaError_t join() { return join_draws(h); }
   };
-  return launch_block_order(Launches{h, blk, timed}, h->block, first_early, early_follows);
+  return launch_block_order(Launches{h, blk, timed}, h->block);
 }
 
 // One iteration at ring slot s in run()'s loop order on the handle's
@@ -1115,13 +1115,12 @@ int ammsb_step(ammsb_handle* h, int64_t n_iters) {
     const NextLaunch next = next_launch(D, s, h->ahead, left, fresh, h->opt.use_graph && !timed, timed);
     const int n = next.n;
     if (next.whole) {
-      // both blocks in turn in one launch, so that every update but the
-      // launch's first follows a theta step inside the graph (and may start early)
+      // both blocks in turn in one launch where that many are asked for
       if (timed && (rc = take_phase_events(h, s, D, (1 - blk) * D))) return rc;
       if (next.both)
         rc = launch(h->graphL[blk], [&] {
-          cudaError_t e = launch_block(h, blk, false, false, true);
-          return e != cudaSuccess ? e : launch_block(h, 1 - blk, false, true);
+          cudaError_t e = launch_block(h, blk, false);
+          return e != cudaSuccess ? e : launch_block(h, 1 - blk, false);
         });
       else
         rc = launch(timed ? h->graphBt[blk] : h->graphB[blk], [&] { return launch_block(h, blk, timed); });

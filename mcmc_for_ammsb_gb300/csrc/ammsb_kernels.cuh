@@ -876,7 +876,7 @@ __device__ __forceinline__ void update_phi_body(const Model& m, const Buffers& b
       }
     }
     // beta, read from here on, is written by the theta step ahead of this
-    // launch; everything read before was complete before that step's own wait ended
+    // launch; everything read before was complete before that step started
     grid_dependency_wait();
     grid_launch_dependents();
     if (active) {

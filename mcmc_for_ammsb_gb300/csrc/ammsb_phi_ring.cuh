@@ -268,7 +268,7 @@ __device__ __forceinline__ void update_phi_ring_body(const Model& m, const Buffe
     node_sync<SPLIT>(group);
     // beta, read from here on, is written by the theta step ahead of this
     // launch; everything read before (node ids, neighbour words and rows,
-    // phi) was complete before that step's own wait ended
+    // phi) was complete before that step started
     grid_dependency_wait();
     grid_launch_dependents();
     S = 0.f;

@@ -1,6 +1,6 @@
 """What csrc/ammsb_plan.h holds, compiled for the host: no round of a minibatch
-examines more candidates than an iteration's scratch area holds, an update that
-starts early finds its draws joined ahead of the theta step before it, the pairs
+examines more candidates than an iteration's scratch area holds, no update starts
+early right behind the join of its draws, the pairs
 that the samplers leave out are rows in order, and a read-out or a ring
 of draws that finds no room on the device makes do with less."""
 import os
@@ -59,9 +59,9 @@ struct Recorder {  // F fork, J join, R and r rows (r early), T theta, X the lau
 int main() {
   for (int count : {1, 3}) {
     std::string pair, failed;
-    ammsb::launch_block_order(Recorder{&pair, -1}, count, false, true);
-    ammsb::launch_block_order(Recorder{&pair, -1}, count, true, false);
-    const int e = ammsb::launch_block_order(Recorder{&failed, count + 1}, count, false, false);
+    ammsb::launch_block_order(Recorder{&pair, -1}, count);
+    ammsb::launch_block_order(Recorder{&pair, -1}, count);
+    const int e = ammsb::launch_block_order(Recorder{&failed, count + 1}, count);
     std::printf("%s %s %d\n", pair.c_str(), failed.c_str(), e);
   }
 }
@@ -162,11 +162,11 @@ def test_a_round_fits_its_scratch_area(tmp_path):
     assert "rounds checked" in compiled_output(tmp_path, ROUNDS)
 
 
-def test_draws_are_joined_before_the_theta_step_ahead(tmp_path):
+def test_no_update_starts_early_behind_the_join_of_its_draws(tmp_path):
     one, three = compiled_output(tmp_path, ORDER).splitlines()
-    # a block whose end the next block's first update (r) overlaps, and that block
-    assert one == "FRJT" "FrTJ" " FRX 1"
-    assert three == "FRTrTrJT" "FrTrTrTJ" " FRTrX 1"
+    # two blocks in turn: R, not r, behind a J
+    assert one == "FRTJ" "FRTJ" " FRX 1"
+    assert three == "FRTrTrTJ" "FRTrTrTJ" " FRTrX 1"
 
 
 def test_left_out_pairs_are_rows_in_order(tmp_path):
