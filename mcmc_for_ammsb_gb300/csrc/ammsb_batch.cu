@@ -526,6 +526,7 @@ int ammsb_batch_step(ammsb_batch* bt, int64_t n_iters) {
     in_sync = bt->h[i]->ring_gen == bt->expect_gen[i] && bt->h[i]->step_count == bt->expect_step[i];
   for (ammsb_handle* h : bt->h) BK(cudaStreamSynchronize(h->stream));
   const int D = bt->block, R = 2 * D;
+  const bool brief = brief_call(D, in_sync ? bt->ahead : 0, n_iters);
   uint32_t drawn = 0;  // iterations drawn by this call
   if (!in_sync) {
     for (size_t i = 0; i < bt->h.size(); ++i) {
@@ -548,7 +549,7 @@ int ammsb_batch_step(ammsb_batch* bt, int64_t n_iters) {
   int64_t left = n_iters;
   while (left > 0) {  // as ammsb_step
     const int s = bt->slot, blk = s / D;
-    const NextLaunch next = next_launch(D, s, bt->ahead, left, !in_sync, true, false);
+    const NextLaunch next = next_launch(D, s, bt->ahead, left, brief, true, false);
     const int n = next.n;
     int rc;
     if (next.whole) {

@@ -1099,8 +1099,8 @@ int ammsb_step(ammsb_handle* h, int64_t n_iters) {
     h->step_count += (uint64_t)n_iters;
     return AMMSB_OK;
   }
-  const bool fresh = h->ahead == 0;
-  if (fresh) {  // the first block's draws
+  const bool brief = brief_call(D, h->ahead, n_iters);
+  if (h->ahead == 0) {  // the first block's draws
     ++h->ring_gen;
     h->slot = 0;
     if ((rc = point_draws(h, h->step_count, h->stream))) return rc;
@@ -1112,7 +1112,7 @@ int ammsb_step(ammsb_handle* h, int64_t n_iters) {
   int64_t left = n_iters;
   while (left > 0) {
     const int s = h->slot, blk = s / D;
-    const NextLaunch next = next_launch(D, s, h->ahead, left, fresh, h->opt.use_graph && !timed, timed);
+    const NextLaunch next = next_launch(D, s, h->ahead, left, brief, h->opt.use_graph && !timed, timed);
     const int n = next.n;
     if (next.whole) {
       // both blocks in turn in one launch where that many are asked for

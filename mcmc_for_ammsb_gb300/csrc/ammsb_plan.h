@@ -66,16 +66,19 @@ auto launch_block_order(Launches&& l, int count) {
 // `pairs` allows it), or a run of n (a power of two, so that few graphs are kept;
 // one with `single`) inside a block, with the other block's draws forked ahead of
 // it (`fork`): with a block's first launch, so that they overlap all of the call
-// that is left; but a `fresh` call, which had to make its first block's draws
-// itself, forks them only if it reaches the block's end.  Short calls that each
-// follow a change of state or step, which drops the draws, then make eight
-// iterations' draws rather than sixteen (set_step and step(1) of the 400,000-node
-// workload: 198 us, now 120).
+// that is left.  A `brief` call -- one that had to make its first block's draws
+// itself, and is over after a quarter of it -- leaves them to a later one unless it
+// reaches the block's end: such calls that each follow a change of state or step,
+// which drops the draws, make eight iterations' draws rather than sixteen (set_step
+// and step(1) of the 400,000-node workload: 198 us, now 121).  Longer ones overlap
+// them (64 chains on streams of their own, step(5) and step(200): 48.5 ms, 60 with
+// the draws of the first call left to the second).
+inline bool brief_call(int D, int ahead, int64_t n) { return ahead == 0 && n <= (D < 8 ? 1 : D / 4); }
 struct NextLaunch {
   int n;
   bool whole, both, fork;
 };
-inline NextLaunch next_launch(int D, int slot, int ahead, int64_t left, bool fresh, bool pairs, bool single) {
+inline NextLaunch next_launch(int D, int slot, int ahead, int64_t left, bool brief, bool pairs, bool single) {
   const int pos = slot % D, rest = D - pos;
   if (pos == 0 && left >= D) {
     const bool both = pairs && left >= 2 * (int64_t)D;
@@ -84,7 +87,7 @@ inline NextLaunch next_launch(int D, int slot, int ahead, int64_t left, bool fre
   const int most = (int)plan_min(left, rest);
   int n = 1;
   while (!single && n < 8 && 2 * n <= most) n *= 2;
-  return {n, false, false, ahead == rest && (left >= rest || (pos == 0 && !fresh))};
+  return {n, false, false, ahead == rest && (left >= rest || (pos == 0 && !brief))};
 }
 
 // The iterations of a draws launch: `want`, or as few as alloc(block), which gives

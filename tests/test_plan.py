@@ -129,7 +129,7 @@ int main() {
             seed = seed * 1664525u + 1013904223u;
             const long long count = 1 + (seed >> 8) % (chain % 2 ? 3 * D + 2 : D);
             for (long long left = count; left > 0;) {
-              const auto next = ammsb::next_launch(D, slot, ahead, left, call == 0, pairs, single);
+              const auto next = ammsb::next_launch(D, slot, ahead, left, call == 0 && ammsb::brief_call(D, 0, count), pairs, single);
               if (next.fork) drawn += D, ahead += D;
               bad += next.n < 1 || next.n > left || next.n > ahead + (next.whole ? next.n : 0);
               bad += next.whole ? slot % D != 0 || ahead != D || next.n != (next.both ? 2 * D : D) || (next.both && !pairs)
@@ -138,9 +138,9 @@ int main() {
               slot = (slot + next.n) % (2 * D);
               done += next.n, left -= next.n;
               bad += drawn - done != ahead || ahead < 1 || ahead > 2 * D || drawn % D != 0;
-              // the first call, after its own draws, makes those of blocks that it reaches; a
-              // later one also those of the block after the one where it ends
-              bad += drawn > ((done + left) / D + (call == 0 ? 1 : 2)) * D;
+              // a brief call, after its own draws, makes those of blocks that it reaches;
+              // another also those of the block after the one where it ends
+              bad += drawn > ((done + left) / D + (call == 0 && count <= (D < 8 ? 1 : D / 4) ? 1 : 2)) * D;
             }
           }
         }
