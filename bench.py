@@ -699,7 +699,7 @@ def chains_arm(args):
     seq_s = time.perf_counter() - t0
     e3 = evals()
     Ks = sorted({s.K for s in samplers})
-    line = {"metric": "edge-evals/s, %d independent chains, one graph launch per iteration" % args.chains,
+    line = {"metric": "edge-evals/s, %d independent chains, 16 iterations per graph launch" % args.chains,
             "value": (e1 - e0) / (ms / 1000.0), "unit": UNIT,
             "ms_per_iteration_all_chains": ms / args.steps,
             "chain_iterations_per_s": args.chains * args.steps / (ms / 1000.0),
